@@ -72,7 +72,7 @@ void Engine::shutdown() {
     hmeta = nullptr;
     hmeta_bytes = 0;
     for (DevBuf* b : {&key0, &keyn, &tvals, &ft, &slot2vtx, &bitmap, &offs, &partials, &vkey0, &vkeyn,
-                      &vv0, &vv1, &nbr, &vf32, &vtx2slot, &sval, &rec, &recw, &grid, &grid2, &tags, &vlist, &dstat, &meta, &img_a, &img_b,
+                      &vv0, &vv1, &nbr, &vf32, &vtx2slot, &sval, &rec, &grid, &grid2, &tags, &vlist, &dstat, &meta, &img_a, &img_b,
                       &img_c, &img_d})
         b->release();
 }
@@ -346,8 +346,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             ((homog || payb == 2) && (rc = E.vf32.ensure(cap_total * vdp * 4))) ||
             (rc = E.vtx2slot.ensure(cap_total * 4)) || (rc = E.sval.ensure(cap_total * vdp * accb)) ||
             (use_tags && (rc = E.tags.ensure(cap_total))) ||
-            (B.replay && (rc = E.rec.ensure((size_t)entries * 4))) ||
-            (replay_w && (rc = E.recw.ensure((size_t)entries * 4))))
+            (B.replay && (rc = E.rec.ensure((size_t)entries * (replay_w ? 8 : 4)))))
             return rc;
 
         // per-lattice descriptors, staged in pinned memory and uploaded by the first copy
@@ -412,8 +411,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             }
             sa.vcount = dM;
             sa.seg_counts = (uint32_t*)(dmeta + L.counts);
-            sa.rec_slot = B.replay ? (uint32_t*)E.rec.p : nullptr;
-            sa.rec_w = replay_w ? (float*)E.recw.p : nullptr;
+            sa.rec_slot = B.replay && !replay_w ? (uint32_t*)E.rec.p : nullptr;
+            sa.rec = replay_w ? E.rec.p : nullptr;
             sa.seg_status = (unsigned*)(dmeta + L.segstat);
             sa.blocks = (uint32_t)blocks;
             sa.tile_blocks = (uint32_t)tile_blocks;
@@ -524,8 +523,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sl.keyn = (uint4*)E.keyn.p;
             sl.cap_total = (uint32_t)cap_total;
             sl.slot2vtx = (const uint32_t*)E.slot2vtx.p;
-            sl.rec_slot = B.replay ? (const uint32_t*)E.rec.p : nullptr;
-            sl.rec_w_in = replay_w ? (const float*)E.recw.p : nullptr;
+            sl.rec_slot = B.replay && !replay_w ? (const uint32_t*)E.rec.p : nullptr;
+            sl.rec = replay_w ? E.rec.p : nullptr;
             sl.svals = E.sval.p;
             sl.vd = vd;
             sl.rec_vtx = B.rec_vtx;
@@ -547,7 +546,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
                 (uint64_t)B.blur_grid, blocks,
                 tile_blocks, slice_blocks, (uint64_t)(uintptr_t)E.key0.p, (uint64_t)(uintptr_t)E.keyn.p,
                 (uint64_t)(uintptr_t)E.tvals.p, (uint64_t)(uintptr_t)E.nbr.p, (uint64_t)(uintptr_t)E.rec.p,
-                (uint64_t)(uintptr_t)E.recw.p, (uint64_t)(uintptr_t)E.meta.p, (uint64_t)(uintptr_t)h,
+                (uint64_t)(uintptr_t)E.meta.p, (uint64_t)(uintptr_t)h,
                 (uint64_t)(uintptr_t)E.sval.p, (uint64_t)(uintptr_t)E.vlist.p, (uint64_t)(uintptr_t)E.vv0.p,
                 (uint64_t)(uintptr_t)E.vv1.p, (uint64_t)(uintptr_t)E.vkey0.p, (uint64_t)(uintptr_t)E.vf32.p,
                 (uint64_t)vrows, (uint64_t)(uintptr_t)E.vtx2slot.p, (uint64_t)nbr_half, (uint64_t)B.tile_w};

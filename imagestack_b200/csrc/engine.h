@@ -63,8 +63,7 @@ struct Engine {
     DevBuf vf32;   // FP32 normalised rows feeding the first blur pass (16-bit homogeneous)
     DevBuf vtx2slot;   // slot of each vertex
     DevBuf sval;       // filtered rows in slot space, arithmetic type, read by the slice
-    DevBuf rec;        // slot of every (point, remainder), [r][n], recorded by the splat
-    DevBuf recw;       // its barycentric weight, [r][n], recorded by the splat
+    DevBuf rec;        // row and weight of every (point, remainder), recorded by the splat
     DevBuf grid, grid2;   // the dense grid of the grid method, and its blur's second buffer
     DevBuf tags;       // one tag byte per hash slot (compaction -> neighbour lookups)
     DevBuf vlist;      // slots in the order the splat created them (the vertex list)

@@ -132,6 +132,14 @@ static uint32_t pow2_at_least(uint32_t x) {
     return p;
 }
 
+static uint32_t log2_of(uint32_t pow2) {
+    uint32_t k = 0;
+    while ((1u << k) < pow2) ++k;
+    return k;
+}
+// floor(2^32 / d) for div_magic
+static uint32_t magic_of(uint32_t d) { return d <= 1 ? 0xFFFFFFFFu : (uint32_t)(0x100000000ull / d); }
+
 void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint32_t* splat,
                       uint32_t* tile, uint32_t* slice, uint32_t tile_w) {
     const PointSource& q = s.src;
@@ -148,10 +156,14 @@ void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint
         s.tile_h = (uint32_t)kTilePixels / s.tile_w;
         s.tiles_x = (W + s.tile_w - 1) / s.tile_w;
         s.tiles_y = (H + s.tile_h - 1) / s.tile_h;
+        s.tile_shift = log2_of(s.tile_w);
+        s.tile_xm = magic_of(s.tiles_x);
+        s.tile_fm = magic_of(s.tiles_x * s.tiles_y);
         *tile = s.tiles_x * s.tiles_y * F;
         *splat = 0;
     } else {
         s.tile_w = s.tile_h = s.tiles_x = s.tiles_y = 0;
+        s.tile_shift = s.tile_xm = s.tile_fm = 0;
         *tile = 0;
         *splat = (uint32_t)((n + kSplatThreads - 1) / kSplatThreads);
     }
@@ -161,8 +173,12 @@ void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint
     s.slice_th = (uint32_t)kSliceThreads / s.slice_tw;
     s.stiles_x = (Ws + s.slice_tw - 1) / s.slice_tw;
     s.stiles_y = (Hs + s.slice_th - 1) / s.slice_th;
+    s.slice_shift = log2_of(s.slice_tw);
+    s.stile_xm = magic_of(s.stiles_x);
+    s.stile_fm = magic_of(s.stiles_x * s.stiles_y);
     *slice = s.stiles_x * s.stiles_y * Fs;
 }
+
 const DimOps* dim_ops(int d) {
     switch (d) {
     case 1: return dim_ops_1();

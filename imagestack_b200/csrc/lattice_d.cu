@@ -100,7 +100,7 @@ void neighbours(const NbrArgs& a, uint32_t vmax, int sms, cudaStream_t st) {
 template <int VDP, typename A>
 void slice_t(const SliceArgs& a, cudaStream_t st) {
     if (!a.blocks) return;
-    if (a.rec_slot && a.rec_w_in && !a.rec_vtx)
+    if (a.rec)
         slice_replay_kernel<D, VDP, A><<<a.blocks, kSliceThreads, 0, st>>>(a);
     else
         slice_kernel<D, VDP, A><<<a.blocks, kSliceThreads, 0, st>>>(a);

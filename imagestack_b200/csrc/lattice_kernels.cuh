@@ -81,8 +81,21 @@ struct Segment {
     uint32_t tile_base;    // first block in the tile splat launch
     uint32_t tile_w, tile_h, tiles_x, tiles_y;     // tile splat geometry (tile_w 0: direct)
     uint32_t slice_tw, slice_th, stiles_x, stiles_y;   // slice geometry
-    uint32_t pad_;
+    // block -> tile without divisions: log2 of the tile widths (powers of two) and
+    // floor(2^32 / divisor) of tiles per row and per frame (div_magic)
+    uint32_t tile_shift, slice_shift;
+    uint32_t tile_xm, tile_fm, stile_xm, stile_fm;
 };
+
+// b / d with m = floor(2^32 / d) (2^32 - 1 for d = 1), for b < 2^31: the multiply-high is the
+// quotient or one less.
+__device__ __forceinline__ uint32_t div_magic(uint32_t b, uint32_t d, uint32_t m, uint32_t* rem) {
+    uint32_t q = __umulhi(b, m);
+    uint32_t r = b - q * d;
+    if (r >= d) ++q, r -= d;
+    *rem = r;
+    return q;
+}
 
 // Segment of block b of a launch whose per-segment first blocks are the field Base: the
 // last segment whose Base <= b (segments are in block order; a segment with no blocks in
@@ -112,7 +125,7 @@ __device__ __forceinline__ int segment_of_slot(const uint32_t* slot_base, int ns
     return lo;
 }
 
-// the block's segment, copied into shared memory by the whole block (ends with a barrier)
+// The block's segment, copied into shared memory by the whole block (ends with a barrier)
 __device__ __forceinline__ void load_segment(const Segment* g, Segment& s) {
     static_assert(sizeof(Segment) % 4 == 0, "Segment is copied as 32-bit words");
     const uint32_t* src = reinterpret_cast<const uint32_t*>(g);
@@ -132,7 +145,7 @@ struct SplatArgs {
     void* vals;            // cap_total * VDP accumulators (float or double), zeroed
     uint32_t* ft;          // cap_total first-touch entries, all ones; null: not tracked
     uint32_t* rec_slot;    // optional [r][n_total] slot of every (point, remainder)
-    float* rec_w;          // optional [r][n_total] barycentric weight of every (point, remainder)
+    void* rec;             // optional replay record: rows and weights (store_record)
     unsigned* seg_status;  // one status word per segment
     uint32_t blocks;       // direct splat blocks of the batch
     uint32_t tile_blocks;  // tile splat blocks of the batch
@@ -266,7 +279,7 @@ struct SliceArgs {
     uint32_t cap_total;
     const uint32_t* slot2vtx;   // parity dumps only
     const uint32_t* rec_slot;   // slots recorded by the splat, [r][n_total]; null: look up
-    const float* rec_w_in;      // weights recorded by the splat, [r][n_total] (replay gather)
+    const void* rec;            // replay record of the splat (store_record), or null
     const void* svals;          // filtered rows in slot space (float, or double)
     int vd;
     int* rec_vtx;               // optional (point, remainder) vertex indices (dumps)
@@ -394,6 +407,40 @@ __device__ __forceinline__ float acc_add(float a, float b) { return __fadd_rn(a,
 __device__ __forceinline__ double acc_add(double a, double b) { return __dadd_rn(a, b); }
 
 // ---------------------------------------------------------------------------------
+// replay record: the row (0xFFFFFFFF: none) and the weight of every remainder of a point.
+// Remainders 2j and 2j+1 of point i are the four words (row, weight, row, weight) at
+// [j][i]; the last of an odd number of remainders is two words behind them.  A warp's
+// accesses are then runs of 16 bytes per lane: 3 stores and 3 loads per point at d = 5
+// instead of 12 each of four bytes.
+// ---------------------------------------------------------------------------------
+template <int D>
+__device__ __forceinline__ void store_record(void* rec, uint32_t n_total, uint32_t i, const uint32_t (&row)[D + 1],
+                                             const float (&w)[D + 1]) {
+    uint4* pairs = reinterpret_cast<uint4*>(rec);
+#pragma unroll
+    for (int j = 0; j < (D + 1) / 2; ++j)
+        pairs[(size_t)j * n_total + i] = make_uint4(row[2 * j], __float_as_uint(w[2 * j]), row[2 * j + 1],
+                                                    __float_as_uint(w[2 * j + 1]));
+    if constexpr (D % 2 == 0)
+        reinterpret_cast<uint2*>(pairs + (size_t)(D / 2) * n_total)[i] = make_uint2(row[D], __float_as_uint(w[D]));
+}
+template <int D>
+__device__ __forceinline__ void load_record(const void* rec, uint32_t n_total, uint32_t i, int (&row)[D + 1],
+                                            float (&w)[D + 1]) {
+    const uint4* pairs = reinterpret_cast<const uint4*>(rec);
+#pragma unroll
+    for (int j = 0; j < (D + 1) / 2; ++j) {
+        const uint4 q = __ldcs(pairs + (size_t)j * n_total + i);
+        row[2 * j] = (int)q.x, w[2 * j] = __uint_as_float(q.y);
+        row[2 * j + 1] = (int)q.z, w[2 * j + 1] = __uint_as_float(q.w);
+    }
+    if constexpr (D % 2 == 0) {
+        const uint2 q = __ldcs(reinterpret_cast<const uint2*>(pairs + (size_t)(D / 2) * n_total) + i);
+        row[D] = (int)q.x, w[D] = __uint_as_float(q.y);
+    }
+}
+
+// ---------------------------------------------------------------------------------
 // splat
 // ---------------------------------------------------------------------------------
 constexpr int kSplatThreads = 256;
@@ -433,7 +480,7 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     float p[D], v[VDP];
     load_point<D, VDP>(sg.src, i, p, v);
     Simplex<D> sx;
-    const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kSplatThreads};
+    const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kSplatThreads, kSplatThreads};
     compute_simplex<D>(p, a.lc, sx, status, scr);
     const uint32_t gi = sg.point_base + i;   // point number in the batch
     const uint32_t e0 = gi * (uint32_t)(D + 1);
@@ -452,7 +499,7 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     first_key<D>(sx, key);
 #pragma unroll
     for (int r = 0; r <= D; ++r) {
-        if (r > 0) key_step<D>(key, scr.coord[(D - (r - 1)) * scr.stride]);
+        if (r > 0) key_step<D>(key, scr.coord[(D - (r - 1)) * scr.coord_stride]);
         if (kKeysInSmem) s_key[r * kSplatThreads + threadIdx.x] = key.w[0];
         const uint32_t hk = key_hash<KW>(key);
         unsigned pr = __match_any_sync(active, hk);
@@ -488,6 +535,7 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     // rarely a run (on the 4K d=5 bilateral every warp has a vertex split over several
     // runs), and gathering them costs more instructions than the L2 atomics it saves.
     // Every lane records the slot for the slice.
+    uint32_t row[D + 1];
 #pragma unroll
     for (int r = 0; r <= D; ++r) {
         const unsigned pr = peers[r];
@@ -513,10 +561,10 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
         }
         s = __shfl_sync(active, s, leader);
         if (s >= 0) atomic_add_row<VDP>(vals + (size_t)s * VDP, c);
-        if (a.rec_slot)
-            a.rec_slot[(size_t)r * a.n_total + gi] = s >= 0 ? sg.slot_base + (uint32_t)s : 0xFFFFFFFFu;
-        if (a.rec_w) a.rec_w[(size_t)r * a.n_total + gi] = sx.bary[r];
+        row[r] = s >= 0 ? sg.slot_base + (uint32_t)s : 0xFFFFFFFFu;
+        if (a.rec_slot) a.rec_slot[(size_t)r * a.n_total + gi] = row[r];
     }
+    if (a.rec) store_record<D>(a.rec, a.n_total, gi, row, sx.bary);
     }
     if (!a.vlist) return;
     __syncthreads();
@@ -529,18 +577,26 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
 // Neighbouring pixels land on the same lattice vertices (on the 4K d=5 bilateral a 16x16
 // tile's 1536 (point, remainder) entries touch about 155 distinct vertices), while the
 // direct splat pays one dependent probe of the global table, a trip to L2 or DRAM, per
-// lane group.  The tile splat resolves every entry's key in a hash table of the block's
-// own in shared memory instead (phase A), inserts each distinct vertex of the tile into
-// the global table once (phase B), and then every lane adds its rows to the global slots
-// with fire-and-forget vector reductions and writes its replay record (phase C).  A local
-// slot's first touch is the smallest entry that reached it, so the global minimum over
-// tiles is the reference's first insertion; the vertex set, keys and records equal the
-// direct splat's, only the order of the FP32 additions differs.  An entry whose probe finds
-// no free local slot within kTileProbe goes to the global table directly, so no tile can
-// overflow.  One-word keys (d <= 7), FP32 accumulators.
+// lane group.  The tile splat first finds each vertex's entries within the tile, in shared
+// memory (phases A and B), inserts each distinct vertex of the tile into the global table
+// once (phase C), and then every lane adds its rows to the global rows with
+// fire-and-forget vector reductions and writes its replay record (phase D).  A vertex's first touch is
+// the smallest entry that reached it, so the global minimum over tiles is the reference's
+// first insertion; the vertex set, keys and records equal the direct splat's, only the order
+// of the FP32 additions differs.  One-word keys (d <= 7), FP32 accumulators.
+//
+// Finding equal keys takes no atomics: every entry stores its key in its own place and its
+// number in a claim table at its key's hash, whichever comes last; after a barrier it
+// reads the claim back and compares the claimant's key with its own.  Entries of one key
+// share a claim, so either all of them find the same claimant, which stands for the
+// vertex, or, where another key's entry came last, none; those (4 % of a 4K frame's
+// entries) go to a small open-addressed table.  (A block-wide compare-and-swap table
+// for all entries starts empty in every tile, so nearly every probe met contended
+// swaps: 12 shared-memory wavefronts per swap, 0.37 of the splat's 0.75 ms per 4K frame.)
 constexpr int kTileThreads = 256;
 constexpr int kTilePixels = 256;        // one pixel per thread
-constexpr int kTileSlots = 1024;        // shared-memory hash slots per block
+constexpr int kTileClaims = 4096;       // claim table entries per block (powers of two)
+constexpr int kTileSlots = 512;         // slots of the table for entries whose claim was lost
 constexpr int kTileProbe = 64;
 #ifndef PGPU_TILE_MIN_BLOCKS_D5
 #define PGPU_TILE_MIN_BLOCKS_D5 5
@@ -549,45 +605,39 @@ __host__ __device__ constexpr int tile_min_blocks(int d) {
     return d <= 5 ? PGPU_TILE_MIN_BLOCKS_D5 : d <= 6 ? 4 : 3;
 }
 
-// dynamic shared memory of a tile splat block: keys, first touches (then global slots),
-// the list of occupied slots, the slots the block creates, and the simplex scratch.  (The
-// rows are not summed in shared memory: float atomics there are compare-and-swap loops,
-// and a variant that summed each tile's rows before one global reduction per vertex took
-// 2.1 ms per 4K frame against 0.73 ms.)
-__host__ __device__ constexpr size_t tile_smem_bytes(int d, int vdp) {
-    return (size_t)kTileSlots * 16 + (size_t)kTileSlots * 4 + (size_t)kTileSlots * 2 +
-           (size_t)kBlockListCap * 4 + (size_t)kBlockListCap * 2 + (size_t)(d + 1) * kTileThreads * 4 +
-           (size_t)(d + 1) * kTileThreads + 16 + 0 * (size_t)vdp;
+// Dynamic shared memory of a tile splat block: per entry 8 bytes for the simplex scratch
+// and then the key, the claims, the lost claims' table, a row and a list place per vertex,
+// and the slots the block creates.  (The rows are not summed in shared memory: float
+// atomics there are compare-and-swap loops, and a variant that summed each tile's rows
+// before one global reduction per vertex took 2.1 ms per 4K frame against 0.73 ms.)
+__host__ __device__ constexpr size_t tile_smem_bytes(int d, int) {
+    const size_t entries = (size_t)(d + 1) * kTileThreads;
+    return entries * 8 + (size_t)kTileSlots * 8 + (entries + kTileSlots) * 4 + (size_t)kBlockListCap * 4 +
+           (size_t)kTileClaims * 2 + (entries + kTileSlots) * 2 + (size_t)kBlockListCap * 2;
 }
 
-// Home slot of a one-word key in a block's table: a cheap multiplicative mix of the three
-// 32-bit words that carry coordinates 0..5 and the low half of the fourth (coordinate 6);
-// the table is small and probing resolves its collisions, so the global hash (a 64-bit
-// mix) is computed only once per distinct vertex, in phase B.
-__device__ __forceinline__ uint32_t tile_home(const uint4& k) {
-    const uint32_t h = k.x * 0x9E3779B1u + k.y * 0x85EBCA77u + k.z * 0xC2B2AE3Du + (k.w & 0xFFFFu) * 0x27D4EB2Fu;
-    return (h ^ (h >> 15)) * 0x2C1B3C6Du >> (32 - 10);
+// Hash of a tile key (32 bits, the high ones used): a multiplicative mix of its halves; the
+// global hash (a 64-bit mix) is computed only once per distinct vertex, in phase C.
+__device__ __forceinline__ uint32_t tile_hash(uint64_t k) {
+    return (uint32_t)k * 0x9E3779B1u + (uint32_t)(k >> 32) * 0x85EBCA77u;
 }
 
-// find-or-insert of a one-word key in the block's table; a new key's slot is appended to
-// the block's list of occupied slots.  -1 when no slot within the probe limit is free (the
-// caller then uses the global table).
-__device__ __forceinline__ int tile_insert(uint4* t_key, uint16_t* t_list, uint32_t* t_count,
-                                           const uint4& k) {
-    const uint4 empty = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-    static_assert(kTileSlots == 1024, "the home slot has 10 bits");
-    uint32_t l = tile_home(k);
+// find-or-insert of a tile key in the block's small table: its slot, or -1 when no slot
+// within the probe limit is free (the caller then uses the global table)
+__device__ __forceinline__ int tile_insert(uint64_t* t_key, uint64_t k, bool* created) {
+    static_assert(kTileSlots == 512, "the home slot has 9 bits");
+    uint32_t l = (tile_hash(k) * 0x2C1B3C6Du) >> (32 - 9);
 #pragma unroll 1
     for (int probe = 0; probe < kTileProbe; ++probe) {
-        uint4 w = t_key[l];
-        if (is_empty_word(w)) {
-            w = atomicCAS_block(&t_key[l], empty, k);
-            if (is_empty_word(w)) {
-                t_list[atomicAdd(t_count, 1u)] = (uint16_t)l;
+        uint64_t w = *reinterpret_cast<const volatile uint64_t*>(t_key + l);
+        if (w == ~0ull) {
+            w = atomicCAS_block(reinterpret_cast<unsigned long long*>(t_key + l), ~0ull, k);
+            if (w == ~0ull) {
+                *created = true;
                 return (int)l;
             }
         }
-        if (words_equal(w, k)) return (int)l;
+        if (w == k) return (int)l;
         l = (l + 1) & (kTileSlots - 1);
     }
     return -1;
@@ -672,7 +722,7 @@ __device__ __forceinline__ uint32_t list_new_vertex(const SplatArgs& a, int kseg
     return v;
 }
 
-// t_ft marker of a vertex the block created and numbers in its flush (never a vertex index:
+// t_row marker of a vertex the block created and numbers in its flush (never a vertex index:
 // indices stay below the 2^31 - 256 slots of a batch)
 constexpr uint32_t kOwnPending = 0x7FFFFFFFu;
 
@@ -693,124 +743,194 @@ __device__ __forceinline__ uint32_t await_vertex(const SplatArgs& a, uint32_t s,
     return 0xFFFFFFFFu;
 }
 
-// One (point, remainder) entry of the tile splat's phase C: its weighted row into row s
-// (VROWS: vertex s; otherwise segment slot s; 0xFFFFFFFF: not placed) and its record.
-template <int D, int VDP, bool VROWS>
-__device__ __forceinline__ void splat_entry(const SplatArgs& a, float* vals, uint32_t slot_base, uint32_t gi,
-                                            int r, uint32_t s, float w, const float (&v)[VDP]) {
-    if (s != 0xFFFFFFFFu) {
-        float c[VDP];
-#pragma unroll
-        for (int q = 0; q < VDP; ++q) c[q] = __fmul_rn(w, v[q]);
-        atomic_add_row<VDP>(vals + (size_t)s * VDP, c);
-    }
-    if (a.rec_slot)
-        a.rec_slot[(size_t)r * a.n_total + gi] = s == 0xFFFFFFFFu ? 0xFFFFFFFFu : VROWS ? s : slot_base + s;
-    if (a.rec_w) a.rec_w[(size_t)r * a.n_total + gi] = w;
-}
-
 // VROWS: number vertices as they are created and accumulate into vertex-ordered rows (the
 // SplatArgs::vrows protocol, d <= 6, no first touches); otherwise rows in slot space.
 template <int D, int VDP, bool VROWS>
 __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) splat_tile_kernel(SplatArgs a) {
     static_assert(key_words(D) == 1, "the tile splat handles one-word keys (d <= 7)");
     static_assert(!VROWS || index_in_key(D), "vertex-ordered rows publish the index in the key word");
+    using K = TileKey<D>;
+    constexpr uint32_t kEntries = (D + 1) * kTileThreads;   // entry (r, thread) is r*kTileThreads + thread
     extern __shared__ __align__(16) unsigned char tile_smem[];
-    uint4* t_key = reinterpret_cast<uint4*>(tile_smem);
-    uint32_t* t_ft = reinterpret_cast<uint32_t*>(t_key + kTileSlots);
-    uint16_t* t_list = reinterpret_cast<uint16_t*>(t_ft + kTileSlots);
-    uint32_t* s_new = reinterpret_cast<uint32_t*>(t_list + kTileSlots);
-    uint16_t* s_new_l = reinterpret_cast<uint16_t*>(s_new + kBlockListCap);
-    float* s_delta = reinterpret_cast<float*>(s_new_l + kBlockListCap);
-    unsigned char* s_coord = reinterpret_cast<unsigned char*>(s_delta + (D + 1) * kTileThreads);
+    uint2* s_scr = reinterpret_cast<uint2*>(tile_smem);     // the simplex, then each entry's key
+    uint64_t* s_key = reinterpret_cast<uint64_t*>(s_scr);
+    uint64_t* t_key = s_key + kEntries;                     // the lost claims' table
+    uint32_t* t_row = reinterpret_cast<uint32_t*>(t_key + kTileSlots);   // per vertex of the tile
+    uint32_t* s_new = t_row + kEntries + kTileSlots;
+    uint16_t* s_claim = reinterpret_cast<uint16_t*>(s_new + kBlockListCap);
+    uint16_t* t_list = s_claim + kTileClaims;               // the tile's vertices
+    uint16_t* s_new_l = t_list + kEntries + kTileSlots;
     __shared__ Segment sg;
     __shared__ uint32_t t_count, s_new_count, s_new_base;
+    __shared__ int s_base[K::kRelative ? D : 1];
     const int kseg = segment_by<&Segment::tile_base>(a.segs, a.nseg, blockIdx.x);
-    for (int l = threadIdx.x; l < kTileSlots; l += kTileThreads) {
-        t_key[l] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-        t_ft[l] = 0xFFFFFFFFu;
-    }
+    for (int l = threadIdx.x; l < kTileSlots / 2; l += kTileThreads)
+        reinterpret_cast<uint4*>(t_key)[l] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+    if (!VROWS && a.ft)
+        for (int l = threadIdx.x; l < (int)kEntries + kTileSlots; l += kTileThreads) t_row[l] = 0xFFFFFFFFu;
     if (threadIdx.x == 0) t_count = 0, s_new_count = 0;
     load_segment(a.segs + kseg, sg);   // ends with a barrier
-    const BlockList blist{s_new, &s_new_count, &s_new_base};
 
     unsigned* status = a.seg_status + kseg;
     const TableView table{a.key0 + sg.slot_base, a.keyn + sg.slot_base, sg.cap, a.cap_total};
     float* vals = VROWS ? reinterpret_cast<float*>(a.vrows)
                         : reinterpret_cast<float*>(a.vals) + (size_t)sg.slot_base * VDP;
     uint32_t* ft = (!VROWS && a.ft) ? a.ft + sg.slot_base : nullptr;
-    const uint32_t b = blockIdx.x - sg.tile_base;
-    const uint32_t per_frame = sg.tiles_x * sg.tiles_y;
-    const uint32_t f = b / per_frame, bt = b - f * per_frame;
-    const uint32_t ty = bt / sg.tiles_x, tx = bt - ty * sg.tiles_x;
-    const uint32_t px = tx * sg.tile_w + threadIdx.x % sg.tile_w;
-    const uint32_t py = ty * sg.tile_h + threadIdx.x / sg.tile_w;
+    uint32_t bt, tx;
+    const uint32_t f = div_magic(blockIdx.x - sg.tile_base, sg.tiles_x * sg.tiles_y, sg.tile_fm, &bt);
+    const uint32_t ty = div_magic(bt, sg.tiles_x, sg.tile_xm, &tx);
+    const uint32_t px = (tx << sg.tile_shift) + (threadIdx.x & (sg.tile_w - 1));
+    const uint32_t py = ty * sg.tile_h + (threadIdx.x >> sg.tile_shift);
     const uint32_t W = (uint32_t)sg.src.width, H = (uint32_t)sg.src.height;
     const bool valid = px < W && py < H;
-    const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kTileThreads};
+    const uint32_t gi = sg.point_base + (f * H + py) * W + px;
+    uint2* scr = s_scr + threadIdx.x;
+    uint64_t* keys = s_key + threadIdx.x;
 
-    // Phase A: this pixel's simplex and the local slot of each of its d+1 vertices.
-    // loc[r] >= 0: local slot; -1: not placed; <= -2: global slot -(loc + 2), taken directly
-    // because the local table was full around the key.
+    // Phase A: this pixel's simplex, its keys and their claims
     float v[VDP];
     float bary[D + 1];
-    int loc[D + 1];
-    uint32_t gi = 0;
-#pragma unroll
-    for (int r = 0; r <= D; ++r) loc[r] = -1;
+    int q[D + 1];
+    bool fits = false;
+    Key<1> kk;   // the first key of a pixel whose keys do not fit tile keys
     if (valid) {
         float pp[D];
         load_point_xyt<D, VDP>(sg.src, px, py, f, pp, v);
-        Simplex<D> sx;
-        compute_simplex<D>(pp, a.lc, sx, status, scr);
-        gi = sg.point_base + (f * H + py) * W + px;
-        const uint32_t e0 = gi * (uint32_t)(D + 1);
-        Key<1> key;
-        first_key<D>(sx, key);
+        fits = tile_simplex<D>(pp, a.lc, q, scr, kTileThreads);
+    }
+    if constexpr (K::kRelative) {
+        if (threadIdx.x == 0) {   // the tile's first pixel, inside every image
+#pragma unroll
+            for (int i = 0; i < D; ++i) s_base[i] = q[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            q[i] = (int)((unsigned)q[i] - (unsigned)s_base[i]);
+            fits = fits && q[i] <= K::kMaxField && q[i] >= -K::kMaxField;
+        }
+    }
+    if (fits) {
+        float srt[D + 1];
+        uint32_t field[D + 1];
+#pragma unroll
+        for (int k = 0; k <= D; ++k) {
+            const uint2 e = scr[k * kTileThreads];
+            srt[k] = __uint_as_float(e.x);
+            field[k] = e.y;
+        }
+        // b[0] = delta(rank d) + (1 + b[d+1]),  b[d+1] = -delta(rank 0) (compute_simplex)
+        bary[0] = __fadd_rn(srt[D], __fadd_rn(1.0f, -srt[0]));
+#pragma unroll
+        for (int k = 1; k <= D; ++k) bary[k] = __fsub_rn(srt[D - k], srt[D + 1 - k]);
+        uint64_t key = tile_first_key<D>(q);
 #pragma unroll
         for (int r = 0; r <= D; ++r) {
-            if (r > 0) key_step<D>(key, scr.coord[(D - (r - 1)) * scr.stride]);
-            bary[r] = sx.bary[r];
-            const int l = tile_insert(t_key, t_list, &t_count, key.w[0]);
-            if (l >= 0) {
-                if (ft) atomicMin(&t_ft[l], e0 + (uint32_t)r);
-                loc[r] = l;
-            } else {
-                const uint32_t home = home_slot(key_hash<1>(key), table.cap);
-                bool created = false;
-                const int s = table_insert<1, VROWS>(table, key, home, __ldcg(&table.key0[home]), status, &created);
-                if (s >= 0) {
-                    if constexpr (VROWS) {
-                        // numbered by the flush (phase C reads the number from the key word)
-                        if (created)
-                            list_new_vertex<VDP>(a, kseg, s_new, s_new_l, &s_new_count,
-                                                 sg.slot_base + (uint32_t)s, 0xFFFFu, key.w[0]);
-                        loc[r] = -(s + 2);
-                    } else {
-                        if (ft) atomicMin(&ft[s], e0 + (uint32_t)r);
-                        if (created && a.vlist) block_list_append(blist, a, kseg, sg.slot_base + (uint32_t)s);
-                        loc[r] = -(s + 2);
-                    }
-                }
-            }
+            if (r > 0) key += 1ull - bit64(field[D - (r - 1)]);
+            keys[r * kTileThreads] = key;
+            s_claim[tile_hash(key) / (uint32_t)(0x100000000ull / kTileClaims)] = (uint16_t)(r * kTileThreads + threadIdx.x);
         }
+    } else if (valid) {
+        // out of a tile key's range: the general simplex, every vertex in the global table
+        float pp[D];
+        load_point_xyt<D, VDP>(sg.src, px, py, f, pp, v);
+        Simplex<D> sx;
+        const SimplexScratch gs{reinterpret_cast<float*>(scr), reinterpret_cast<unsigned char*>(scr) + 4,
+                                2 * kTileThreads, 8 * kTileThreads};
+        compute_simplex<D>(pp, a.lc, sx, status, gs);
+        first_key<D>(sx, kk);
+#pragma unroll
+        for (int r = 0; r <= D; ++r) bary[r] = sx.bary[r];
     }
     __syncthreads();
 
-    // Phase B: each distinct vertex of the tile (the list of occupied local slots) into the
-    // global table once
+    // Phase B: the vertex of each entry, by its number in the tile: that of the entry that
+    // stands for it, or kEntries + its slot in the lost claims' table.
+    // loc[r] >= 0: that number; -1: not placed; <= -2: global slot -(loc + 2), taken directly
+    // because the key does not fit a tile key or the small table was full around it.
+    int loc[D + 1];
+    uint32_t todo = 0;   // remainders to place in the global table
+    if (fits) {
+        uint32_t stands = 0;   // remainders whose entry stands for its vertex
+#pragma unroll
+        for (int r = 0; r <= D; ++r) {
+            const uint64_t key = keys[r * kTileThreads];
+            const uint32_t c = s_claim[tile_hash(key) / (uint32_t)(0x100000000ull / kTileClaims)];
+            loc[r] = (int)c;
+            if (s_key[c] != key) todo |= 1u << r;
+            else if (c == (uint32_t)r * kTileThreads + threadIdx.x) stands |= 1u << r;
+        }
+        if (stands) {
+            uint32_t j = atomicAdd(&t_count, (uint32_t)__popc(stands));
+#pragma unroll
+            for (int r = 0; r <= D; ++r)
+                if ((stands >> r) & 1u) t_list[j++] = (uint16_t)(r * kTileThreads + threadIdx.x);
+        }
+#pragma unroll
+        for (int r = 0; r <= D; ++r) {
+            if (!((todo >> r) & 1u)) continue;
+            bool created = false;
+            const int l = tile_insert(t_key, keys[r * kTileThreads], &created);
+            if (l < 0) continue;
+            loc[r] = (int)kEntries + l;
+            todo &= ~(1u << r);
+            if (created) t_list[atomicAdd(&t_count, 1u)] = (uint16_t)(kEntries + l);
+        }
+        if (ft) {
+#pragma unroll
+            for (int r = 0; r <= D; ++r)
+                if (!((todo >> r) & 1u)) atomicMin(&t_row[loc[r]], gi * (uint32_t)(D + 1) + (uint32_t)r);
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r <= D; ++r) loc[r] = -1;
+        if (valid) todo = (1u << (D + 1)) - 1u;
+    }
+    if (todo) {
+        // rare: rolled, with the results in the scratch (no other thread reads these entries:
+        // they stand for no vertex)
+#pragma unroll 1
+        for (int r = 0; r <= D; ++r) {
+            if (!fits && r > 0) key_step<D>(kk, (int)(scr[(D - (r - 1)) * kTileThreads].y & 0xFFu));
+            if (!((todo >> r) & 1u)) continue;
+            Key<1> key = kk;
+            if (fits) tile_full_key<D>(keys[r * kTileThreads], s_base, key);
+            const uint32_t home = home_slot(key_hash<1>(key), table.cap);
+            bool created = false;
+            const int s = table_insert<1, VROWS>(table, key, home, __ldcg(&table.key0[home]), status, &created);
+            if (s >= 0) {
+                if constexpr (VROWS) {   // numbered by the flush; phase D reads the key word
+                    if (created)
+                        list_new_vertex<VDP>(a, kseg, s_new, s_new_l, &s_new_count, sg.slot_base + (uint32_t)s,
+                                             0xFFFFu, key.w[0]);
+                } else {
+                    if (ft) atomicMin(&ft[s], gi * (uint32_t)(D + 1) + (uint32_t)r);
+                    if (created && a.vlist)
+                        block_list_append(BlockList{s_new, &s_new_count, &s_new_base}, a, kseg,
+                                          sg.slot_base + (uint32_t)s);
+                }
+            }
+            scr[r * kTileThreads].x = (uint32_t)(s >= 0 ? -(s + 2) : -1);
+        }
+#pragma unroll
+        for (int r = 0; r <= D; ++r)
+            if ((todo >> r) & 1u) loc[r] = (int)scr[r * kTileThreads].x;
+    }
+    __syncthreads();
+
+    // Phase C: each distinct vertex of the tile into the global table once
     const uint32_t count = t_count;
 #pragma unroll 1
     for (uint32_t j = threadIdx.x; j < count; j += kTileThreads) {
         const int l = t_list[j];
-        Key<1> kk;
-        kk.w[0] = t_key[l];
-        const uint32_t h = home_slot(key_hash<1>(kk), table.cap);
+        Key<1> key;
+        tile_full_key<D>(s_key[l], s_base, key);   // the small table's keys follow the entries'
+        const uint32_t h = home_slot(key_hash<1>(key), table.cap);
         bool created = false;
         uint4 seen = make_uint4(0u, 0u, 0u, 0u);
-        const int s = table_insert<1, VROWS>(table, kk, h, __ldcg(&table.key0[h]), status, &created, &seen);
+        const int s = table_insert<1, VROWS>(table, key, h, __ldcg(&table.key0[h]), status, &created, &seen);
         if constexpr (VROWS) {
-            // t_ft[l]: the vertex index; kOwnPending for a vertex this block numbers in its
+            // t_row[l]: the vertex index; kOwnPending for a vertex this block numbers in its
             // flush; 0x80000000 | global slot while another block's vertex is not numbered
             uint32_t val = 0xFFFFFFFFu;
             if (s >= 0) {
@@ -818,24 +938,25 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) splat_tile_k
                 val = 0x80000000u | gs;
                 if (created) {
                     const uint32_t vv = list_new_vertex<VDP>(a, kseg, s_new, s_new_l, &s_new_count, gs,
-                                                             (uint16_t)l, kk.w[0]);
+                                                             (uint16_t)l, key.w[0]);
                     val = vv != 0xFFFFFFFFu ? vv : kOwnPending;
                 } else if (has_index(seen.w)) {
                     val = dec_index(seen.w);
                 }
             }
-            t_ft[l] = val;
+            t_row[l] = val;
         } else {
-            if (s >= 0 && ft) atomicMin(&ft[s], t_ft[l]);
-            if (created && a.vlist) block_list_append(blist, a, kseg, sg.slot_base + (uint32_t)s);
-            t_ft[l] = s >= 0 ? (uint32_t)s : 0xFFFFFFFFu;   // now the global slot (segment-relative)
+            if (s >= 0 && ft) atomicMin(&ft[s], t_row[l]);
+            if (created && a.vlist)
+                block_list_append(BlockList{s_new, &s_new_count, &s_new_base}, a, kseg, sg.slot_base + (uint32_t)s);
+            t_row[l] = s >= 0 ? (uint32_t)s : 0xFFFFFFFFu;   // the global slot (segment-relative)
         }
     }
     __syncthreads();
     if constexpr (VROWS) {
         // number the block's new vertices with one atomic and publish them; in the same
         // pass, learn (once per vertex) the numbers of the tile's vertices other blocks
-        // created, which is faster than every lane waiting for its own entries in phase C
+        // created, which is faster than every lane waiting for its own entries in phase D
         const uint32_t n = min(s_new_count, kBlockListCap);
         if (n) {
             if (threadIdx.x == 0) {
@@ -848,39 +969,50 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) splat_tile_k
         for (uint32_t jj = threadIdx.x; jj < n; jj += kTileThreads) {
             const int l = s_new_l[jj];
             if (l != 0xFFFF) {
-                publish_vertex<VDP>(a, s_new[jj], base + jj, t_key[l]);
-                t_ft[l] = base + jj;
-            } else {   // placed in the global table directly in phase A
+                Key<1> key;
+                tile_full_key<D>(s_key[l], s_base, key);
+                publish_vertex<VDP>(a, s_new[jj], base + jj, key.w[0]);
+                t_row[l] = base + jj;
+            } else {   // placed in the global table directly in phase B
                 publish_vertex<VDP>(a, s_new[jj], base + jj, __ldcg(&a.key0[s_new[jj]]));
             }
         }
 #pragma unroll 1
         for (uint32_t j = threadIdx.x; j < count; j += kTileThreads) {
             const int l = t_list[j];
-            const uint32_t val = t_ft[l];
-            if (val != 0xFFFFFFFFu && (val & 0x80000000u)) t_ft[l] = await_vertex(a, val & 0x7FFFFFFFu, status);
+            const uint32_t val = t_row[l];
+            if (val != 0xFFFFFFFFu && (val & 0x80000000u)) t_row[l] = await_vertex(a, val & 0x7FFFFFFFu, status);
         }
         __syncthreads();
     } else {
-        if (a.vlist) block_list_flush(blist, a, kseg);
+        if (a.vlist) block_list_flush(BlockList{s_new, &s_new_count, &s_new_base}, a, kseg);
     }
 
-    // Phase C: every lane's rows into its vertices' global rows, and the replay record
+    // Phase D: every lane's rows into its vertices' global rows (VROWS: by vertex index;
+    // otherwise segment slots; 0xFFFFFFFF: not placed), and the replay record
     if (!valid) return;
+    uint32_t row[D + 1];
 #pragma unroll
     for (int r = 0; r <= D; ++r) {
         const int l = loc[r];
-        uint32_t s;
+        uint32_t s = 0xFFFFFFFFu;
         if (l >= 0) {
-            s = t_ft[l];
+            s = t_row[l];
         } else if (l <= -2) {
             s = (uint32_t)(-(l + 2));
             if constexpr (VROWS) s = await_vertex(a, sg.slot_base + s, status);
-        } else {
-            s = 0xFFFFFFFFu;
         }
-        splat_entry<D, VDP, VROWS>(a, vals, sg.slot_base, gi, r, s, bary[r], v);
+        if (s != 0xFFFFFFFFu) {
+            float c[VDP];
+#pragma unroll
+            for (int k = 0; k < VDP; ++k) c[k] = __fmul_rn(bary[r], v[k]);
+            atomic_add_row<VDP>(vals + (size_t)s * VDP, c);
+            if (!VROWS) s += sg.slot_base;
+        }
+        row[r] = s;
+        if (a.rec_slot) a.rec_slot[(size_t)r * a.n_total + gi] = s;
     }
+    if (a.rec) store_record<D>(a.rec, a.n_total, gi, row, bary);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1278,12 +1410,11 @@ __global__ void __launch_bounds__(kSliceThreads, slice_min_blocks(D)) slice_kern
     load_segment(a.segs + kseg, sg);
     // a block is a slice_tw x slice_th tile of one frame: neighbouring pixels gather the
     // same vertex rows, which then come from L1
-    const uint32_t b = blockIdx.x - sg.block_base;
-    const uint32_t per_frame = sg.stiles_x * sg.stiles_y;
-    const uint32_t fr = b / per_frame, bt = b - fr * per_frame;
-    const uint32_t ty = bt / sg.stiles_x, tx = bt - ty * sg.stiles_x;
-    const uint32_t px = tx * sg.slice_tw + threadIdx.x % sg.slice_tw;
-    const uint32_t py = ty * sg.slice_th + threadIdx.x / sg.slice_tw;
+    uint32_t bt, tx;
+    const uint32_t fr = div_magic(blockIdx.x - sg.block_base, sg.stiles_x * sg.stiles_y, sg.stile_fm, &bt);
+    const uint32_t ty = div_magic(bt, sg.stiles_x, sg.stile_xm, &tx);
+    const uint32_t px = (tx << sg.slice_shift) + (threadIdx.x & (sg.slice_tw - 1));
+    const uint32_t py = ty * sg.slice_th + (threadIdx.x >> sg.slice_shift);
     if (px >= (uint32_t)sg.src.width || py >= (uint32_t)sg.src.height) return;
     const uint32_t i = (fr * (uint32_t)sg.src.height + py) * (uint32_t)sg.src.width + px;
     unsigned* status = a.seg_status + kseg;
@@ -1294,7 +1425,7 @@ __global__ void __launch_bounds__(kSliceThreads, slice_min_blocks(D)) slice_kern
     float p[D];
     load_position<D>(sg.src, i, p);
     Simplex<D> sx;
-    const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kSliceThreads};
+    const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kSliceThreads, kSliceThreads};
     compute_simplex<D>(p, a.lc, sx, status, scr);
     const A* sv = reinterpret_cast<const A*>(a.svals);
     A acc[VDP];
@@ -1328,7 +1459,7 @@ __global__ void __launch_bounds__(kSliceThreads, slice_min_blocks(D)) slice_kern
         if (a.rec_slot) {
             s = (int)__ldg(a.rec_slot + (size_t)r * a.n_total + gi);
         } else {
-            if (r > 0) key_step<D>(key, scr.coord[(D - (r - 1)) * scr.stride]);
+            if (r > 0) key_step<D>(key, scr.coord[(D - (r - 1)) * scr.coord_stride]);
             const TableView table{a.key0 + sg.slot_base, a.keyn + sg.slot_base, sg.cap, a.cap_total};
             const int ls = table_find<D>(table, key, key_hash<KW>(key));
             s = ls >= 0 ? (int)sg.slot_base + ls : -1;
@@ -1373,12 +1504,11 @@ __global__ void __launch_bounds__(kSliceThreads) slice_replay_kernel(SliceArgs a
     __shared__ Segment sg;
     const int kseg = segment_of_block(a.segs, a.nseg, blockIdx.x);
     load_segment(a.segs + kseg, sg);
-    const uint32_t b = blockIdx.x - sg.block_base;
-    const uint32_t per_frame = sg.stiles_x * sg.stiles_y;
-    const uint32_t fr = b / per_frame, bt = b - fr * per_frame;
-    const uint32_t ty = bt / sg.stiles_x, tx = bt - ty * sg.stiles_x;
-    const uint32_t px = tx * sg.slice_tw + threadIdx.x % sg.slice_tw;
-    const uint32_t py = ty * sg.slice_th + threadIdx.x / sg.slice_tw;
+    uint32_t bt, tx;
+    const uint32_t fr = div_magic(blockIdx.x - sg.block_base, sg.stiles_x * sg.stiles_y, sg.stile_fm, &bt);
+    const uint32_t ty = div_magic(bt, sg.stiles_x, sg.stile_xm, &tx);
+    const uint32_t px = (tx << sg.slice_shift) + (threadIdx.x & (sg.slice_tw - 1));
+    const uint32_t py = ty * sg.slice_th + (threadIdx.x >> sg.slice_shift);
     const uint32_t W = (uint32_t)sg.src.width, H = (uint32_t)sg.src.height;
     if (px >= W || py >= H) return;
     // an image whose splat overflowed its table is rerun by the host; write nothing
@@ -1387,11 +1517,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_replay_kernel(SliceArgs a
     const A* sv = reinterpret_cast<const A*>(a.svals);
     int sl[D + 1];
     float w[D + 1];
-#pragma unroll
-    for (int r = 0; r <= D; ++r) {
-        sl[r] = (int)__ldcs(a.rec_slot + (size_t)r * a.n_total + gi);
-        w[r] = __ldcs(a.rec_w_in + (size_t)r * a.n_total + gi);
-    }
+    load_record<D>(a.rec, a.n_total, gi, sl, w);
     A acc[VDP];
 #pragma unroll
     for (int k = 0; k < VDP; ++k) acc[k] = (A)0;

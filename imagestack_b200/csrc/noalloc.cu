@@ -193,7 +193,7 @@ extern "C" int pgpu_bilateral_noalloc(const float* d_in, float* d_out, int width
     sa.seg_status = dstatus;
     sa.blocks = splat_blocks;
     sa.tile_blocks = 0;
-    sa.rec_w = nullptr;   // the slice recomputes the weights
+    sa.rec = nullptr;     // the slice recomputes the weights
     sa.vlist = nullptr;   // vertices numbered by first touch (mark, scan, assign below)
     sa.vcount = nullptr;
     sa.seg_counts = nullptr;

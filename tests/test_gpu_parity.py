@@ -391,3 +391,23 @@ def test_both_splat_kernels_match_the_oracle_on_images(gpu, monkeypatch, mode, w
     ref = oracle.oracle_lattice(pos, val).out
     norm = (ref[:, :c] / ref[:, c:c + 1]).reshape(h, w, c).transpose(2, 0, 1)
     assert rel_err(out, norm) <= RTOL_FP32
+
+
+@pytest.mark.parametrize("mode", ["direct", "tile"])
+@pytest.mark.parametrize("d,offset", [(1, 9000.0), (4, 5000.0), (5, 5000.0), (6, 2000.0), (7, 1500.0)])
+def test_positions_far_from_the_origin(gpu, monkeypatch, mode, d, offset):
+    """Some points near the origin and some thousands of sigmas away (still within the
+    reference's int16 keys): keys, vertex order and replay records bit for bit, whatever
+    form a kernel keeps its keys in."""
+    monkeypatch.setenv("PGPU_SPLAT", mode)
+    rng = np.random.default_rng(d)
+    pos = np.cumsum(rng.uniform(-0.2, 0.3, (700, d)), 0).astype(np.float32)
+    pos[200:300, d - 1] += offset
+    pos[300:400, 0] -= offset
+    val = rng.uniform(0, 1, (700, 3)).astype(np.float32)
+    ref = oracle.oracle_lattice(pos, val)
+    got = gpu.lattice_dump(pos, val)
+    for k in ("keys", "replay_vtx", "replay_w"):
+        np.testing.assert_array_equal(got[k], getattr(ref, k))
+    for k in ("splat", "blur", "out"):
+        assert rel_err(got[k], getattr(ref, k)) <= RTOL_FP32
