@@ -14,6 +14,7 @@
 #include <cstring>
 #include <string>
 #include <unordered_map>
+#include <unordered_set>
 #include <vector>
 
 #include "engine.h"
@@ -71,7 +72,7 @@ void Engine::shutdown() {
     if (hmeta) cudaFreeHost(hmeta);
     hmeta = nullptr;
     hmeta_bytes = 0;
-    for (DevBuf* b : {&key0, &keyn, &tvals, &ft, &slot2vtx, &bitmap, &offs, &partials, &vkey0, &vkeyn,
+    for (DevBuf* b : {&key0, &keyn, &tvals, &ft, &slot2vtx, &bitmap, &offs, &partials, &vkey, &vkey0, &vkeyn,
                       &vv0, &vv1, &nbr, &vf32, &vtx2slot, &sval, &rec, &grid, &grid2, &tags, &vlist, &dstat, &meta, &img_a, &img_b,
                       &img_c, &img_d})
         b->release();
@@ -88,6 +89,16 @@ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 std::mutex g_ratio_mu;
 std::unordered_map<uint64_t, double> g_ratio_by_sig;
 std::map<int, double> g_ratio;
+// signatures of images whose keys did not fit compact keys: their later lattices start on
+// int16-lane keys (a wrong entry costs time, not results)
+std::unordered_set<uint64_t> g_wide_sigs;
+
+// Lattices on int16-lane keys: asked for (a rerun), FP64 accumulators, PGPU_KEYS=wide in the
+// environment (tests), or an image known not to fit
+bool wide_forced(const BatchJob& B) {
+    const char* mode = std::getenv("PGPU_KEYS");
+    return B.wide || B.payload == kPayloadF64 || (mode && !strcmp(mode, "wide"));
+}
 
 inline uint64_t mix64(uint64_t h, uint64_t v) {
     h ^= v + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
@@ -130,12 +141,20 @@ void learned_ratios(const BatchJob& B, std::vector<uint64_t>* sig, std::vector<d
     }
 }
 
-// Splat kernel per lattice: the tile splat (shared-memory table per 16x16 tile) where
+// whether each image is known not to fit compact keys
+std::vector<char> known_wide(const std::vector<uint64_t>& sig) {
+    std::vector<char> w(sig.size(), 0);
+    std::lock_guard<std::mutex> lk(g_ratio_mu);
+    if (!g_wide_sigs.empty())
+        for (size_t k = 0; k < sig.size(); ++k) w[k] = g_wide_sigs.count(sig[k]) ? 1 : 0;
+    return w;
+}
+
+// Splat kernel per lattice: the tile splat (vertices found per 8x8 pixels first) where
 // neighbouring points share vertices, which the learned vertices-per-point ratio tells
-// (4K d=5 bilateral: 0.18; a 16x16 tile then holds about 155 of its 1536 entries'
-// vertices); the direct splat for sparse lattices (ratio above kTileRatioMax: measured
-// on the mixed batch, 1.5 beats 0.8 by 2 % and 0.4 by 3 %), multi-word keys and FP64
-// accumulators.  With nothing learned yet for the image or its d, the tile splat.
+// (4K d=5 bilateral: 0.18); the direct splat for sparse lattices (ratio above
+// kTileRatioMax: measured on the mixed batch, 1.5 beats 0.8 by 2 % and 0.4 by 3 %), keys of
+// 128 bits and int16-lane keys.  With nothing learned yet for the image or its d, the tile splat.
 // PGPU_SPLAT=direct or =tile in the environment overrides the choice where both exist
 // (the parity tests compare the two).
 #ifndef PGPU_TILE_RATIO_MAX
@@ -148,8 +167,8 @@ int splat_forced() {
     return !mode ? 0 : !strcmp(mode, "direct") ? 1 : !strcmp(mode, "tile") ? 2 : 0;
 }
 
-bool tile_splat_for(const BatchJob& B, int forced, double density, uint32_t n) {
-    const bool tile_ok = key_words(B.d) == 1 && B.payload != kPayloadF64 && forced != 1 &&
+bool tile_splat_for(const BatchJob& B, bool wide, int forced, double density, uint32_t n) {
+    const bool tile_ok = key_words(B.d) == 1 && !wide && forced != 1 &&
                          (forced == 2 || B.splat == 0);
     return tile_ok && (forced == 2 || (density <= kTileRatioMax && n >= 256));
 }
@@ -162,8 +181,7 @@ bool vertex_rows_wanted(const BatchJob& B) {
                     : rows_mode && !strcmp(rows_mode, "slot")   ? false
                                                                 : !B.slot_rows;
     const bool dumps = B.rec_vtx || B.dump_splat;
-    return want && !dumps && B.replay && key_words(B.d) == 1 && index_in_key(B.d) &&
-           B.payload != kPayloadF64;
+    return want && !dumps && B.replay && B.d <= 6 && !wide_forced(B);
 }
 
 // device (and pinned host) metadata of one batch
@@ -199,8 +217,6 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     if (nseg == 0) return PGPU_OK;
     const DimOps* ops = dim_ops(d);
     if (!ops) return fail(PGPU_ERR_UNSUPPORTED, "%d position dimensions (supported: 1..%d)", d, kMaxD);
-    if (!ops->prepare())
-        return fail(PGPU_ERR_CUDA, "tile splat set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
     const int vdp = vdp_for(vd);
     if (!vdp) return fail(PGPU_ERR_UNSUPPORTED, "%d value channels (supported: 1..8)", vd);
     if (B.payload < 0 || B.payload > 3) return fail(PGPU_ERR_ARGUMENT, "unknown payload %d", B.payload);
@@ -217,7 +233,6 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     // lower d most neighbours exist and the table fits in L2, where the tag is one more
     // dependent load (4K d=5: neighbours 0.18 -> 0.23 ms with tags; 2M points d=16:
     // 25.8 -> 20.5 ms).
-    const bool use_tags = kw > 1;
     const bool graph = B.use_graph && !dumps;
     // Vertices are numbered in the reference's first-insertion order only for parity dumps
     // (first touches, a bitmap and its prefix popcount); otherwise in the order the splat
@@ -248,6 +263,10 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     std::vector<uint64_t> sig;
     std::vector<double> ratio, density;
     learned_ratios(B, &sig, &ratio, &density);
+    bool wide = wide_forced(B);
+    for (char w : known_wide(sig)) wide = wide || w;
+    const bool use_tags = wide && kw > 1;
+    const int kb = compact_key_bytes(d);
     std::vector<uint64_t> cap(nseg);
     for (int k = 0; k < nseg; ++k) {
         if (cap_in) {
@@ -274,10 +293,10 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
         sgm.out = it.out;
         sgm.n = it.n;
         sgm.point_base = pbase[k];
-        const bool tiled = tile_splat_for(B, forced, density[k], it.n);
+        const bool tiled = tile_splat_for(B, wide, forced, density[k], it.n);
         uint32_t nb_splat = 0, nb_tile = 0, nb_slice = 0;
         segment_geometry(sgm, B.replay ? it.splat : it.slice, tiled, &nb_splat, &nb_tile, &nb_slice,
-                         (uint32_t)B.tile_w);
+                         wide ? kSplatThreads : kDirectThreads, (uint32_t)B.tile_w);
         tiled_count += tiled ? 1 : 0;
         sgm.splat_base = (uint32_t)blocks;
         sgm.tile_base = (uint32_t)tile_blocks;
@@ -297,13 +316,12 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
         return fail(PGPU_ERR_UNSUPPORTED, "too many points for one batch (%llu)",
                     (unsigned long long)n_total);
 
-    // Vertex-ordered rows: where every image takes the tile splat with one-word keys that
-    // hold their vertex index (d <= 6) and the slice replays the splat points, the splat
-    // numbers the vertices as it creates them and accumulates straight into
-    // vertex-ordered FP32 rows, so no compaction runs; the first blur pass reads those
+    // Vertex-ordered rows: where every image takes the tile splat (d <= 6) and the slice
+    // replays the splat points, the splat can number the vertices before it adds rows and
+    // accumulate straight into vertex-ordered FP32 rows; the first blur pass reads those
     // rows (16-bit payloads: FP32 rows, homogeneous ones normalised by the neighbour
     // search, once per vertex) and the slice reads rows by vertex index.
-    const bool vrows = vertex_rows_wanted(B) && tiled_count == nseg;
+    const bool vrows = vertex_rows_wanted(B) && !wide && tiled_count == nseg;
     // PGPU_BLUR=pairs or =single in the environment overrides the blur pairing (tests)
     const char* blur_mode = std::getenv("PGPU_BLUR");
     const bool blur_pairs = blur_mode && !strcmp(blur_mode, "pairs") ? true
@@ -332,15 +350,18 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
         sbase[nseg] = cap_total;
         if (cap_total > 0x7FFFFF00ull) return fail(PGPU_ERR_CAPACITY, "batch needs more than 2^31 hash slots");
 
-        if ((rc = E.key0.ensure(cap_total * 16)) || (rc = E.keyn.ensure((kw - 1) * cap_total * 16)) ||
-            (rc = E.tvals.ensure(cap_total * vdp * accb)) ||
+        if ((rc = E.key0.ensure(cap_total * (wide ? 16 : kb))) ||
+            (rc = E.keyn.ensure(wide ? (kw - 1) * cap_total * 16 : 0)) ||
+            (!vrows && (rc = E.tvals.ensure(cap_total * vdp * accb))) ||
             (rc = E.slot2vtx.ensure(cap_total * 4)) ||
             (exact_order && (rc = E.ft.ensure(cap_total * 4))) ||
             (exact_order && (rc = E.bitmap.ensure((size_t)nwords * 4))) ||
             (exact_order && (rc = E.offs.ensure((size_t)nwords * 4))) ||
             (exact_order && (rc = E.partials.ensure((size_t)scan_parts(nwords) * 4 + 16))) ||
-            (!exact_order && (rc = E.vlist.ensure(cap_total * 4))) ||
-            (rc = E.vkey0.ensure(cap_total * 16)) || (rc = E.vkeyn.ensure((kw - 1) * cap_total * 16)) ||
+            (wide && !exact_order && (rc = E.vlist.ensure(cap_total * 4))) ||
+            (!wide && (rc = E.vkey.ensure(cap_total * kb))) ||
+            ((wide || dumps) && (rc = E.vkey0.ensure(cap_total * 16))) ||
+            ((wide || dumps) && (rc = E.vkeyn.ensure((kw - 1) * cap_total * 16))) ||
             (rc = E.vv0.ensure(cap_total * vdp * payb)) || (rc = E.vv1.ensure(cap_total * vdp * payb)) ||
             (rc = E.nbr.ensure((size_t)(d + 1) * cap_total * 8)) ||
             ((homog || payb == 2) && (rc = E.vf32.ensure(cap_total * vdp * 4))) ||
@@ -372,15 +393,17 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
 
         unsigned char* dmeta = (unsigned char*)E.meta.p;
         uint32_t* dM = (uint32_t*)dmeta + 1;
+        // where the splat accumulates
+        void* rows0 = !vrows ? E.tvals.p : (homog || f32_rows) ? E.vf32.p : E.vv0.p;
         auto enqueue = [&](bool timed) -> int {
             // the lattice's time (and so the autotuner's) includes clearing its tables
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[6], st));
             CUDA_TRY(cudaMemcpyAsync(dmeta + L.slotbase, h + L.slotbase, L.total - L.slotbase,
                                      cudaMemcpyHostToDevice, st));
             CUDA_TRY(cudaMemsetAsync(dmeta, 0, L.slotbase, st));
-            CUDA_TRY(cudaMemsetAsync(E.key0.p, 0xFF, cap_total * 16, st));
-            if (!vrows) CUDA_TRY(cudaMemsetAsync(E.tvals.p, 0, cap_total * vdp * accb, st));
-            else CUDA_TRY(cudaMemsetAsync((homog || f32_rows) ? E.vf32.p : E.vv0.p, 0, cap_total * vdp * 4, st));
+            CUDA_TRY(cudaMemsetAsync(E.key0.p, 0xFF, cap_total * (wide ? 16 : kb), st));
+            CUDA_TRY(cudaMemsetAsync(rows0, 0, cap_total * vdp * accb, st));
+            if (vrows) CUDA_TRY(cudaMemsetAsync(E.slot2vtx.p, 0xFF, cap_total * 4, st));
             if (exact_order) {
                 CUDA_TRY(cudaMemsetAsync(E.ft.p, 0xFF, cap_total * 4, st));
                 CUDA_TRY(cudaMemsetAsync(E.bitmap.p, 0, (size_t)nwords * 4, st));
@@ -388,6 +411,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             if (use_tags) CUDA_TRY(cudaMemsetAsync(E.tags.p, 0, cap_total, st));
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[0], st));
 
+            if (wide) {
             SplatArgs sa;
             sa.segs = (const Segment*)(dmeta + L.segs);
             sa.nseg = nseg;
@@ -398,27 +422,38 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sa.cap_total = (uint32_t)cap_total;
             sa.vals = E.tvals.p;
             sa.ft = exact_order ? (uint32_t*)E.ft.p : nullptr;
-            sa.vlist = (exact_order || vrows) ? nullptr : (uint32_t*)E.vlist.p;
-            if (vrows) {
-                sa.vrows = (homog || f32_rows) ? E.vf32.p : E.vv0.p;
-                sa.vkey0 = (uint4*)E.vkey0.p;
-                sa.vtx2slot = (uint32_t*)E.vtx2slot.p;
-                if (nbr_half) {
-                    sa.nbr_init = (int2*)E.nbr.p;
-                    sa.nbr_stride = (uint32_t)cap_total;
-                    sa.nbr_axes = d + 1;
-                }
-            }
+            sa.vlist = exact_order ? nullptr : (uint32_t*)E.vlist.p;
             sa.vcount = dM;
             sa.seg_counts = (uint32_t*)(dmeta + L.counts);
             sa.rec_slot = B.replay && !replay_w ? (uint32_t*)E.rec.p : nullptr;
             sa.rec = replay_w ? E.rec.p : nullptr;
             sa.seg_status = (unsigned*)(dmeta + L.segstat);
             sa.blocks = (uint32_t)blocks;
-            sa.tile_blocks = (uint32_t)tile_blocks;
             if (!ops->splat(sa, vdp, B.payload, st)) return fail(PGPU_ERR_UNSUPPORTED, "splat variant");
-            CUDA_TRY(cudaGetLastError());
-            if (!ops->splat_tile(sa, vdp, B.payload, st)) return fail(PGPU_ERR_UNSUPPORTED, "tile splat variant");
+            } else {
+            CompactSplatArgs sa;
+            sa.segs = (const Segment*)(dmeta + L.segs);
+            sa.nseg = nseg;
+            sa.n_total = (uint32_t)n_total;
+            sa.lc = lc;
+            sa.keys = E.key0.p;
+            sa.rows = rows0;
+            sa.ft = exact_order ? (uint32_t*)E.ft.p : nullptr;
+            sa.rec_slot = B.replay && !replay_w ? (uint32_t*)E.rec.p : nullptr;
+            sa.rec = replay_w ? E.rec.p : nullptr;
+            sa.seg_status = (unsigned*)(dmeta + L.segstat);
+            sa.blocks = (uint32_t)blocks;
+            sa.tile_blocks = (uint32_t)tile_blocks;
+            sa.vcount = exact_order ? nullptr : dM;
+            sa.seg_counts = (uint32_t*)(dmeta + L.counts);
+            sa.vkey = E.vkey.p;
+            sa.vtx2slot = (uint32_t*)E.vtx2slot.p;
+            sa.slot2vtx = (uint32_t*)E.slot2vtx.p;
+            sa.nbr_init = nbr_half ? (int2*)E.nbr.p : nullptr;
+            sa.nbr_stride = (uint32_t)cap_total;
+            sa.number_rows = vrows ? 1 : 0;
+            if (!ops->compact_splat(sa, vdp, st)) return fail(PGPU_ERR_UNSUPPORTED, "splat variant");
+            }
             CUDA_TRY(cudaGetLastError());
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[1], st));
 
@@ -430,9 +465,9 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
                                       (const uint32_t*)(dmeta + L.entry), nseg,
                                       (uint32_t*)(dmeta + L.counts), st);
             }
+            if (wide) {
             CompactArgs ca;
             memset(&ca, 0, sizeof(ca));
-            if (!vrows) {
             ca.table = TableView{(uint4*)E.key0.p, (uint4*)E.keyn.p, (uint32_t)cap_total, (uint32_t)cap_total};
             ca.ft = (const uint32_t*)E.ft.p;
             ca.bitmap = (uint32_t*)E.bitmap.p;
@@ -457,14 +492,27 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             }
             if (!launch_assign(ca, kw, vdp, B.payload, homog, E.sms, st))
                 return fail(PGPU_ERR_UNSUPPORTED, "assign variant");
-            CUDA_TRY(cudaGetLastError());
+            } else if (exact_order) {
+                CompactRankArgs ra;
+                ra.keys = E.key0.p;
+                ra.cap = (uint32_t)cap_total;
+                ra.ft = (const uint32_t*)E.ft.p;
+                ra.bitmap = (const uint32_t*)E.bitmap.p;
+                ra.offs = (const uint32_t*)E.offs.p;
+                ra.vkey = E.vkey.p;
+                ra.vtx2slot = (uint32_t*)E.vtx2slot.p;
+                ra.slot2vtx = (uint32_t*)E.slot2vtx.p;
+                ra.nbr_init = nbr_half ? (int2*)E.nbr.p : nullptr;
+                ra.nbr_stride = (uint32_t)cap_total;
+                ra.wide0 = (uint4*)E.vkey0.p;
+                ra.widen = (uint4*)E.vkeyn.p;
+                ra.wide_stride = (uint32_t)cap_total;
+                ops->compact_rank(ra, E.sms, st);
             }
-            if (B.dump_splat)
-                CUDA_TRY(cudaMemcpyAsync(B.dump_splat, E.vv0.p,
-                                         std::min<size_t>(cap_total * vdp * payb, B.dump_bytes),
-                                         cudaMemcpyDeviceToDevice, st));
+            CUDA_TRY(cudaGetLastError());
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[2], st));
 
+            if (wide) {
             NbrArgs na;
             na.key0 = (uint4*)E.key0.p;
             na.keyn = (uint4*)E.keyn.p;
@@ -481,13 +529,36 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             na.tags = use_tags ? (const uint8_t*)E.tags.p : nullptr;
             na.seg_status = (const unsigned*)(dmeta + L.segstat);
             na.half = nbr_half ? 1 : 0;
-            if (vrows && homog) {   // the splat's sums, normalised once per vertex here
-                na.norm_rows = (float*)E.vf32.p;
-                na.vdp = vdp;
-                na.wc = vd - 1;
-            }
             ops->neighbours(na, (uint32_t)cap_total, E.sms, st);
+            } else {
+            CompactNbrArgs na;
+            na.keys = E.key0.p;
+            na.segs = (const Segment*)(dmeta + L.segs);
+            na.nseg = nseg;
+            na.seg_slot_base = (const uint32_t*)(dmeta + L.slotbase);
+            na.seg_status = (const unsigned*)(dmeta + L.segstat);
+            na.vkey = E.vkey.p;
+            na.vtx2slot = (const uint32_t*)E.vtx2slot.p;
+            na.slot2vtx = (const uint32_t*)E.slot2vtx.p;
+            na.nverts = dM;
+            na.nbr = (int2*)E.nbr.p;
+            na.stride = (uint32_t)cap_total;
+            na.half = nbr_half ? 1 : 0;
+            // the splat's slot rows go to vertex order here; vertex-ordered homogeneous rows
+            // are only normalised
+            na.gather = vrows ? kRowsInPlace : homog ? kRowsNormalise : B.payload == kPayloadF16 ? kRowsHalf
+                        : B.payload == kPayloadBF16 ? kRowsBf16 : kRowsCopy;
+            na.rows_in = !vrows ? (const float*)E.tvals.p : homog ? (const float*)E.vf32.p : nullptr;
+            na.rows_out = homog ? E.vf32.p : E.vv0.p;
+            na.vdp = vdp;
+            na.wc = vd - 1;
+            ops->compact_neighbours(na, (uint32_t)cap_total, E.sms, st);
+            }
             CUDA_TRY(cudaGetLastError());
+            if (B.dump_splat)
+                CUDA_TRY(cudaMemcpyAsync(B.dump_splat, E.vv0.p,
+                                         std::min<size_t>(cap_total * vdp * payb, B.dump_bytes),
+                                         cudaMemcpyDeviceToDevice, st));
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[3], st));
 
             BlurPlan bp;
@@ -514,6 +585,18 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             CUDA_TRY(cudaGetLastError());
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[4], st));
 
+            if (!wide && !B.replay) {
+            CompactSliceArgs sl;
+            sl.segs = (const Segment*)(dmeta + L.slsegs);
+            sl.nseg = nseg;
+            sl.lc = lc;
+            sl.keys = E.key0.p;
+            sl.rows = (const float*)E.sval.p;
+            sl.vd = vd;
+            sl.seg_status = (unsigned*)(dmeta + L.segstat);
+            sl.blocks = (uint32_t)slice_blocks;
+            if (!ops->compact_slice(sl, vdp, st)) return fail(PGPU_ERR_UNSUPPORTED, "slice variant");
+            } else {
             SliceArgs sl;
             sl.segs = (const Segment*)(dmeta + (B.replay ? L.segs : L.slsegs));
             sl.nseg = nseg;
@@ -532,6 +615,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sl.seg_status = (unsigned*)(dmeta + L.segstat);
             sl.blocks = (uint32_t)slice_blocks;
             if (!ops->slice(sl, vdp, B.payload, homog, st)) return fail(PGPU_ERR_UNSUPPORTED, "slice variant");
+            }
             CUDA_TRY(cudaGetLastError());
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[5], st));
             CUDA_TRY(cudaMemcpyAsync(h, dmeta, L.slotbase, cudaMemcpyDeviceToHost, st));
@@ -549,7 +633,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
                 (uint64_t)(uintptr_t)E.meta.p, (uint64_t)(uintptr_t)h,
                 (uint64_t)(uintptr_t)E.sval.p, (uint64_t)(uintptr_t)E.vlist.p, (uint64_t)(uintptr_t)E.vv0.p,
                 (uint64_t)(uintptr_t)E.vv1.p, (uint64_t)(uintptr_t)E.vkey0.p, (uint64_t)(uintptr_t)E.vf32.p,
-                (uint64_t)vrows, (uint64_t)(uintptr_t)E.vtx2slot.p, (uint64_t)nbr_half, (uint64_t)B.tile_w};
+                (uint64_t)vrows, (uint64_t)wide, (uint64_t)(uintptr_t)E.vkey.p,
+                (uint64_t)(uintptr_t)E.slot2vtx.p, (uint64_t)(uintptr_t)E.vtx2slot.p, (uint64_t)nbr_half, (uint64_t)B.tile_w};
             gk.reserve(gk.size() + 2 * (size_t)nseg);
             for (int k = 0; k < nseg; ++k) {
                 gk.push_back(cap[k]);
@@ -606,17 +691,25 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
                        std::vector<uint64_t>* cap_next) {
     const int d = B.d, nseg = (int)B.items.size();
     if (nseg == 0) return PGPU_OK;
-    const unsigned char* h = ps.h;
+    unsigned char* h = ps.h;
     const uint32_t M = ((const uint32_t*)h)[1];
     const unsigned* segstat = (const unsigned*)(h + ps.segstat);
-    const uint32_t* counts = (const uint32_t*)(h + ps.counts);
+    uint32_t* counts = (uint32_t*)(h + ps.counts);
+    if (nseg == 1) counts[0] = M;   // the compact splat counts per image only in batches
     bool retry = false;
     for (int k = 0; k < nseg; ++k) {
         if (segstat[k] & kStatusKeyRange)
             return fail(PGPU_ERR_ARGUMENT,
                         "image %d: positions leave the lattice's int16 key range (the reference's "
                         "keys wrap there and its rank indices leave [0, d]); scale them down", k);
-        if (segstat[k] & (kStatusProbeLimit | kStatusSpinLimit)) {
+        if (segstat[k] & kStatusWide) {   // rerun on int16-lane keys, now and later
+            failed->push_back(k);
+            if (cap_next) cap_next->push_back(ps.cap[k]);
+            retry = true;
+            std::lock_guard<std::mutex> lk(g_ratio_mu);
+            if (g_wide_sigs.size() > 4096) g_wide_sigs.clear();
+            g_wide_sigs.insert(ps.sig[k]);
+        } else if (segstat[k] & (kStatusProbeLimit | kStatusSpinLimit)) {
             uint64_t c = std::max<uint64_t>((uint64_t)(ps.cap[k] * 2.5), (uint64_t)(counts[k] / ps.load * 2));
             failed->push_back(k);
             if (cap_next) cap_next->push_back((c + 31) & ~31ull);
@@ -863,6 +956,8 @@ static int run_passes(Engine& E, BatchJob cur, cudaStream_t st, pgpu_stats* sum)
             sum->tile_w = s.tile_w;
             return PGPU_OK;
         }
+        // (an image that did not fit compact keys is known by now, so the pass, with every
+        // image in it, runs on int16-lane keys)
         BatchJob again = cur;
         again.items.clear();
         for (int k : failed) again.items.push_back(cur.items[k]);
@@ -874,9 +969,9 @@ static int run_passes(Engine& E, BatchJob cur, cudaStream_t st, pgpu_stats* sum)
 
 // Every image of a batch is filtered in place, so an image whose range overflowed cannot
 // simply be rerun with its whole batch: the others are finished.  Only the overflowed
-// ones go again (run_passes).  Vertex-ordered rows need every image of the launches on
-// the tile splat; a batch that asks for them but has images for the direct splat runs as
-// two, the tile-splat images with vertex-ordered rows, the others with slot-space rows.
+// ones go again (run_passes).  The images of one pass share a form of keys and of rows: a batch runs
+// as up to three, images known to need int16-lane keys, and, where it asks for
+// vertex-ordered rows (every image on the tile splat), the tile-splat images and the others.
 int run_batch(Engine& E, const BatchJob& B, cudaStream_t st) {
     if (B.items.empty()) return PGPU_OK;
     BatchJob cur = B;
@@ -893,35 +988,47 @@ int run_batch(Engine& E, const BatchJob& B, cudaStream_t st) {
         }
     }
     const int nseg = (int)cur.items.size();
-    std::vector<char> tiled(nseg, 0);
-    int nt = 0;
-    if (nseg > 1 && vertex_rows_wanted(cur)) {
+    BatchJob part[3] = {cur, cur, cur};   // vertex-ordered or plain, slot rows, int16-lane keys
+    part[1].slot_rows = true;
+    part[2].wide = true;
+    if (nseg > 1) {
         std::vector<uint64_t> sig;
         std::vector<double> ratio, density;
         learned_ratios(cur, &sig, &ratio, &density);
+        const std::vector<char> wide = known_wide(sig);
+        const bool vrows = vertex_rows_wanted(cur), all_wide = wide_forced(cur);
         const int forced = splat_forced();
-        for (int k = 0; k < nseg; ++k) nt += (tiled[k] = tile_splat_for(cur, forced, density[k], cur.items[k].n)) ? 1 : 0;
+        for (BatchJob& p : part) p.items.clear();
+        for (int k = 0; k < nseg; ++k) {
+            const int to = !all_wide && wide[k] ? 2
+                           : vrows && !tile_splat_for(cur, false, forced, density[k], cur.items[k].n) ? 1 : 0;
+            part[to].items.push_back(cur.items[k]);
+        }
+    } else {
+        part[1].items.clear();
+        part[2].items.clear();
     }
+    // (per-image results are asked for by single-image jobs only)
     pgpu_stats sum;
-    int rc;
-    if (nt > 0 && nt < nseg) {
-        BatchJob a = cur, b = cur;
-        a.items.clear();
-        b.items.clear();
-        b.slot_rows = true;
-        for (int k = 0; k < nseg; ++k) (tiled[k] ? a : b).items.push_back(cur.items[k]);
-        pgpu_stats sa, sb;
-        if ((rc = run_passes(E, a, st, &sa)) || (rc = run_passes(E, b, st, &sb))) return rc;
-        sum = sa;
-        sum.points += sb.points, sum.vertices += sb.vertices;
-        sum.capacity = std::max(sum.capacity, sb.capacity);
-        sum.retries = std::max(sum.retries, sb.retries);
-        sum.ms_splat += sb.ms_splat, sum.ms_compact += sb.ms_compact;
-        sum.ms_neighbours += sb.ms_neighbours, sum.ms_blur += sb.ms_blur;
-        sum.ms_slice += sb.ms_slice, sum.ms_total += sb.ms_total;
-        sum.tiled += sb.tiled;
-    } else if ((rc = run_passes(E, cur, st, &sum))) {
-        return rc;
+    memset(&sum, 0, sizeof(sum));
+    bool first = true;
+    for (const BatchJob& p : part) {
+        if (p.items.empty()) continue;
+        pgpu_stats s;
+        const int rc = run_passes(E, p, st, &s);
+        if (rc) return rc;
+        if (first) {
+            sum = s;
+            first = false;
+            continue;
+        }
+        sum.points += s.points, sum.vertices += s.vertices;
+        sum.capacity = std::max(sum.capacity, s.capacity);
+        sum.retries = std::max(sum.retries, s.retries);
+        sum.ms_splat += s.ms_splat, sum.ms_compact += s.ms_compact;
+        sum.ms_neighbours += s.ms_neighbours, sum.ms_blur += s.ms_blur;
+        sum.ms_slice += s.ms_slice, sum.ms_total += s.ms_total;
+        sum.tiled += s.tiled;
     }
     sum.tuned = tune ? 1 : tunable(B) ? 2 : 0;
     if (tune) tune_record(*tune, trial, sum);

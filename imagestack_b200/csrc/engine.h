@@ -58,8 +58,8 @@ struct Engine {
     DevBuf key0, keyn, tvals, ft, slot2vtx;
     // compaction
     DevBuf bitmap, offs, partials;
-    // vertex space
-    DevBuf vkey0, vkeyn, vv0, vv1, nbr;
+    // vertex space (vkey: compact keys, vkey0/vkeyn: int16-lane keys)
+    DevBuf vkey, vkey0, vkeyn, vv0, vv1, nbr;
     DevBuf vf32;   // FP32 normalised rows feeding the first blur pass (16-bit homogeneous)
     DevBuf vtx2slot;   // slot of each vertex
     DevBuf sval;       // filtered rows in slot space, arithmetic type, read by the slice
@@ -163,6 +163,7 @@ struct BatchJob {
     bool slot_rows = true;    // rows in slot space with a compaction; false: the tile splat
                               // numbers vertices and fills vertex-ordered rows where it can
     int nbr_half = 1;         // one neighbour lookup per axis (1) or two (0)
+    bool wide = false;        // int16-lane keys (a lattice whose keys do not fit compact keys)
     int tile_w = 0;           // tile splat tile width in pixels (0: the default, 16; height 256 / width)
     std::vector<BatchItem> items;
     // parity dumps (single-item jobs)

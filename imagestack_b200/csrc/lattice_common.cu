@@ -141,7 +141,7 @@ static uint32_t log2_of(uint32_t pow2) {
 static uint32_t magic_of(uint32_t d) { return d <= 1 ? 0xFFFFFFFFu : (uint32_t)(0x100000000ull / d); }
 
 void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint32_t* splat,
-                      uint32_t* tile, uint32_t* slice, uint32_t tile_w) {
+                      uint32_t* tile, uint32_t* slice, uint32_t splat_threads, uint32_t tile_w) {
     const PointSource& q = s.src;
     s.src.pos_is_val = q.pos.base == q.val.base && q.pos.ystride == q.val.ystride &&
                        q.pos.tstride == q.val.tstride && q.pos.cstride == q.val.cstride &&
@@ -149,23 +149,24 @@ void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint
     const uint32_t W = (uint32_t)s.src.width, H = (uint32_t)s.src.height, F = (uint32_t)s.src.frames;
     const uint64_t n = (uint64_t)W * H * F;
     if (tiled) {
-        // tile_w x (kTilePixels / tile_w) tiles (16x16 by default: a warp is two rows of
-        // 16 pixels); a point list (one row) in runs of kTilePixels
+        // tile_w x (kTilePixels / tile_w) tiles (16x16 by default); a point list (one row) in runs of kTilePixels
         const uint32_t tw = tile_w ? tile_w : (uint32_t)PGPU_TILE_W;
         s.tile_w = (H == 1 && F == 1) ? (uint32_t)kTilePixels : std::min<uint32_t>(tw, pow2_at_least(W));
         s.tile_h = (uint32_t)kTilePixels / s.tile_w;
         s.tiles_x = (W + s.tile_w - 1) / s.tile_w;
         s.tiles_y = (H + s.tile_h - 1) / s.tile_h;
         s.tile_shift = log2_of(s.tile_w);
+        // 8 x 8 pixels per warp; a narrower image's tile width, or a run of a point list
+        s.warp_shift = s.tile_h == 1 ? log2_of((uint32_t)kWarpPixels) : std::min<uint32_t>(3u, s.tile_shift);
         s.tile_xm = magic_of(s.tiles_x);
         s.tile_fm = magic_of(s.tiles_x * s.tiles_y);
         *tile = s.tiles_x * s.tiles_y * F;
         *splat = 0;
     } else {
         s.tile_w = s.tile_h = s.tiles_x = s.tiles_y = 0;
-        s.tile_shift = s.tile_xm = s.tile_fm = 0;
+        s.tile_shift = s.warp_shift = s.tile_xm = s.tile_fm = 0;
         *tile = 0;
-        *splat = (uint32_t)((n + kSplatThreads - 1) / kSplatThreads);
+        *splat = (uint32_t)((n + splat_threads - 1) / splat_threads);
     }
     const uint32_t Ws = (uint32_t)slice_src.width, Hs = (uint32_t)slice_src.height,
                    Fs = (uint32_t)slice_src.frames;

@@ -23,6 +23,7 @@ constexpr int kMaxSpin = 1 << 20;
 constexpr unsigned kStatusProbeLimit = 1u;   // hash table too full: rerun with more slots
 constexpr unsigned kStatusSpinLimit = 2u;    // a pending slot never became ready
 constexpr unsigned kStatusKeyRange = 4u;     // an elevated coordinate left the int16 range
+constexpr unsigned kStatusWide = 8u;         // keys out of the compact keys' range: rerun with int16 lanes
 
 // ---------------------------------------------------------------------------------
 // Keys.  A vertex key is d int16 coordinates (the (d+1)-th is implied, the keys of
@@ -144,12 +145,10 @@ __device__ __forceinline__ uint32_t home_slot(uint32_t h, uint32_t cap) { return
 // Insert-or-find during the splat, starting at slot `home` whose word 0 the caller has
 // already loaded into `first` (so the loads of several keys can be in flight at once);
 // returns the slot or -1 (status bit set).  *inserted, when given, is set when this call
-// created the slot; *seen, when given, receives the word a found slot held.  XYZ: one-word
-// keys of d <= 6 are compared on lanes 0..5 only, because a splat that numbers vertices as
-// it creates them publishes each vertex's index in lanes 6-7 while others still insert.
-template <int KW, bool XYZ = false>
+// created the slot.
+template <int KW>
 __device__ int table_insert(const TableView& t, const Key<KW>& k, uint32_t home, uint4 first,
-                            unsigned* status, bool* inserted = nullptr, uint4* seen = nullptr) {
+                            unsigned* status, bool* inserted = nullptr) {
     const uint4 empty = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
     uint32_t s = home;
     for (int probe = 0; probe < kMaxProbe; ++probe) {
@@ -174,12 +173,7 @@ __device__ int table_insert(const TableView& t, const Key<KW>& k, uint32_t home,
             }
         }
         if (KW == 1) {
-            const bool eq = XYZ ? (w.x == k.w[0].x && w.y == k.w[0].y && w.z == k.w[0].z)
-                                : words_equal(w, k.w[0]);
-            if (eq) {
-                if (seen) *seen = w;
-                return (int)s;
-            }
+            if (words_equal(w, k.w[0])) return (int)s;
         } else if (prefix_equal(w, k.w[0])) {
             int spins = 0;
             while (word_state(w) == kStatePending) {
@@ -204,8 +198,7 @@ __device__ int table_insert(const TableView& t, const Key<KW>& k, uint32_t home,
 }
 
 // For d <= 6 a one-word key leaves lanes 6 and 7 (the state lane) free of coordinates;
-// the compaction (or the splat that numbers vertices as it creates them) stores the
-// vertex's index there, so a neighbour lookup returns the index with the key.  Keys are
+// the compaction stores the vertex's index there, so a neighbour lookup returns the index with the key.  Keys are
 // then compared on lanes 0..5 only.  The index is stored as (v << 1) | 1: odd, so it never
 // reads as the unnumbered word's lanes 6-7 (0x00008000) nor as an empty word's.
 #ifndef PGPU_INDEX_IN_KEY_MAX_D
@@ -213,7 +206,6 @@ __device__ int table_insert(const TableView& t, const Key<KW>& k, uint32_t home,
 #endif
 __host__ __device__ constexpr bool index_in_key(int d) { return d <= PGPU_INDEX_IN_KEY_MAX_D; }
 __device__ __forceinline__ uint32_t enc_index(uint32_t v) { return (v << 1) | 1u; }
-__device__ __forceinline__ bool has_index(uint32_t w) { return (w & 1u) != 0; }
 __device__ __forceinline__ uint32_t dec_index(uint32_t w) { return w >> 1; }
 
 template <int D>
@@ -411,125 +403,6 @@ __device__ __forceinline__ void compute_simplex(const float (&p)[D], const Latti
     sx.bary[0] = __fadd_rn(srt[D], __fadd_rn(1.0f, -srt[0]));
 #pragma unroll
     for (int k = 1; k <= D; ++k) sx.bary[k] = __fsub_rn(srt[D - k], srt[D + 1 - k]);
-}
-
-// ---------------------------------------------------------------------------------
-// Tile keys: one-word keys (d <= 7) in 63 bits, for a block's table in shared memory.
-// Every coordinate of the key of remainder r is (d+1)*q_i + r with an integer quotient q_i,
-// so a key is r and d quotients; they are summed as fields of one 64-bit word, each field
-// biased by half its range.  Remainder r+1 is remainder r with r grown by one and the
-// quotient of the coordinate ranked d-r dropped by one (canonical[r][j] = r for j <= d-r,
-// else r-(d+1), src/Permutohedral.h:247-254): one 64-bit add instead of a step of every
-// 16-bit lane, and a probe reads and compares 8 bytes instead of 16.
-// Fields are 16 bits wide up to d = 3, then 15, 12, 10 and 8 bits.  Up to d = 5 the
-// quotients themselves fit them for positions within thousands of sigmas of the origin;
-// for d = 6 and 7 the block's fields hold differences to its first pixel's quotients.
-// A point whose keys do not fit is placed in the global table directly.
-// ---------------------------------------------------------------------------------
-template <int D>
-struct TileKey {
-    static_assert(key_words(D) == 1, "tile keys exist for one-word keys");
-    static constexpr int kRemBits = D + 1 <= 2 ? 1 : D + 1 <= 4 ? 2 : 3;
-    static constexpr int kFieldBits = (63 - kRemBits) / D < 16 ? (63 - kRemBits) / D : 16;
-    static constexpr bool kRelative = kFieldBits < 12;
-    // largest quotient (difference) a field holds, with room for the d+1 remainders' steps
-    static constexpr int kMaxField = (1 << (kFieldBits - 1)) - 2;
-    // largest quotient whose coordinates stay clear of the int16 range's ends, where the
-    // reference's short keys would wrap
-    static constexpr int kMaxAbs = 32767 / (D + 1) - 2;
-    static constexpr int kMaxQ = (kRelative || kMaxAbs < kMaxField) ? kMaxAbs : kMaxField;
-    static constexpr uint64_t kEmpty = ~0ull;   // no key: keys use the low 63 bits
-    __host__ __device__ static constexpr int shift(int i) { return kRemBits + i * kFieldBits; }
-    __host__ __device__ static constexpr uint64_t bias() {
-        uint64_t b = 0;
-        for (int i = 0; i < D; ++i) b += 1ull << (shift(i) + kFieldBits - 1);
-        return b;
-    }
-};
-
-// key of remainder 0 from the quotients (differences) of coordinates 0..d-1
-template <int D>
-__device__ __forceinline__ uint64_t tile_first_key(const int (&q)[D + 1]) {
-    uint64_t k = TileKey<D>::bias();
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-        const int s = TileKey<D>::shift(i);
-        if (s < 31) k += (uint64_t)((int64_t)q[i] * (int64_t)(1 << s));
-        else k += (uint64_t)((uint32_t)q[i] << (s - 32)) << 32;
-    }
-    return k;
-}
-
-// The simplex of one point (the arithmetic of compute_simplex, bit for bit) in the form the
-// tile splat uses: quotients of the greedy point in q, and in the thread's scratch column,
-// by rank, the coordinate's delta and the bit position of its quotient's field (64: the
-// implied coordinate, which has none).  Ranks are 4-bit fields of one register.  False,
-// with nothing to use, when a quotient is out of range or not a number.
-// scr: d+1 entries, kTileThreads apart.
-template <int D>
-__device__ __forceinline__ bool tile_simplex(const float (&p)[D], const LatticeConsts& lc, int (&q)[D + 1],
-                                             uint2* scr, int stride) {
-    using K = TileKey<D>;
-    float e[D + 1];
-    elevate<D>(p, lc, e);
-    const float scale = lc.inv_d1;
-    constexpr float dp1 = (float)(D + 1);
-    float g[D + 1], diff[D + 1];
-    int sum = 0;
-    bool fits = true;
-#pragma unroll
-    for (int i = 0; i <= D; ++i) {
-        const float fl = floorf(__fmul_rn(e[i], scale));
-        const float down = __fmul_rn(fl, dp1);
-        const float up = __fadd_rn(down, dp1);
-        const bool pick_up = __fsub_rn(up, e[i]) < __fsub_rn(e[i], down);
-        g[i] = pick_up ? up : down;
-        fits = fits && fabsf(g[i]) <= (float)K::kMaxQ * dp1;
-        q[i] = __float2int_rz(fl) + (pick_up ? 1 : 0);
-        sum += q[i];
-        diff[i] = __fsub_rn(e[i], g[i]);
-    }
-    uint32_t ranks = 0;   // of equal differences, the later coordinate ranks higher
-#pragma unroll
-    for (int i = 1; i <= D; ++i) ranks += (uint32_t)i << (4 * i);
-#pragma unroll
-    for (int i = 0; i < D; ++i)
-#pragma unroll
-        for (int j = i + 1; j <= D; ++j)
-            if (diff[i] < diff[j]) ranks += (1u << (4 * i)) - (1u << (4 * j));
-#pragma unroll
-    for (int i = 0; i <= D; ++i) {
-        int t = (int)((ranks >> (4 * i)) & 15u) + sum;
-        float gi = g[i];
-        if (t > D) t -= D + 1, q[i] -= 1, gi = __fsub_rn(gi, dp1);
-        else if (t < 0) t += D + 1, q[i] += 1, gi = __fadd_rn(gi, dp1);
-        const float delta = __fmul_rn(__fsub_rn(e[i], gi), scale);
-        scr[min((unsigned)t, (unsigned)D) * stride] =
-            make_uint2(__float_as_uint(delta), i < D ? (uint32_t)K::shift(i) : 64u);
-    }
-    return fits;
-}
-
-// 1 << s, 0 for s = 64
-__device__ __forceinline__ uint64_t bit64(uint32_t s) {
-    uint64_t r;
-    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(1ull), "r"(s));
-    return r;
-}
-
-// the full key of a tile key; base: the quotients the fields are relative to (d = 6, 7)
-template <int D>
-__device__ __forceinline__ void tile_full_key(uint64_t k, const int* base, Key<1>& out) {
-    using K = TileKey<D>;
-    const int r = (int)(k & ((1u << K::kRemBits) - 1));
-    int kc[D];
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-        int q = (int)((k >> K::shift(i)) & ((1u << K::kFieldBits) - 1)) - (1 << (K::kFieldBits - 1));
-        if (K::kRelative) q += base[i];
-        kc[i] = q * (D + 1) + r;
-    }
-    pack_key<D>(kc, out);
 }
 
 // Key of remainder 0: the greedy point itself (canonical[0][j] = 0 for every j).

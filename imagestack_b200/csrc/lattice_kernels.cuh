@@ -83,7 +83,7 @@ struct Segment {
     uint32_t slice_tw, slice_th, stiles_x, stiles_y;   // slice geometry
     // block -> tile without divisions: log2 of the tile widths (powers of two) and
     // floor(2^32 / divisor) of tiles per row and per frame (div_magic)
-    uint32_t tile_shift, slice_shift;
+    uint32_t tile_shift, slice_shift, warp_shift;   // warp_shift: of a tile splat warp's pixels
     uint32_t tile_xm, tile_fm, stile_xm, stile_fm;
 };
 
@@ -148,26 +148,11 @@ struct SplatArgs {
     void* rec;             // optional replay record: rows and weights (store_record)
     unsigned* seg_status;  // one status word per segment
     uint32_t blocks;       // direct splat blocks of the batch
-    uint32_t tile_blocks;  // tile splat blocks of the batch
     // optional vertex list: every slot the splat creates is appended to vlist (vcount
     // entries, zeroed), and counted in its segment's seg_counts entry (zeroed)
     uint32_t* vlist;
     uint32_t* vcount;
     uint32_t* seg_counts;
-    // Vertex-ordered rows (the tile splat, d <= 6): with vrows set, the splat numbers each
-    // vertex as it creates it (the position the vertex list would give it) and
-    // accumulates every lane's row into vrows[v*VDP..] (FP32, zeroed before the launch);
-    // the record holds vertex indices instead of slots; the creator writes the vertex's
-    // key (vkey0), its slot (vtx2slot) and its index into the key word, where other blocks
-    // read it.  No compaction is needed afterwards.
-    void* vrows = nullptr;
-    uint4* vkey0 = nullptr;
-    uint32_t* vtx2slot = nullptr;
-    // with vrows: the creator also marks its vertex's neighbour pairs (nbr_axes axes,
-    // nbr_stride apart) absent, for a neighbour search that looks up one direction per axis
-    int2* nbr_init = nullptr;
-    uint32_t nbr_stride = 0;
-    int nbr_axes = 0;
 };
 
 // Appends of one block to the batch's vertex list: slots go to the block's shared-memory
@@ -244,14 +229,8 @@ struct NbrArgs {
     const uint8_t* tags = nullptr;   // slot tags of the compaction, or null: plain lookups
     const unsigned* seg_status = nullptr;   // the splat's per-segment status, or null
     // one lookup per axis: vertex v finds u = n1(v) and, as n2(u) = v, writes v into u's
-    // pair too; every pair must hold (-1, -1) beforehand (written by the splat's creators
-    // with vertex-ordered rows, by the compaction otherwise)
+    // pair too; every pair must hold (-1, -1) beforehand (written by the compaction)
     int half = 0;
-    // homogeneous FP32 rows the splat left as plain sums (w*m_0.., w), vertex-ordered:
-    // each vertex's row is normalised here in place to (m_0.., w), as the compaction
-    // would have stored it; null: nothing to do
-    float* norm_rows = nullptr;
-    int vdp = 0, wc = 0;
 };
 
 // One launch blurs along one axis (nbrA) or, fused, along two consecutive axes (nbrA then
@@ -384,14 +363,17 @@ __device__ __forceinline__ void load_position_xyt(const PointSource& s, uint32_t
 // ---------------------------------------------------------------------------------
 // accumulator rows
 // ---------------------------------------------------------------------------------
+// (reductions written out: for atomicAdd the compiler may pick atomics that return the old
+// value, which double the splat's time)
 template <int VDP>
 __device__ __forceinline__ void atomic_add_row(float* dst, const float (&c)[VDP]) {
     if constexpr (VDP == 2) {
-        atomicAdd(reinterpret_cast<float2*>(dst), make_float2(c[0], c[1]));
+        asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" :: "l"(dst), "f"(c[0]), "f"(c[1]) : "memory");
     } else {
 #pragma unroll
         for (int k = 0; k < VDP; k += 4)
-            atomicAdd(reinterpret_cast<float4*>(dst + k), make_float4(c[k], c[k + 1], c[k + 2], c[k + 3]));
+            asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                         :: "l"(dst + k), "f"(c[k]), "f"(c[k + 1]), "f"(c[k + 2]), "f"(c[k + 3]) : "memory");
     }
 }
 template <int VDP>
@@ -444,6 +426,10 @@ __device__ __forceinline__ void load_record(const void* rec, uint32_t n_total, u
 // splat
 // ---------------------------------------------------------------------------------
 constexpr int kSplatThreads = 256;
+#ifndef PGPU_TILE_PX
+#define PGPU_TILE_PX 2
+#endif
+constexpr int kTilePixels = 128 * PGPU_TILE_PX;        // pixels of a tile splat block (lattice_compact.cuh)
 // Tuning (measured on the 4K d=5 and d=3 bilaterals and the 2M-point d=16 transform): the
 // splat is latency bound, so resident warps matter more than a few spilled registers —
 // 6 blocks of 256 per SM up to d=5 (40 registers; 0.94 -> 0.77 ms at 4K d=5), 4 for d=6,
@@ -571,78 +557,6 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     block_list_flush(blist, a, kseg);
 }
 
-// ---------------------------------------------------------------------------------
-// tile splat: one block per 2D tile of kTilePixels pixels of one frame
-// ---------------------------------------------------------------------------------
-// Neighbouring pixels land on the same lattice vertices (on the 4K d=5 bilateral a 16x16
-// tile's 1536 (point, remainder) entries touch about 155 distinct vertices), while the
-// direct splat pays one dependent probe of the global table, a trip to L2 or DRAM, per
-// lane group.  The tile splat first finds each vertex's entries within the tile, in shared
-// memory (phases A and B), inserts each distinct vertex of the tile into the global table
-// once (phase C), and then every lane adds its rows to the global rows with
-// fire-and-forget vector reductions and writes its replay record (phase D).  A vertex's first touch is
-// the smallest entry that reached it, so the global minimum over tiles is the reference's
-// first insertion; the vertex set, keys and records equal the direct splat's, only the order
-// of the FP32 additions differs.  One-word keys (d <= 7), FP32 accumulators.
-//
-// Finding equal keys takes no atomics: every entry stores its key in its own place and its
-// number in a claim table at its key's hash, whichever comes last; after a barrier it
-// reads the claim back and compares the claimant's key with its own.  Entries of one key
-// share a claim, so either all of them find the same claimant, which stands for the
-// vertex, or, where another key's entry came last, none; those (4 % of a 4K frame's
-// entries) go to a small open-addressed table.  (A block-wide compare-and-swap table
-// for all entries starts empty in every tile, so nearly every probe met contended
-// swaps: 12 shared-memory wavefronts per swap, 0.37 of the splat's 0.75 ms per 4K frame.)
-constexpr int kTileThreads = 256;
-constexpr int kTilePixels = 256;        // one pixel per thread
-constexpr int kTileClaims = 4096;       // claim table entries per block (powers of two)
-constexpr int kTileSlots = 512;         // slots of the table for entries whose claim was lost
-constexpr int kTileProbe = 64;
-#ifndef PGPU_TILE_MIN_BLOCKS_D5
-#define PGPU_TILE_MIN_BLOCKS_D5 5
-#endif
-__host__ __device__ constexpr int tile_min_blocks(int d) {
-    return d <= 5 ? PGPU_TILE_MIN_BLOCKS_D5 : d <= 6 ? 4 : 3;
-}
-
-// Dynamic shared memory of a tile splat block: per entry 8 bytes for the simplex scratch
-// and then the key, the claims, the lost claims' table, a row and a list place per vertex,
-// and the slots the block creates.  (The rows are not summed in shared memory: float
-// atomics there are compare-and-swap loops, and a variant that summed each tile's rows
-// before one global reduction per vertex took 2.1 ms per 4K frame against 0.73 ms.)
-__host__ __device__ constexpr size_t tile_smem_bytes(int d, int) {
-    const size_t entries = (size_t)(d + 1) * kTileThreads;
-    return entries * 8 + (size_t)kTileSlots * 8 + (entries + kTileSlots) * 4 + (size_t)kBlockListCap * 4 +
-           (size_t)kTileClaims * 2 + (entries + kTileSlots) * 2 + (size_t)kBlockListCap * 2;
-}
-
-// Hash of a tile key (32 bits, the high ones used): a multiplicative mix of its halves; the
-// global hash (a 64-bit mix) is computed only once per distinct vertex, in phase C.
-__device__ __forceinline__ uint32_t tile_hash(uint64_t k) {
-    return (uint32_t)k * 0x9E3779B1u + (uint32_t)(k >> 32) * 0x85EBCA77u;
-}
-
-// find-or-insert of a tile key in the block's small table: its slot, or -1 when no slot
-// within the probe limit is free (the caller then uses the global table)
-__device__ __forceinline__ int tile_insert(uint64_t* t_key, uint64_t k, bool* created) {
-    static_assert(kTileSlots == 512, "the home slot has 9 bits");
-    uint32_t l = (tile_hash(k) * 0x2C1B3C6Du) >> (32 - 9);
-#pragma unroll 1
-    for (int probe = 0; probe < kTileProbe; ++probe) {
-        uint64_t w = *reinterpret_cast<const volatile uint64_t*>(t_key + l);
-        if (w == ~0ull) {
-            w = atomicCAS_block(reinterpret_cast<unsigned long long*>(t_key + l), ~0ull, k);
-            if (w == ~0ull) {
-                *created = true;
-                return (int)l;
-            }
-        }
-        if (w == k) return (int)l;
-        l = (l + 1) & (kTileSlots - 1);
-    }
-    return -1;
-}
-
 // point (x, y, t) of a source: positions and values as load_point
 template <int D, int VDP>
 __device__ __forceinline__ void load_point_xyt(const PointSource& s, uint32_t x, uint32_t y, uint32_t t,
@@ -686,333 +600,6 @@ __device__ __forceinline__ void load_point_xyt(const PointSource& s, uint32_t x,
 #pragma unroll
         for (int k = 0; k < D; ++k) if (k == c) p[k] = f;
         ++c; }
-}
-
-// Vertex v, created by this block in global slot s (batch numbering): its key and slot in
-// vertex order (read by later kernels), then its index in the key word, which tells other
-// blocks the vertex's number.  The rows were zeroed before the launch, so no fence is
-// needed between the two: nothing a reader does with v depends on the creator's stores.
-template <int VDP>
-__device__ __forceinline__ void publish_vertex(const SplatArgs& a, uint32_t s, uint32_t v, uint4 key) {
-    key.w = 0x00008000u;   // lane 6 = coordinate 0 (none for d <= 6), lane 7 = ready state
-    a.vkey0[v] = key;
-    a.vtx2slot[v] = s;
-    if (a.nbr_init)
-        for (int j = 0; j < a.nbr_axes; ++j) a.nbr_init[(size_t)j * a.nbr_stride + v] = make_int2(-1, -1);
-    __stcg(reinterpret_cast<unsigned*>(a.key0 + s) + 3, enc_index(v));
-}
-
-// A vertex this block created in global slot gs (local slot l, or 0xFFFF for one placed in
-// the global table directly): onto the block's list, numbered and published by the flush;
-// when the list is full, numbered and published at once (returns its number then, else
-// 0xFFFFFFFF).
-template <int VDP>
-__device__ __forceinline__ uint32_t list_new_vertex(const SplatArgs& a, int kseg, uint32_t* s_new,
-                                                    uint16_t* s_new_l, uint32_t* s_new_count,
-                                                    uint32_t gs, uint16_t l, const uint4& key) {
-    const uint32_t jj = atomicAdd(s_new_count, 1u);
-    if (jj < kBlockListCap) {
-        s_new[jj] = gs;
-        s_new_l[jj] = l;
-        return 0xFFFFFFFFu;
-    }
-    const uint32_t v = atomicAdd(a.vcount, 1u);
-    atomicAdd(a.seg_counts + kseg, 1u);
-    publish_vertex<VDP>(a, gs, v, key);
-    return v;
-}
-
-// t_row marker of a vertex the block created and numbers in its flush (never a vertex index:
-// indices stay below the 2^31 - 256 slots of a batch)
-constexpr uint32_t kOwnPending = 0x7FFFFFFFu;
-
-// the vertex index of global slot s, created by another block: wait (bounded) until its
-// creator has published it, which takes the creator's global inserts and one atomic
-// (microseconds); 0xFFFFFFFF with the spin-limit status bit if it is not published within
-// kAwaitSpin polls, or at once when another wait of the lattice has given up already
-constexpr int kAwaitSpin = 1 << 14;
-__device__ __forceinline__ uint32_t await_vertex(const SplatArgs& a, uint32_t s, unsigned* status) {
-    const unsigned* w = reinterpret_cast<const unsigned*>(a.key0 + s) + 3;
-    for (int spin = 0; spin < kAwaitSpin; ++spin) {
-        const unsigned x = __ldcg(w);
-        if (has_index(x)) return dec_index(x);
-        if ((spin & 63) == 63 && (__ldcg(status) & kStatusSpinLimit)) return 0xFFFFFFFFu;
-        __nanosleep(64);
-    }
-    atomicOr(status, kStatusSpinLimit);
-    return 0xFFFFFFFFu;
-}
-
-// VROWS: number vertices as they are created and accumulate into vertex-ordered rows (the
-// SplatArgs::vrows protocol, d <= 6, no first touches); otherwise rows in slot space.
-template <int D, int VDP, bool VROWS>
-__global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) splat_tile_kernel(SplatArgs a) {
-    static_assert(key_words(D) == 1, "the tile splat handles one-word keys (d <= 7)");
-    static_assert(!VROWS || index_in_key(D), "vertex-ordered rows publish the index in the key word");
-    using K = TileKey<D>;
-    constexpr uint32_t kEntries = (D + 1) * kTileThreads;   // entry (r, thread) is r*kTileThreads + thread
-    extern __shared__ __align__(16) unsigned char tile_smem[];
-    uint2* s_scr = reinterpret_cast<uint2*>(tile_smem);     // the simplex, then each entry's key
-    uint64_t* s_key = reinterpret_cast<uint64_t*>(s_scr);
-    uint64_t* t_key = s_key + kEntries;                     // the lost claims' table
-    uint32_t* t_row = reinterpret_cast<uint32_t*>(t_key + kTileSlots);   // per vertex of the tile
-    uint32_t* s_new = t_row + kEntries + kTileSlots;
-    uint16_t* s_claim = reinterpret_cast<uint16_t*>(s_new + kBlockListCap);
-    uint16_t* t_list = s_claim + kTileClaims;               // the tile's vertices
-    uint16_t* s_new_l = t_list + kEntries + kTileSlots;
-    __shared__ Segment sg;
-    __shared__ uint32_t t_count, s_new_count, s_new_base;
-    __shared__ int s_base[K::kRelative ? D : 1];
-    const int kseg = segment_by<&Segment::tile_base>(a.segs, a.nseg, blockIdx.x);
-    for (int l = threadIdx.x; l < kTileSlots / 2; l += kTileThreads)
-        reinterpret_cast<uint4*>(t_key)[l] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-    if (!VROWS && a.ft)
-        for (int l = threadIdx.x; l < (int)kEntries + kTileSlots; l += kTileThreads) t_row[l] = 0xFFFFFFFFu;
-    if (threadIdx.x == 0) t_count = 0, s_new_count = 0;
-    load_segment(a.segs + kseg, sg);   // ends with a barrier
-
-    unsigned* status = a.seg_status + kseg;
-    const TableView table{a.key0 + sg.slot_base, a.keyn + sg.slot_base, sg.cap, a.cap_total};
-    float* vals = VROWS ? reinterpret_cast<float*>(a.vrows)
-                        : reinterpret_cast<float*>(a.vals) + (size_t)sg.slot_base * VDP;
-    uint32_t* ft = (!VROWS && a.ft) ? a.ft + sg.slot_base : nullptr;
-    uint32_t bt, tx;
-    const uint32_t f = div_magic(blockIdx.x - sg.tile_base, sg.tiles_x * sg.tiles_y, sg.tile_fm, &bt);
-    const uint32_t ty = div_magic(bt, sg.tiles_x, sg.tile_xm, &tx);
-    const uint32_t px = (tx << sg.tile_shift) + (threadIdx.x & (sg.tile_w - 1));
-    const uint32_t py = ty * sg.tile_h + (threadIdx.x >> sg.tile_shift);
-    const uint32_t W = (uint32_t)sg.src.width, H = (uint32_t)sg.src.height;
-    const bool valid = px < W && py < H;
-    const uint32_t gi = sg.point_base + (f * H + py) * W + px;
-    uint2* scr = s_scr + threadIdx.x;
-    uint64_t* keys = s_key + threadIdx.x;
-
-    // Phase A: this pixel's simplex, its keys and their claims
-    float v[VDP];
-    float bary[D + 1];
-    int q[D + 1];
-    bool fits = false;
-    Key<1> kk;   // the first key of a pixel whose keys do not fit tile keys
-    if (valid) {
-        float pp[D];
-        load_point_xyt<D, VDP>(sg.src, px, py, f, pp, v);
-        fits = tile_simplex<D>(pp, a.lc, q, scr, kTileThreads);
-    }
-    if constexpr (K::kRelative) {
-        if (threadIdx.x == 0) {   // the tile's first pixel, inside every image
-#pragma unroll
-            for (int i = 0; i < D; ++i) s_base[i] = q[i];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < D; ++i) {
-            q[i] = (int)((unsigned)q[i] - (unsigned)s_base[i]);
-            fits = fits && q[i] <= K::kMaxField && q[i] >= -K::kMaxField;
-        }
-    }
-    if (fits) {
-        float srt[D + 1];
-        uint32_t field[D + 1];
-#pragma unroll
-        for (int k = 0; k <= D; ++k) {
-            const uint2 e = scr[k * kTileThreads];
-            srt[k] = __uint_as_float(e.x);
-            field[k] = e.y;
-        }
-        // b[0] = delta(rank d) + (1 + b[d+1]),  b[d+1] = -delta(rank 0) (compute_simplex)
-        bary[0] = __fadd_rn(srt[D], __fadd_rn(1.0f, -srt[0]));
-#pragma unroll
-        for (int k = 1; k <= D; ++k) bary[k] = __fsub_rn(srt[D - k], srt[D + 1 - k]);
-        uint64_t key = tile_first_key<D>(q);
-#pragma unroll
-        for (int r = 0; r <= D; ++r) {
-            if (r > 0) key += 1ull - bit64(field[D - (r - 1)]);
-            keys[r * kTileThreads] = key;
-            s_claim[tile_hash(key) / (uint32_t)(0x100000000ull / kTileClaims)] = (uint16_t)(r * kTileThreads + threadIdx.x);
-        }
-    } else if (valid) {
-        // out of a tile key's range: the general simplex, every vertex in the global table
-        float pp[D];
-        load_point_xyt<D, VDP>(sg.src, px, py, f, pp, v);
-        Simplex<D> sx;
-        const SimplexScratch gs{reinterpret_cast<float*>(scr), reinterpret_cast<unsigned char*>(scr) + 4,
-                                2 * kTileThreads, 8 * kTileThreads};
-        compute_simplex<D>(pp, a.lc, sx, status, gs);
-        first_key<D>(sx, kk);
-#pragma unroll
-        for (int r = 0; r <= D; ++r) bary[r] = sx.bary[r];
-    }
-    __syncthreads();
-
-    // Phase B: the vertex of each entry, by its number in the tile: that of the entry that
-    // stands for it, or kEntries + its slot in the lost claims' table.
-    // loc[r] >= 0: that number; -1: not placed; <= -2: global slot -(loc + 2), taken directly
-    // because the key does not fit a tile key or the small table was full around it.
-    int loc[D + 1];
-    uint32_t todo = 0;   // remainders to place in the global table
-    if (fits) {
-        uint32_t stands = 0;   // remainders whose entry stands for its vertex
-#pragma unroll
-        for (int r = 0; r <= D; ++r) {
-            const uint64_t key = keys[r * kTileThreads];
-            const uint32_t c = s_claim[tile_hash(key) / (uint32_t)(0x100000000ull / kTileClaims)];
-            loc[r] = (int)c;
-            if (s_key[c] != key) todo |= 1u << r;
-            else if (c == (uint32_t)r * kTileThreads + threadIdx.x) stands |= 1u << r;
-        }
-        if (stands) {
-            uint32_t j = atomicAdd(&t_count, (uint32_t)__popc(stands));
-#pragma unroll
-            for (int r = 0; r <= D; ++r)
-                if ((stands >> r) & 1u) t_list[j++] = (uint16_t)(r * kTileThreads + threadIdx.x);
-        }
-#pragma unroll
-        for (int r = 0; r <= D; ++r) {
-            if (!((todo >> r) & 1u)) continue;
-            bool created = false;
-            const int l = tile_insert(t_key, keys[r * kTileThreads], &created);
-            if (l < 0) continue;
-            loc[r] = (int)kEntries + l;
-            todo &= ~(1u << r);
-            if (created) t_list[atomicAdd(&t_count, 1u)] = (uint16_t)(kEntries + l);
-        }
-        if (ft) {
-#pragma unroll
-            for (int r = 0; r <= D; ++r)
-                if (!((todo >> r) & 1u)) atomicMin(&t_row[loc[r]], gi * (uint32_t)(D + 1) + (uint32_t)r);
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r <= D; ++r) loc[r] = -1;
-        if (valid) todo = (1u << (D + 1)) - 1u;
-    }
-    if (todo) {
-        // rare: rolled, with the results in the scratch (no other thread reads these entries:
-        // they stand for no vertex)
-#pragma unroll 1
-        for (int r = 0; r <= D; ++r) {
-            if (!fits && r > 0) key_step<D>(kk, (int)(scr[(D - (r - 1)) * kTileThreads].y & 0xFFu));
-            if (!((todo >> r) & 1u)) continue;
-            Key<1> key = kk;
-            if (fits) tile_full_key<D>(keys[r * kTileThreads], s_base, key);
-            const uint32_t home = home_slot(key_hash<1>(key), table.cap);
-            bool created = false;
-            const int s = table_insert<1, VROWS>(table, key, home, __ldcg(&table.key0[home]), status, &created);
-            if (s >= 0) {
-                if constexpr (VROWS) {   // numbered by the flush; phase D reads the key word
-                    if (created)
-                        list_new_vertex<VDP>(a, kseg, s_new, s_new_l, &s_new_count, sg.slot_base + (uint32_t)s,
-                                             0xFFFFu, key.w[0]);
-                } else {
-                    if (ft) atomicMin(&ft[s], gi * (uint32_t)(D + 1) + (uint32_t)r);
-                    if (created && a.vlist)
-                        block_list_append(BlockList{s_new, &s_new_count, &s_new_base}, a, kseg,
-                                          sg.slot_base + (uint32_t)s);
-                }
-            }
-            scr[r * kTileThreads].x = (uint32_t)(s >= 0 ? -(s + 2) : -1);
-        }
-#pragma unroll
-        for (int r = 0; r <= D; ++r)
-            if ((todo >> r) & 1u) loc[r] = (int)scr[r * kTileThreads].x;
-    }
-    __syncthreads();
-
-    // Phase C: each distinct vertex of the tile into the global table once
-    const uint32_t count = t_count;
-#pragma unroll 1
-    for (uint32_t j = threadIdx.x; j < count; j += kTileThreads) {
-        const int l = t_list[j];
-        Key<1> key;
-        tile_full_key<D>(s_key[l], s_base, key);   // the small table's keys follow the entries'
-        const uint32_t h = home_slot(key_hash<1>(key), table.cap);
-        bool created = false;
-        uint4 seen = make_uint4(0u, 0u, 0u, 0u);
-        const int s = table_insert<1, VROWS>(table, key, h, __ldcg(&table.key0[h]), status, &created, &seen);
-        if constexpr (VROWS) {
-            // t_row[l]: the vertex index; kOwnPending for a vertex this block numbers in its
-            // flush; 0x80000000 | global slot while another block's vertex is not numbered
-            uint32_t val = 0xFFFFFFFFu;
-            if (s >= 0) {
-                const uint32_t gs = sg.slot_base + (uint32_t)s;
-                val = 0x80000000u | gs;
-                if (created) {
-                    const uint32_t vv = list_new_vertex<VDP>(a, kseg, s_new, s_new_l, &s_new_count, gs,
-                                                             (uint16_t)l, key.w[0]);
-                    val = vv != 0xFFFFFFFFu ? vv : kOwnPending;
-                } else if (has_index(seen.w)) {
-                    val = dec_index(seen.w);
-                }
-            }
-            t_row[l] = val;
-        } else {
-            if (s >= 0 && ft) atomicMin(&ft[s], t_row[l]);
-            if (created && a.vlist)
-                block_list_append(BlockList{s_new, &s_new_count, &s_new_base}, a, kseg, sg.slot_base + (uint32_t)s);
-            t_row[l] = s >= 0 ? (uint32_t)s : 0xFFFFFFFFu;   // the global slot (segment-relative)
-        }
-    }
-    __syncthreads();
-    if constexpr (VROWS) {
-        // number the block's new vertices with one atomic and publish them; in the same
-        // pass, learn (once per vertex) the numbers of the tile's vertices other blocks
-        // created, which is faster than every lane waiting for its own entries in phase D
-        const uint32_t n = min(s_new_count, kBlockListCap);
-        if (n) {
-            if (threadIdx.x == 0) {
-                s_new_base = atomicAdd(a.vcount, n);
-                atomicAdd(a.seg_counts + kseg, n);
-            }
-            __syncthreads();
-        }
-        const uint32_t base = s_new_base;
-        for (uint32_t jj = threadIdx.x; jj < n; jj += kTileThreads) {
-            const int l = s_new_l[jj];
-            if (l != 0xFFFF) {
-                Key<1> key;
-                tile_full_key<D>(s_key[l], s_base, key);
-                publish_vertex<VDP>(a, s_new[jj], base + jj, key.w[0]);
-                t_row[l] = base + jj;
-            } else {   // placed in the global table directly in phase B
-                publish_vertex<VDP>(a, s_new[jj], base + jj, __ldcg(&a.key0[s_new[jj]]));
-            }
-        }
-#pragma unroll 1
-        for (uint32_t j = threadIdx.x; j < count; j += kTileThreads) {
-            const int l = t_list[j];
-            const uint32_t val = t_row[l];
-            if (val != 0xFFFFFFFFu && (val & 0x80000000u)) t_row[l] = await_vertex(a, val & 0x7FFFFFFFu, status);
-        }
-        __syncthreads();
-    } else {
-        if (a.vlist) block_list_flush(BlockList{s_new, &s_new_count, &s_new_base}, a, kseg);
-    }
-
-    // Phase D: every lane's rows into its vertices' global rows (VROWS: by vertex index;
-    // otherwise segment slots; 0xFFFFFFFF: not placed), and the replay record
-    if (!valid) return;
-    uint32_t row[D + 1];
-#pragma unroll
-    for (int r = 0; r <= D; ++r) {
-        const int l = loc[r];
-        uint32_t s = 0xFFFFFFFFu;
-        if (l >= 0) {
-            s = t_row[l];
-        } else if (l <= -2) {
-            s = (uint32_t)(-(l + 2));
-            if constexpr (VROWS) s = await_vertex(a, sg.slot_base + s, status);
-        }
-        if (s != 0xFFFFFFFFu) {
-            float c[VDP];
-#pragma unroll
-            for (int k = 0; k < VDP; ++k) c[k] = __fmul_rn(bary[r], v[k]);
-            atomic_add_row<VDP>(vals + (size_t)s * VDP, c);
-            if (!VROWS) s += sg.slot_base;
-        }
-        row[r] = s;
-        if (a.rec_slot) a.rec_slot[(size_t)r * a.n_total + gi] = s;
-    }
-    if (a.rec) store_record<D>(a.rec, a.n_total, gi, row, bary);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1167,12 +754,6 @@ __global__ void neighbours_kernel(NbrArgs a) {
             if (!a.half)
                 for (int j = 0; j <= D; ++j) a.nbr[(size_t)j * a.vcap + vtx] = make_int2(-1, -1);
             continue;
-        }
-        if (a.norm_rows) {   // m = sum / w, 0 where w is 0 (the compaction's arithmetic)
-            float* r = a.norm_rows + (size_t)vtx * a.vdp;
-            const float w = r[a.wc];
-            for (int k = 0; k < a.wc; ++k) r[k] = w != 0.0f ? r[k] / w : 0.0f;
-            for (int k = a.wc + 1; k < a.vdp; ++k) r[k] = 0.0f;
         }
         const uint32_t base = __ldg(a.seg_slot_base + kseg);
         const TableView table{a.key0 + base, a.keyn + base, __ldg(a.seg_slot_base + kseg + 1) - base,
@@ -1420,7 +1001,7 @@ __global__ void __launch_bounds__(kSliceThreads, slice_min_blocks(D)) slice_kern
     unsigned* status = a.seg_status + kseg;
     // A splat that overflowed the table is rerun by the host with more slots; its
     // output may be the caller's input image (in-place filtering), so write nothing.
-    if (__ldcg(status) & (kStatusProbeLimit | kStatusSpinLimit | kStatusKeyRange)) return;
+    if (__ldcg(status) & (kStatusProbeLimit | kStatusSpinLimit | kStatusKeyRange | kStatusWide)) return;
     const uint32_t gi = sg.point_base + i;
     float p[D];
     load_position<D>(sg.src, i, p);
@@ -1512,7 +1093,7 @@ __global__ void __launch_bounds__(kSliceThreads) slice_replay_kernel(SliceArgs a
     const uint32_t W = (uint32_t)sg.src.width, H = (uint32_t)sg.src.height;
     if (px >= W || py >= H) return;
     // an image whose splat overflowed its table is rerun by the host; write nothing
-    if (__ldcg(a.seg_status + kseg) & (kStatusProbeLimit | kStatusSpinLimit | kStatusKeyRange)) return;
+    if (__ldcg(a.seg_status + kseg) & (kStatusProbeLimit | kStatusSpinLimit | kStatusKeyRange | kStatusWide)) return;
     const uint32_t gi = sg.point_base + (fr * H + py) * W + px;
     const A* sv = reinterpret_cast<const A*>(a.svals);
     int sl[D + 1];

@@ -1,7 +1,7 @@
 // Launch interface between the host pipeline (engine.cu) and the kernels.
 #pragma once
 
-#include "lattice_kernels.cuh"
+#include "lattice_compact.cuh"
 
 namespace pgpu {
 
@@ -16,15 +16,19 @@ inline int accum_bytes(int payload) { return payload == kPayloadF64 ? 8 : 4; }
 // kernels whose code depends on the number of position dimensions d
 struct DimOps {
     bool (*splat)(const SplatArgs&, int vdp, int payload, cudaStream_t);
-    // the tile splat over the segments with tile_w > 0 (a.tile_blocks blocks); false when
-    // this d or payload has no tile splat (multi-word keys, FP64 accumulators)
-    bool (*splat_tile)(const SplatArgs&, int vdp, int payload, cudaStream_t);
-    // one-time per-device set-up of the tile splat's kernels (their shared-memory limit);
-    // called outside any stream capture, before the first launch
-    bool (*prepare)();
     void (*neighbours)(const NbrArgs&, uint32_t vmax, int sms, cudaStream_t);
     bool (*slice)(const SliceArgs&, int vdp, int payload, bool homog, cudaStream_t);
+    // on compact keys (FP32 accumulators): the direct splat of a.blocks blocks and the tile
+    // splat of a.tile_blocks (false: no tile splat for this d), the vertex order of parity
+    // dumps, the neighbour search, and the slice at other positions than the splat's
+    bool (*compact_splat)(const CompactSplatArgs&, int vdp, cudaStream_t);
+    void (*compact_rank)(const CompactRankArgs&, int sms, cudaStream_t);
+    void (*compact_neighbours)(const CompactNbrArgs&, uint32_t vmax, int sms, cudaStream_t);
+    bool (*compact_slice)(const CompactSliceArgs&, int vdp, cudaStream_t);
 };
+
+// bytes of a compact key
+inline int compact_key_bytes(int d) { return d <= 7 ? 8 : 16; }
 
 // one definition per d, in lattice_d.cu compiled once per d
 #define PGPU_DECLARE_DIM(D) const DimOps* dim_ops_##D();
@@ -37,10 +41,10 @@ PGPU_DECLARE_DIM(13) PGPU_DECLARE_DIM(14) PGPU_DECLARE_DIM(15) PGPU_DECLARE_DIM(
 const DimOps* dim_ops(int d);
 
 // Launch geometry of one segment (its src, the splat points, and slice_src, the points
-// sliced, are set): the direct-splat blocks or, when `tiled`, the tile-splat tiles, and
+// sliced, are set): the direct-splat blocks (of splat_threads points) or, when `tiled`, the tile-splat tiles, and
 // the slice tiles.  Returns the blocks of each launch through *splat, *tile and *slice.
 void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint32_t* splat,
-                      uint32_t* tile, uint32_t* slice, uint32_t tile_w = 0);
+                      uint32_t* tile, uint32_t* slice, uint32_t splat_threads, uint32_t tile_w = 0);
 
 void launch_mark(const uint32_t* ft, uint32_t cap, uint32_t* bitmap, int sms, cudaStream_t st);
 // per-segment vertex counts from the first-touch bitmap and its prefix popcount

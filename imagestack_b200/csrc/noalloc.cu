@@ -171,7 +171,7 @@ extern "C" int pgpu_bilateral_noalloc(const float* d_in, float* d_out, int width
     seg.n = n;
     seg.cap = cap;
     uint32_t splat_blocks = 0, tile_blocks = 0, slice_blocks = 0;
-    segment_geometry(seg, src, false, &splat_blocks, &tile_blocks, &slice_blocks);
+    segment_geometry(seg, src, false, &splat_blocks, &tile_blocks, &slice_blocks, kSplatThreads);
     const uint32_t slot_bounds[2] = {0u, cap};
     CUDA_TRY(cudaMemcpyAsync(base + kOffSeg, &seg, sizeof(seg), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(base + kOffSlotBase, slot_bounds, sizeof(slot_bounds),
@@ -192,7 +192,6 @@ extern "C" int pgpu_bilateral_noalloc(const float* d_in, float* d_out, int width
     sa.rec_slot = (uint32_t*)(base + kOffRec);
     sa.seg_status = dstatus;
     sa.blocks = splat_blocks;
-    sa.tile_blocks = 0;
     sa.rec = nullptr;     // the slice recomputes the weights
     sa.vlist = nullptr;   // vertices numbered by first touch (mark, scan, assign below)
     sa.vcount = nullptr;

@@ -411,3 +411,45 @@ def test_positions_far_from_the_origin(gpu, monkeypatch, mode, d, offset):
         np.testing.assert_array_equal(got[k], getattr(ref, k))
     for k in ("splat", "blur", "out"):
         assert rel_err(got[k], getattr(ref, k)) <= RTOL_FP32
+
+
+@pytest.mark.parametrize("keys", ["compact", "wide"])
+@pytest.mark.parametrize("d", [1, 2, 4, 6, 7, 8, 9, 12, 13, 15, 16])
+def test_key_forms_match_the_oracle(gpu, monkeypatch, d, keys):
+    """Every width of a compact key's fields (64 bits to d = 7, 128 above; 16 remainders and
+    more) and the int16-lane keys: keys, vertex order and records bit for bit, and the slice
+    at other positions, some of whose vertices the splat never made."""
+    monkeypatch.setenv("PGPU_KEYS", keys)
+    rng = np.random.default_rng(100 + d)
+    n = 1533
+    pos = (rng.integers(0, 3, (n, 1)) * 2.5 + rng.normal(0, 0.4, (n, d))).astype(np.float32)
+    val = rng.uniform(0, 1, (n, 5 if d % 2 else 2)).astype(np.float32)
+    other = (pos[::-1] + rng.normal(0, 0.3, (n, d))).astype(np.float32)
+    ref = oracle.oracle_lattice(pos, val, slice_pos=other)
+    got = gpu.lattice_dump(pos, val)
+    for k in ("keys", "replay_vtx", "replay_w"):
+        np.testing.assert_array_equal(got[k], getattr(ref, k))
+    here = oracle.oracle_lattice(pos, val).out
+    assert rel_err(got["out"], here) <= RTOL_FP32
+    planar = lambda a: np.ascontiguousarray(a.T).reshape(a.shape[1], 1, n)
+    out = gpu.GaussTransform.apply(planar(other), planar(pos), planar(val), [1.0] * d)
+    assert rel_err(out.reshape(-1, n).T, ref.out) <= RTOL_FP32
+    out = gpu.GaussTransform.apply(None, planar(pos), planar(val), [1.0] * d)
+    assert rel_err(out.reshape(-1, n).T, here) <= RTOL_FP32
+
+
+@pytest.mark.parametrize("payload,tol", [("fp32", RTOL_FP32), ("fp16", 1e-3), ("bf16", 1e-2)])
+def test_batch_with_images_out_of_the_compact_keys_range(gpu, payload, tol):
+    """A batch in which one image's keys do not fit compact keys (filtered again on int16
+    lanes, then, known, apart from the others) equals the images filtered one by one."""
+    imgs = [synth.image(w, h, 3, rects=6, seed=w) for w, h in ((150, 90), (97, 133), (64, 64))]
+    imgs[1] = (imgs[1] * 3000).astype(np.float32)   # colours thousands of sigmas apart
+    fw, cs = [6.0, 5.0, 8.0], [0.1, 0.8, 0.2]
+    expect = [im.copy() for im in imgs]
+    for im, f, c in zip(expect, fw, cs):
+        gpu.Bilateral.apply(im, f, f, 0.0, c, payload="fp64")
+    for _ in range(2):
+        out = [im.copy() for im in imgs]
+        gpu.bilateral_batch(out, fw, cs, payload=payload)
+        for a, b in zip(out, expect):
+            assert rel_err(a, b, floor_frac=1e-2) <= tol
