@@ -265,7 +265,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     learned_ratios(B, &sig, &ratio, &density);
     bool wide = wide_forced(B);
     for (char w : known_wide(sig)) wide = wide || w;
-    const bool use_tags = wide && kw > 1;
+    const bool use_tags = kw > 1;
     const int kb = compact_key_bytes(d);
     std::vector<uint64_t> cap(nseg);
     for (int k = 0; k < nseg; ++k) {
@@ -449,9 +449,10 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sa.vkey = E.vkey.p;
             sa.vtx2slot = (uint32_t*)E.vtx2slot.p;
             sa.slot2vtx = (uint32_t*)E.slot2vtx.p;
-            sa.nbr_init = nbr_half ? (int2*)E.nbr.p : nullptr;
+            sa.nbr_init = nbr_half ? (int*)E.nbr.p : nullptr;
             sa.nbr_stride = (uint32_t)cap_total;
             sa.number_rows = vrows ? 1 : 0;
+            sa.tags = use_tags && !exact_order ? (uint8_t*)E.tags.p : nullptr;
             if (!ops->compact_splat(sa, vdp, st)) return fail(PGPU_ERR_UNSUPPORTED, "splat variant");
             }
             CUDA_TRY(cudaGetLastError());
@@ -486,7 +487,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             ca.nverts = dM;
             ca.index_in_key = index_in_key(d) ? 1 : 0;   // the neighbour lookups expect it
             if (nbr_half) {
-                ca.nbr_init = (int2*)E.nbr.p;
+                ca.nbr_init = (int*)E.nbr.p;
                 ca.nbr_stride = (uint32_t)cap_total;
                 ca.nbr_axes = d + 1;
             }
@@ -502,8 +503,9 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
                 ra.vkey = E.vkey.p;
                 ra.vtx2slot = (uint32_t*)E.vtx2slot.p;
                 ra.slot2vtx = (uint32_t*)E.slot2vtx.p;
-                ra.nbr_init = nbr_half ? (int2*)E.nbr.p : nullptr;
+                ra.nbr_init = nbr_half ? (int*)E.nbr.p : nullptr;
                 ra.nbr_stride = (uint32_t)cap_total;
+                ra.tags = use_tags ? (uint8_t*)E.tags.p : nullptr;
                 ra.wide0 = (uint4*)E.vkey0.p;
                 ra.widen = (uint4*)E.vkeyn.p;
                 ra.wide_stride = (uint32_t)cap_total;
@@ -525,7 +527,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             na.vkeyn = (const uint4*)E.vkeyn.p;
             na.vcap = (uint32_t)cap_total;
             na.nverts = dM;
-            na.nbr = (int2*)E.nbr.p;
+            na.nbr = (int*)E.nbr.p;
             na.tags = use_tags ? (const uint8_t*)E.tags.p : nullptr;
             na.seg_status = (const unsigned*)(dmeta + L.segstat);
             na.half = nbr_half ? 1 : 0;
@@ -541,9 +543,10 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             na.vtx2slot = (const uint32_t*)E.vtx2slot.p;
             na.slot2vtx = (const uint32_t*)E.slot2vtx.p;
             na.nverts = dM;
-            na.nbr = (int2*)E.nbr.p;
+            na.nbr = (int*)E.nbr.p;
             na.stride = (uint32_t)cap_total;
             na.half = nbr_half ? 1 : 0;
+            na.tags = use_tags ? (const uint8_t*)E.tags.p : nullptr;
             // the splat's slot rows go to vertex order here; vertex-ordered homogeneous rows
             // are only normalised
             na.gather = vrows ? kRowsInPlace : homog ? kRowsNormalise : B.payload == kPayloadF16 ? kRowsHalf
@@ -567,7 +570,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             bp.payload = B.payload;
             bp.homog = homog;
             bp.src_f32 = homog || f32_rows;
-            bp.nbr = (const int2*)E.nbr.p;
+            bp.nbr = (const int*)E.nbr.p;
             bp.nbr_stride = cap_total;
             bp.nverts = dM;
             bp.vmax = (uint32_t)cap_total;
@@ -634,7 +637,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
                 (uint64_t)(uintptr_t)E.sval.p, (uint64_t)(uintptr_t)E.vlist.p, (uint64_t)(uintptr_t)E.vv0.p,
                 (uint64_t)(uintptr_t)E.vv1.p, (uint64_t)(uintptr_t)E.vkey0.p, (uint64_t)(uintptr_t)E.vf32.p,
                 (uint64_t)vrows, (uint64_t)wide, (uint64_t)(uintptr_t)E.vkey.p,
-                (uint64_t)(uintptr_t)E.slot2vtx.p, (uint64_t)(uintptr_t)E.vtx2slot.p, (uint64_t)nbr_half, (uint64_t)B.tile_w};
+                (uint64_t)(uintptr_t)E.slot2vtx.p, (uint64_t)(uintptr_t)E.tags.p, (uint64_t)(uintptr_t)E.vtx2slot.p, (uint64_t)nbr_half, (uint64_t)B.tile_w};
             gk.reserve(gk.size() + 2 * (size_t)nseg);
             for (int k = 0; k < nseg; ++k) {
                 gk.push_back(cap[k]);

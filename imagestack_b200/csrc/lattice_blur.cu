@@ -96,8 +96,9 @@ int blur_all_axes(const BlurPlan& p, cudaStream_t st) {
                 hflip ^= 1;
             }
             BlurArgs ba;
-            ba.nbrA = p.nbr + (size_t)j * p.nbr_stride;
+            ba.nbrA = p.nbr + 2 * (size_t)j * p.nbr_stride;
             ba.nbrB = nullptr;
+            ba.nbr_stride = p.nbr_stride;
             ba.nverts = p.nverts;
             ba.src = cur;
             ba.dst = dst;
@@ -121,8 +122,9 @@ int blur_all_axes(const BlurPlan& p, cudaStream_t st) {
         const int step = pair ? 2 : 1;
         const bool last = j + step >= axes;
         BlurArgs ba;
-        ba.nbrA = p.nbr + (size_t)j * p.nbr_stride;
-        ba.nbrB = pair ? p.nbr + (size_t)(j + 1) * p.nbr_stride : nullptr;
+        ba.nbrA = p.nbr + 2 * (size_t)j * p.nbr_stride;
+        ba.nbrB = pair ? p.nbr + 2 * (size_t)(j + 1) * p.nbr_stride : nullptr;
+        ba.nbr_stride = p.nbr_stride;
         ba.nverts = p.nverts;
         ba.src = src;
         ba.dst = last ? p.sval : p.bufs[flip];

@@ -299,6 +299,37 @@ __device__ __forceinline__ int ck_find(const typename CompactKey<D>::T* tab, uin
     return -1;
 }
 
+// a slot's tag: odd, from hash bits that the home sector does not use
+__device__ __forceinline__ uint8_t ck_tag(uint32_t mix) { return (uint8_t)(ck_fold(mix) | 1u); }
+
+// the slot of a 128-bit key by the slots' tags, from slot s (a sector's first) on; word: the
+// eight tags that hold s's.  -1 if absent.  Slots of a sector fill in order, so tags behind the
+// first empty one are not the key's.
+__device__ __forceinline__ int ck_find_tagged(const uint4* tab, const uint64_t* tags, uint32_t cap, const uint4& key,
+                                              uint32_t s, uint64_t word) {
+    constexpr uint64_t kOnes = 0x0101010101010101ull, kTops = 0x8080808080808080ull;
+    const uint64_t tag = ck_tag(ck_mix(key)) * kOnes;
+#pragma unroll 1
+    for (int probe = 0; probe < kMaxProbe / 8; ++probe) {
+        const uint32_t sh = (s & 7u) * 8u;
+        // tags from s on, low byte first; behind the word's end, neither empty nor any key's
+        const uint64_t x = sh ? (word >> sh) | (0x0202020202020202ull << (64u - sh)) : word;
+        const uint64_t empty = (x - kOnes) & ~x & kTops;   // lowest set: the first zero byte
+        const uint64_t y = x ^ tag;
+        uint64_t match = (y - kOnes) & ~y & kTops;         // bytes equal to the tag (and perhaps some above)
+        if (empty) match &= (empty & (0 - empty)) - 1;
+        for (; match; match &= match - 1) {
+            const uint32_t at = s + ((uint32_t)(__ffsll((long long)match) - 1) >> 3);
+            if (words_equal(__ldg(tab + at), key)) return (int)at;
+        }
+        if (empty) return -1;
+        s = (s | 7u) + 1u;
+        if (s >= cap) s = 0;
+        word = __ldg(tags + (s >> 3));
+    }
+    return -1;
+}
+
 // ---------------------------------------------------------------------------------
 // simplex
 // ---------------------------------------------------------------------------------
@@ -392,15 +423,15 @@ struct CompactSplatArgs {
     uint32_t tile_blocks;  // tile splat blocks of the batch
     // The vertices, numbered in the order the splat creates them (null with ft, whose vertices
     // are numbered afterwards, by first touch): the creator writes a vertex's key and slot,
-    // marks its neighbour pairs absent (nbr_init, d+1 axes, nbr_stride apart), and
-    // leaves the number at the slot.
+    // marks its lower neighbours absent (nbr_init), and leaves the number at the slot.
     uint32_t* vcount;      // vertices so far
     uint32_t* seg_counts;  // per segment (batches of several)
     void* vkey;
     uint32_t* vtx2slot;
     uint32_t* slot2vtx;    // number_rows: all ones before
-    int2* nbr_init;
+    int* nbr_init;         // as CompactNbrArgs::nbr
     uint32_t nbr_stride;
+    uint8_t* tags;         // optional tag per slot (CompactNbrArgs), zeros before
     // rows by vertex: the splat looks up each vertex's number (waiting, where another
     // warp created it a moment ago) and adds to rows[number]; otherwise to rows[slot]
     int number_rows;
@@ -412,7 +443,8 @@ __device__ __forceinline__ void publish_vertex(const CompactSplatArgs& a, uint32
     reinterpret_cast<typename CompactKey<D>::T*>(a.vkey)[v] = key;
     a.vtx2slot[v] = slot;
     if (a.nbr_init)
-        for (int j = 0; j <= D; ++j) a.nbr_init[(size_t)j * a.nbr_stride + v] = make_int2(-1, -1);
+        for (int j = 0; j <= D; ++j) a.nbr_init[(size_t)(2 * j + 1) * a.nbr_stride + v] = -1;
+    if (D > 7 && a.tags) a.tags[slot] = ck_tag(ck_mix(key));
     // rows were zeroed before the launch and a reader of the number uses nothing else the
     // creator wrote, so no fence orders these stores
     __stcg(a.slot2vtx + slot, v);
@@ -798,12 +830,19 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile
 // d >= 8.  The probes of kAhead remainders are in flight together.
 // ---------------------------------------------------------------------------------
 constexpr int kDirectThreads = 128;
+#ifndef PGPU_DIRECT_MB
+#define PGPU_DIRECT_MB 6
+#endif
+#ifndef PGPU_DIRECT_AH
+#define PGPU_DIRECT_AH 2
+#endif
+__host__ __device__ constexpr int direct_min_blocks(int d) { return d <= 7 ? 6 : PGPU_DIRECT_MB; }
 template <int D>
-__host__ __device__ constexpr int direct_ahead() { return D <= 7 ? (D + 1 < 4 ? D + 1 : 4) : 4; }
+__host__ __device__ constexpr int direct_ahead() { return D <= 7 ? (D + 1 < 4 ? D + 1 : 4) : PGPU_DIRECT_AH; }
 __host__ __device__ constexpr size_t direct_smem_bytes(int d) { return (size_t)(d + 1) * kDirectThreads * 12; }
 
 template <int D, int VDP>
-__global__ void __launch_bounds__(kDirectThreads) compact_direct_kernel(CompactSplatArgs a) {
+__global__ void __launch_bounds__(kDirectThreads, direct_min_blocks(D)) compact_direct_kernel(CompactSplatArgs a) {
     using K = CompactKey<D>;
     using T = typename K::T;
     constexpr int AH = direct_ahead<D>();
@@ -882,17 +921,19 @@ __global__ void __launch_bounds__(kDirectThreads) compact_direct_kernel(CompactS
         }
     }
     if (a.vcount) {
-        const uint32_t n = (uint32_t)__popc(mine), end = warp_sum_to(n, lane);
+        // numbered remainder by remainder, so that a warp's stores to vertex order are runs
+        const uint32_t end = warp_sum_to((uint32_t)__popc(mine), lane);
         uint32_t at = 0;
         if (lane == 31) at = reserve_numbers(a, kseg, end);
-        at = __shfl_sync(0xFFFFFFFFu, at, 31) + end - n;
-        if (mine) {
-            T key = first;
+        at = __shfl_sync(0xFFFFFFFFu, at, 31);
+        T key = first;
 #pragma unroll 1
-            for (int r = 0; r <= D; ++r) {
-                if (r > 0) ck_step<D>(key, scr[(D - (r - 1)) * kDirectThreads].y, r - 1);
-                if ((mine >> r) & 1u) publish_vertex<D>(a, s_row[r * kDirectThreads], at++, key);
-            }
+        for (int r = 0; r <= D; ++r) {
+            const bool made = (mine >> r) & 1u;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, made);
+            if (valid && r > 0) ck_step<D>(key, scr[(D - (r - 1)) * kDirectThreads].y, r - 1);
+            if (made) publish_vertex<D>(a, s_row[r * kDirectThreads], at + __popc(m & ((1u << lane) - 1u)), key);
+            at += __popc(m);
         }
     }
 }
@@ -910,8 +951,9 @@ struct CompactRankArgs {
     void* vkey;
     uint32_t* vtx2slot;
     uint32_t* slot2vtx;
-    int2* nbr_init;
+    int* nbr_init;
     uint32_t nbr_stride;
+    uint8_t* tags;
     uint4* wide0;          // the int16-lane keys in vertex order: word 0 ...
     uint4* widen;          // ... and later words, (KW-1) x wide_stride
     uint32_t wide_stride;
@@ -929,7 +971,8 @@ __global__ void compact_rank_kernel(CompactRankArgs a) {
         a.vtx2slot[v] = s;
         a.slot2vtx[s] = v;
         if (a.nbr_init)
-            for (int j = 0; j <= D; ++j) a.nbr_init[(size_t)j * a.nbr_stride + v] = make_int2(-1, -1);
+            for (int j = 0; j <= D; ++j) a.nbr_init[(size_t)(2 * j + 1) * a.nbr_stride + v] = -1;
+        if (a.tags) a.tags[s] = ck_tag(ck_mix(key));
         Key<key_words(D)> k;
         ck_widen<D>(key, k);
         a.wide0[v] = k.w[0];
@@ -953,11 +996,15 @@ struct CompactNbrArgs {
     const uint32_t* vtx2slot;
     const uint32_t* slot2vtx;
     const uint32_t* nverts;
-    int2* nbr;             // (d+1) x stride pairs
+    int* nbr;              // neighbours of axis j: up (n1) at 2j*stride, down (n2) at (2j+1)*stride
     uint32_t stride;
-    // one lookup per axis: vertex v finds u = n1(v) and, as n2(u) = v, writes v into u's pair
-    // too; every pair holds (-1, -1) beforehand
+    // one lookup per axis: vertex v finds u = n1(v) and, as n2(u) = v, writes v as u's lower
+    // neighbour; every lower neighbour is -1 beforehand
     int half;
+    // One byte per slot, 0 where empty, else from the key's hash (d >= 8): most neighbours of
+    // those lattices are absent and their keys lie all over a table larger than L2, while
+    // the tags stay in L2 and tell all but 1 in 100 of the absent ones.
+    const uint8_t* tags;
     // the splat's rows (slot space, FP32) copied into vertex order: as they are, rounded to
     // 16 bits, or (homogeneous rows) normalised by their weight, (m_0.., w); kRowsInPlace
     // with rows_in set: normalised in place (rows by vertex)
@@ -984,12 +1031,21 @@ __device__ __forceinline__ void gather_row(const CompactNbrArgs& a, uint32_t slo
     else store_row<VDP, float, float>(reinterpret_cast<float*>(a.rows_out), v, r);
 }
 
+#ifndef PGPU_NBR_MB
+#define PGPU_NBR_MB 4
+#endif
 template <int D>
-__global__ void compact_neighbours_kernel(CompactNbrArgs a) {
+__global__ void __launch_bounds__(256, D <= 7 ? 3 : PGPU_NBR_MB) compact_neighbours_kernel(CompactNbrArgs a) {
     using K = CompactKey<D>;
     using T = typename K::T;
     // axes whose probes are in flight together
-    constexpr int AH = D <= 7 ? (D + 1) : 4;
+#ifndef PGPU_NBR_AH
+#define PGPU_NBR_AH 6
+#endif
+#ifndef PGPU_NBR_MB
+#define PGPU_NBR_MB 4
+#endif
+    constexpr int AH = D <= 7 ? (D + 1) : PGPU_NBR_AH;
     const uint32_t m = *a.nverts;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
         const T key = reinterpret_cast<const T*>(a.vkey)[v];
@@ -999,8 +1055,9 @@ __global__ void compact_neighbours_kernel(CompactNbrArgs a) {
         // a lattice whose splat failed is rerun by the host: its full table would make every
         // lookup of an absent key probe to the limit, so skip it
         if (__ldcg(a.seg_status + kseg) & kStatusFailed) {
-            if (!a.half)
-                for (int j = 0; j <= D; ++j) a.nbr[(size_t)j * a.stride + v] = make_int2(-1, -1);
+            // (its vertices still take part in the blur: none may be left a stale neighbour)
+            for (int j = 0; j < 2 * (D + 1); ++j)
+                if (!a.half || j % 2 == 0) a.nbr[(size_t)j * a.stride + v] = -1;
             continue;
         }
         if (a.rows_in) {
@@ -1011,28 +1068,34 @@ __global__ void compact_neighbours_kernel(CompactNbrArgs a) {
         const uint32_t base = __ldg(a.seg_slot_base + kseg);
         const uint32_t sectors = (__ldg(a.seg_slot_base + kseg + 1) - base) / K::kBucket;
         const T* tab = reinterpret_cast<const T*>(a.keys) + base;
+        const uint64_t* tags = reinterpret_cast<const uint64_t*>(a.tags + (K::kOneWord ? 0 : base));
 #pragma unroll 1
         for (int sign = 1; sign >= (a.half ? 1 : -1); sign -= 2) {
             const T all = ck_shift_all<D>(key, sign);
 #pragma unroll
             for (int j0 = 0; j0 <= D; j0 += AH) {
                 T in[AH][K::kBucket];
+                uint64_t word[AH];
                 uint32_t b[AH];
 #pragma unroll
                 for (int j = 0; j < AH; ++j) {
                     if (j0 + j > D) break;
                     const T k = ck_axis<D>(all, j0 + j, sign);
                     b[j] = __umulhi(ck_fold(ck_mix(k)), sectors);
-                    read_sector(tab + (size_t)b[j] * K::kBucket, in[j]);
+                    if constexpr (K::kOneWord) read_sector(tab + (size_t)b[j] * K::kBucket, in[j]);
+                    else word[j] = __ldg(tags + (b[j] * K::kBucket >> 3));
                 }
 #pragma unroll
                 for (int j = 0; j < AH; ++j) {
                     if (j0 + j > D) break;
-                    const int s = ck_find<D>(tab, sectors, ck_axis<D>(all, j0 + j, sign), b[j], in[j]);
+                    const T k = ck_axis<D>(all, j0 + j, sign);
+                    int s;
+                    if constexpr (K::kOneWord) s = ck_find<D>(tab, sectors, k, b[j], in[j]);
+                    else s = ck_find_tagged(tab, tags, sectors * K::kBucket, k, b[j] * K::kBucket, word[j]);
                     const int u = s >= 0 ? (int)__ldg(a.slot2vtx + base + s) : -1;
-                    int* pair = reinterpret_cast<int*>(a.nbr + (size_t)(j0 + j) * a.stride);
-                    pair[2 * (size_t)v + (sign > 0 ? 0 : 1)] = u;
-                    if (a.half && u >= 0) pair[2 * (size_t)u + 1] = (int)v;
+                    int* nbr = a.nbr + (size_t)(2 * (j0 + j)) * a.stride;
+                    nbr[(sign > 0 ? 0 : (size_t)a.stride) + v] = u;
+                    if (a.half && u >= 0) nbr[(size_t)a.stride + u] = (int)v;
                 }
             }
         }

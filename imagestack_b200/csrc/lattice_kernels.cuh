@@ -206,9 +206,9 @@ struct CompactArgs {
     const uint32_t* vlist = nullptr;    // the splat's vertex list (list order), or null:
     const uint32_t* nverts = nullptr;   // first-touch order through ft and the bitmap
     int index_in_key = 0;   // store each vertex's index in its key word (d <= 6)
-    // optional: mark every vertex's neighbour pairs absent (nbr_axes axes, nbr_stride apart)
+    // optional: mark every vertex's lower neighbours absent (nbr_axes axes, as NbrArgs::nbr)
     // for the neighbour search that looks up one direction per axis
-    int2* nbr_init = nullptr;
+    int* nbr_init = nullptr;
     uint32_t nbr_stride = 0;
     int nbr_axes = 0;
 };
@@ -225,19 +225,20 @@ struct NbrArgs {
     const uint4* vkeyn;
     uint32_t vcap;
     const uint32_t* nverts;
-    int2* nbr;             // (d+1) x vcap pairs
+    int* nbr;              // neighbours of axis j: up (n1) at 2j*vcap, down (n2) at (2j+1)*vcap
     const uint8_t* tags = nullptr;   // slot tags of the compaction, or null: plain lookups
     const unsigned* seg_status = nullptr;   // the splat's per-segment status, or null
-    // one lookup per axis: vertex v finds u = n1(v) and, as n2(u) = v, writes v into u's
-    // pair too; every pair must hold (-1, -1) beforehand (written by the compaction)
+    // one lookup per axis: vertex v finds u = n1(v) and, as n2(u) = v, writes v as u's lower
+    // neighbour; every lower neighbour must be -1 beforehand (written by the compaction)
     int half = 0;
 };
 
 // One launch blurs along one axis (nbrA) or, fused, along two consecutive axes (nbrA then
 // nbrB): the first axis's result stays in registers instead of being stored and reloaded.
 struct BlurArgs {
-    const int2* nbrA;           // neighbours along the first axis of the pass
-    const int2* nbrB;           // neighbours along the second axis (fused passes)
+    const int* nbrA;            // neighbours along the first axis of the pass: up, and nbr_stride on, down
+    const int* nbrB;            // neighbours along the second axis (fused passes)
+    size_t nbr_stride;
     const uint32_t* nverts;
     const void* src;            // rows in vertex order
     void* dst;                  // rows in vertex order, or in slot space with dst_map
@@ -637,7 +638,7 @@ __device__ __forceinline__ void assign_vertex(const CompactArgs& a, uint32_t s, 
     a.slot2vtx[s] = vtx;
     a.vtx2slot[vtx] = s;
     if (a.nbr_init)
-        for (int j = 0; j < a.nbr_axes; ++j) a.nbr_init[(size_t)j * a.nbr_stride + vtx] = make_int2(-1, -1);
+        for (int j = 0; j < a.nbr_axes; ++j) a.nbr_init[(size_t)(2 * j + 1) * a.nbr_stride + vtx] = -1;
     const uint4 k0 = a.table.key0[s];
     a.vkey0[vtx] = k0;
     if (KW == 1 && a.index_in_key) a.table.key0[s] = make_uint4(k0.x, k0.y, k0.z, enc_index(vtx));
@@ -751,8 +752,9 @@ __global__ void neighbours_kernel(NbrArgs a) {
         // a lattice whose splat overflowed is rerun by the host: its full table would make
         // every lookup of an absent key probe to the limit, so skip it
         if (a.seg_status && (__ldcg(a.seg_status + kseg) & (kStatusProbeLimit | kStatusSpinLimit))) {
-            if (!a.half)
-                for (int j = 0; j <= D; ++j) a.nbr[(size_t)j * a.vcap + vtx] = make_int2(-1, -1);
+            // (its vertices still take part in the blur: none may be left a stale neighbour)
+            for (int j = 0; j < 2 * (D + 1); ++j)
+                if (!a.half || j % 2 == 0) a.nbr[(size_t)j * a.vcap + vtx] = -1;
             continue;
         }
         const uint32_t base = __ldg(a.seg_slot_base + kseg);
@@ -770,9 +772,8 @@ __global__ void neighbours_kernel(NbrArgs a) {
                 Key<KW> k1;
                 neighbour_key<D>(key, j, +1, k1);
                 const int u1 = neighbour_index<D>(a, table, base, k1);
-                int* pair = reinterpret_cast<int*>(a.nbr + (size_t)j * a.vcap);
-                pair[2 * (size_t)vtx] = u1;
-                if (u1 >= 0) pair[2 * (size_t)u1 + 1] = (int)vtx;
+                a.nbr[(size_t)(2 * j) * a.vcap + vtx] = u1;
+                if (u1 >= 0) a.nbr[(size_t)(2 * j + 1) * a.vcap + u1] = (int)vtx;
             }
             continue;
         }
@@ -785,7 +786,8 @@ __global__ void neighbours_kernel(NbrArgs a) {
             neighbour_key<D>(key, j, -1, k2);
             const int u1 = neighbour_index<D>(a, table, base, k1);
             const int u2 = neighbour_index<D>(a, table, base, k2);
-            a.nbr[(size_t)j * a.vcap + vtx] = make_int2(u1, u2);
+            a.nbr[(size_t)(2 * j) * a.vcap + vtx] = u1;
+            a.nbr[(size_t)(2 * j + 1) * a.vcap + vtx] = u2;
         }
     }
 }
@@ -884,16 +886,23 @@ __device__ __forceinline__ void combine3(const A (&r1)[VDP], const A (&r0)[VDP],
     }
 }
 
+// the neighbours of vertex u along an axis: up and down.  They lie in arrays of their own: the
+// search writes every up neighbour in whole sectors, and only the down neighbours need marking
+// absent beforehand.
+__device__ __forceinline__ int2 load_pair(const int* nbr, size_t stride, uint32_t u) {
+    return make_int2(__ldg(nbr + u), __ldg(nbr + stride + u));
+}
+
 // the first-axis blur at vertex u (zeros when u is absent)
 template <int VDP, typename PS, typename A, bool HOMOG>
-__device__ __forceinline__ void blurred_row(const PS* src, const int2* nbr, int u, int wc,
+__device__ __forceinline__ void blurred_row(const PS* src, const int* nbr, size_t stride, int u, int wc,
                                             A (&out)[VDP]) {
     if (u < 0) {
 #pragma unroll
         for (int k = 0; k < VDP; ++k) out[k] = (A)0;
         return;
     }
-    const int2 nb = __ldg(nbr + u);
+    const int2 nb = load_pair(nbr, stride, (uint32_t)u);
     A r1[VDP], r0[VDP], r2[VDP];
     load_row<VDP, PS, A>(src, nb.x, r1);
     load_row<VDP, PS, A>(src, u, r0);
@@ -936,18 +945,18 @@ __global__ void blur_kernel(BlurArgs a) {
     for (uint32_t vtx = blockIdx.x * blockDim.x + threadIdx.x; vtx < m; vtx += stride * ILP) {
         A out[VDP];
         if constexpr (PAIR) {
-            const int2 nb = __ldg(a.nbrB + vtx);
+            const int2 nb = load_pair(a.nbrB, a.nbr_stride, vtx);
             A r1[VDP], r0[VDP], r2[VDP];
-            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, nb.x, a.wc, r1);
-            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, (int)vtx, a.wc, r0);
-            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, nb.y, a.wc, r2);
+            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, a.nbr_stride, nb.x, a.wc, r1);
+            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, a.nbr_stride, (int)vtx, a.wc, r0);
+            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, a.nbr_stride, nb.y, a.wc, r2);
             combine3<VDP, A, HOMOG>(r1, r0, r2, a.wc, out);
             put_row<VDP, PD, A, HOMOG>(a, dst, vtx, out);
         } else if constexpr (ILP == 2) {
             const uint32_t v2 = vtx + stride;
             const bool two = v2 < m;
-            const int2 na = __ldg(a.nbrA + vtx);
-            const int2 nb = two ? __ldg(a.nbrA + v2) : make_int2(-1, -1);
+            const int2 na = load_pair(a.nbrA, a.nbr_stride, vtx);
+            const int2 nb = two ? load_pair(a.nbrA, a.nbr_stride, v2) : make_int2(-1, -1);
             A p1[VDP], p0[VDP], p2[VDP], q1[VDP], q0[VDP], q2[VDP];
             load_row<VDP, PS, A>(src, na.x, p1);
             load_row<VDP, PS, A>(src, (int)vtx, p0);
@@ -963,7 +972,7 @@ __global__ void blur_kernel(BlurArgs a) {
                 put_row<VDP, PD, A, HOMOG>(a, dst, v2, out2);
             }
         } else {
-            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, (int)vtx, a.wc, out);
+            blurred_row<VDP, PS, A, HOMOG>(src, a.nbrA, a.nbr_stride, (int)vtx, a.wc, out);
             put_row<VDP, PD, A, HOMOG>(a, dst, vtx, out);
         }
     }

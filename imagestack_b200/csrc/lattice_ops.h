@@ -69,7 +69,7 @@ bool launch_blur(const BlurArgs& a, int blocks, int ilp, int vdp, int payload, b
 struct BlurPlan {
     int d, vdp, payload;
     bool homog, src_f32;
-    const int2* nbr;       // (d+1) x nbr_stride neighbour pairs
+    const int* nbr;        // neighbours of axis j: up at 2j*nbr_stride, down at (2j+1)*nbr_stride
     size_t nbr_stride;
     const uint32_t* nverts;
     uint32_t vmax;

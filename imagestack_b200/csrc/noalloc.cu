@@ -234,7 +234,7 @@ extern "C" int pgpu_bilateral_noalloc(const float* d_in, float* d_out, int width
     na.vkeyn = (const uint4*)(base + kOffVkey0);
     na.vcap = cap;
     na.nverts = dM;
-    na.nbr = (int2*)(base + kOffNbr);
+    na.nbr = (int*)(base + kOffNbr);
     ops->neighbours(na, cap, sms, st);
 
     BlurPlan bp;
@@ -243,7 +243,7 @@ extern "C" int pgpu_bilateral_noalloc(const float* d_in, float* d_out, int width
     bp.payload = kPayloadF32;
     bp.homog = false;
     bp.src_f32 = false;
-    bp.nbr = (const int2*)(base + kOffNbr);
+    bp.nbr = (const int*)(base + kOffNbr);
     bp.nbr_stride = cap;
     bp.nverts = dM;
     bp.vmax = cap;
