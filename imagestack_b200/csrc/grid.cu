@@ -5,16 +5,18 @@
 // into the 2^d corners of each point's cell, two [1 2 1]/4 passes per dimension (taps 5),
 // and multilinear slicing.
 //
-//   preview  min and max of every scaled position coordinate (block reduction, then
-//            order-preserving integer atomics: exact in any order)
-//   splat    one thread per point; FP32 atomics into the corners (the reference adds in
-//            point order, so sums agree to rounding)
+//   preview  min and max of every scaled guide channel (block reduction, then
+//            order-preserving integer atomics: exact in any order); pixel coordinates grow
+//            with the pixel, so the host takes theirs from the image's ends
+//   splat    one to four pixels per thread; FP32 reductions into the corners (the reference
+//            adds in point order, so sums agree to rounding)
 //   blur     one launch per dimension, one thread per grid value: the reference's two
 //            in-place passes (src/DenseGrid.h:199-236) evaluated out of place, cell by cell,
 //            with their exact arithmetic, including the last cell's double-precision step
 //   slice    one thread per point; the corners gathered in the reference's order
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -34,8 +36,12 @@ struct GridArgs {
     float sf;                            // scaleFactor, the same in every dimension
     float minp[kGridMaxD];               // minPosition
     int sizes[kGridMaxD];
-    long long stride[kGridMaxD + 1];     // stride[0] = vd
+    uint32_t stride[kGridMaxD + 1];      // stride[0] = vd; grids hold at most 2^30 values
     float* grid;
+    // Splat in pairs (two values per cell): grid[2*offset..] holds, for the cell at offset, its
+    // own two values and what its points add to the next cell along dimension 0, so that
+    // a point's two corners there take one reduction of four floats.
+    int pairs;
 };
 
 // float <-> unsigned mapping that preserves order, for min/max by integer atomics
@@ -50,10 +56,12 @@ float unordered_float(unsigned u) {
     return f;
 }
 
-// DenseGrid::preview (src/DenseGrid.h:142-160): the bounding box of position * scaleFactor
+// DenseGrid::preview (src/DenseGrid.h:142-160): the bounding box of position * scaleFactor, guide
+// channels only.  Blocks stride over pieces of kMinmaxPixels pixels of a row.
+constexpr uint32_t kMinmaxPixels = 4 * kGridThreads;
 template <int D>
-__global__ void __launch_bounds__(kGridThreads) grid_minmax_kernel(PointSource src, uint32_t n, float sf,
-                                                                   unsigned* mm) {
+__global__ void __launch_bounds__(kGridThreads) grid_minmax_kernel(PointSource src, float sf, uint32_t pieces,
+                                                                   uint32_t total, unsigned* mm) {
     __shared__ unsigned smin[D], smax[D];
     if (threadIdx.x < D) {
         smin[threadIdx.x] = 0xFFFFFFFFu;
@@ -63,30 +71,35 @@ __global__ void __launch_bounds__(kGridThreads) grid_minmax_kernel(PointSource s
     unsigned lo[D], hi[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) lo[c] = 0xFFFFFFFFu, hi[c] = 0u;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float p[D];
-        load_position<D>(src, i, p);
+    for (uint32_t b = blockIdx.x; b < total; b += gridDim.x) {
+        const uint32_t row = b / pieces, x0 = (b - row * pieces) * kMinmaxPixels + threadIdx.x;
+        const uint32_t t = row / (uint32_t)src.height, y = row - t * (uint32_t)src.height;
+        const float* at = src.pos.base + (long long)t * src.pos.tstride + (long long)y * src.pos.ystride;
 #pragma unroll
-        for (int c = 0; c < D; ++c) {
-            const unsigned o = ordered_bits(__fmul_rn(p[c], sf));
-            lo[c] = min(lo[c], o);
-            hi[c] = max(hi[c], o);
+        for (int c = 0; c < D; ++c, at += src.pos.cstride) {
+            if (c >= src.pos_channels) break;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t x = x0 + k * kGridThreads;
+                if (x >= (uint32_t)src.width) break;
+                const unsigned o = ordered_bits(__fmul_rn(__fmul_rn(__ldg(at + x), src.pos_scale[c]), sf));
+                lo[c] = min(lo[c], o);
+                hi[c] = max(hi[c], o);
+            }
         }
     }
 #pragma unroll
     for (int c = 0; c < D; ++c) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[c] = min(lo[c], __shfl_xor_sync(0xFFFFFFFFu, lo[c], o));
-            hi[c] = max(hi[c], __shfl_xor_sync(0xFFFFFFFFu, hi[c], o));
-        }
+        if (c >= src.pos_channels) break;
+        lo[c] = __reduce_min_sync(0xFFFFFFFFu, lo[c]);
+        hi[c] = __reduce_max_sync(0xFFFFFFFFu, hi[c]);
         if ((threadIdx.x & 31u) == 0) {
             atomicMin(&smin[c], lo[c]);
             atomicMax(&smax[c], hi[c]);
         }
     }
     __syncthreads();
-    if (threadIdx.x < D) {
+    if ((int)threadIdx.x < src.pos_channels) {
         atomicMin(&mm[threadIdx.x], smin[threadIdx.x]);
         atomicMax(&mm[D + threadIdx.x], smax[threadIdx.x]);
     }
@@ -110,58 +123,65 @@ __device__ __forceinline__ void grid_cell(const GridArgs& g, const float (&p)[D]
 // past the grid's last cell has weight exactly 0 (the point lies on the last plane) and is
 // skipped, as DenseGrid::query's bounds checks do.
 template <int D>
-__device__ __forceinline__ bool grid_base(const GridArgs& g, const int (&I)[D], long long& base, unsigned& hi_ok) {
+__device__ __forceinline__ bool grid_base(const GridArgs& g, const int (&I)[D], uint32_t& base, unsigned& hi_ok) {
     base = 0;
     hi_ok = 0;
     bool ok = true;
 #pragma unroll
     for (int j = 0; j < D; ++j) {
         ok = ok && I[j] >= 0 && I[j] < g.sizes[j];
-        base += (long long)I[j] * g.stride[j];
+        base += (uint32_t)I[j] * g.stride[j];
         if (I[j] + 1 < g.sizes[j]) hi_ok |= 1u << j;
     }
     return ok;
 }
 
 // Corner `corner` of the cell (unrolled by the caller): its weight in the reference's
-// product order and its offset from the cell's base.
+// product order and its offset from the cell's base.  (Corners share the first products.)
 template <int D>
-__device__ __forceinline__ float grid_corner_weight(const GridArgs& g, const float (&F)[D], const float (&Fi)[D],
-                                                    int corner, long long base, long long& off) {
-    float w = 1.0f;
-    off = base;
+__device__ __forceinline__ float grid_corner_weight(const float (&F)[D], const float (&Fi)[D], int corner) {
+    float w = (corner & 1) ? F[0] : Fi[0];   // 1 * it
 #pragma unroll
-    for (int j = 0; j < D; ++j) {
-        const bool up = (corner >> j) & 1;
-        w = __fmul_rn(w, up ? F[j] : Fi[j]);
-        if (up) off += g.stride[j];
-    }
+    for (int j = 1; j < D; ++j) w = __fmul_rn(w, ((corner >> j) & 1) ? F[j] : Fi[j]);
     return w;
+}
+template <int D>
+__device__ __forceinline__ uint32_t grid_corner_offset(const GridArgs& g, int corner) {
+    uint32_t off = 0;
+#pragma unroll
+    for (int j = 0; j < D; ++j)
+        if ((corner >> j) & 1) off += g.stride[j];
+    return off;
 }
 
 // Blocks of the splat and slice: tiles of (bw * kp) x (kGridThreads/bw) pixels of one frame
 // (bw = 32 for images, kGridThreads for point lists of one row; kp consecutive pixels of a
 // row per thread), so a thread finds its pixels without dividing.
 struct PixelTiles {
-    unsigned bw;
+    unsigned bshift;   // log2 of bw
     dim3 grid;
 };
 PixelTiles pixel_tiles(const PointSource& s, unsigned kp) {
     PixelTiles t;
-    t.bw = s.height == 1 ? (unsigned)kGridThreads : 32u;
-    const unsigned bh = kGridThreads / t.bw, w = t.bw * kp;
+    t.bshift = s.height == 1 ? 8u : 5u;
+    static_assert(kGridThreads == 256, "bw of a one-row tile");
+    const unsigned bw = 1u << t.bshift, bh = kGridThreads / bw, w = bw * kp;
     t.grid = dim3(((unsigned)s.width + w - 1) / w, ((unsigned)s.height + bh - 1) / bh, (unsigned)s.frames);
     return t;
 }
 
-// the splat's atomic of one corner: VD values of a cell are 8- or 16-byte aligned when VD is
-// 2 or 4, so one vector atomic adds them; otherwise one float atomic per value
+// the splat's reduction of one corner: VD values of a cell are 8- or 16-byte aligned when VD is
+// 2 or 4, so one vector reduction adds them; otherwise one float atomic per value
+__device__ __forceinline__ void red4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :: "l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
 template <int VD>
-__device__ __forceinline__ void grid_add(const GridArgs& g, long long off, const float* c) {
+__device__ __forceinline__ void grid_add(const GridArgs& g, uint32_t off, const float* c) {
     if constexpr (VD == 2) {
-        atomicAdd(reinterpret_cast<float2*>(g.grid + off), make_float2(c[0], c[1]));
+        asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" :: "l"(g.grid + off), "f"(c[0]), "f"(c[1]) : "memory");
     } else if constexpr (VD == 4) {
-        atomicAdd(reinterpret_cast<float4*>(g.grid + off), make_float4(c[0], c[1], c[2], c[3]));
+        red4(g.grid + off, c[0], c[1], c[2], c[3]);
     } else {
 #pragma unroll
         for (int k = 0; k < kGridMaxVd; ++k)
@@ -171,41 +191,48 @@ __device__ __forceinline__ void grid_add(const GridArgs& g, long long off, const
 
 // KP consecutive pixels of a row per thread.  With KP > 1 (small grids: the 2^D corners x
 // VD values fit in registers) a run of pixels that fall into the same cell is summed in
-// registers first and sent as one set of corner atomics: neighbouring pixels share cells,
-// and the splat is bound by the atomics' rate (4K grey d=3: 66 M float2 atomics).  The sums
-// differ from the reference's point-by-point additions only in rounding order.
-template <int D, int VD, int KP>
-__global__ void __launch_bounds__(kGridThreads) grid_splat_kernel(PointSource src, unsigned bw, GridArgs g) {
+// registers first and sent as one set of corner reductions: neighbouring pixels share cells,
+// and the splat is bound by the reductions' rate.  The sums differ from the reference's
+// point-by-point additions only in rounding order.  PAIRS: GridArgs::pairs, half as many
+// reductions (4K grey d=3: see run_grid).
+template <int D, int VD, int KP, bool PAIRS>
+__global__ void __launch_bounds__(kGridThreads) grid_splat_kernel(PointSource src, unsigned bshift, GridArgs g) {
+    static_assert(!PAIRS || (VD == 2 && KP > 1), "pairs hold two values per cell");
     constexpr int NC = 1 << D;
     constexpr int NV = VD > 0 ? VD : kGridMaxVd;
-    const uint32_t x0 = (blockIdx.x * bw + threadIdx.x % bw) * KP;
-    const uint32_t y = blockIdx.y * (kGridThreads / bw) + threadIdx.x / bw;
+    const uint32_t x0 = ((blockIdx.x << bshift) + (threadIdx.x & ((1u << bshift) - 1u))) * KP;
+    const uint32_t y = blockIdx.y * (kGridThreads >> bshift) + (threadIdx.x >> bshift);
     if (x0 >= (uint32_t)src.width || y >= (uint32_t)src.height) return;
     float acc[KP > 1 ? NC : 1][NV];
-    long long run_base = -1;
+    uint32_t run_base = 0xFFFFFFFFu;   // no run: no grid has this offset
     unsigned run_hi = 0;
     auto flush = [&]() {
-        if (run_base < 0) return;
+        if (run_base == 0xFFFFFFFFu) return;
 #pragma unroll
         for (int corner = 0; corner < NC; ++corner) {
+            if (PAIRS && (corner & 1)) continue;
             if (corner & ~run_hi) continue;
-            long long off = run_base;
-#pragma unroll
-            for (int j = 0; j < D; ++j)
-                if ((corner >> j) & 1) off += g.stride[j];
-            grid_add<VD>(g, off, acc[KP > 1 ? corner : 0]);
+            const uint32_t off = run_base + grid_corner_offset<D>(g, corner);
+            // (the next cell's half of a pair whose next cell lies outside is never read)
+            if constexpr (PAIRS) {
+                const float* lo = acc[KP > 1 ? corner : 0];
+                const float* hi = acc[KP > 1 ? corner + 1 : 0];
+                red4(g.grid + 2 * (size_t)off, lo[0], lo[1], hi[0], hi[1]);
+            } else {
+                grid_add<VD>(g, off, acc[KP > 1 ? corner : 0]);
+            }
         }
     };
 #pragma unroll
     for (int kp = 0; kp < KP; ++kp) {
         const uint32_t x = x0 + kp;
         if (x >= (uint32_t)src.width) break;
-        float p[D], v[kGridMaxVd];
-        load_point_xyt<D, kGridMaxVd>(src, x, y, blockIdx.z, p, v);
+        float p[D], v[NV];
+        load_point_xyt<D, NV>(src, x, y, blockIdx.z, p, v);
         int I[D];
         float F[D], Fi[D];
         grid_cell<D>(g, p, I, F, Fi);
-        long long base;
+        uint32_t base;
         unsigned hi_ok;
         if (!grid_base<D>(g, I, base, hi_ok)) continue;
         if constexpr (KP > 1) {
@@ -220,8 +247,7 @@ __global__ void __launch_bounds__(kGridThreads) grid_splat_kernel(PointSource sr
             }
 #pragma unroll
             for (int corner = 0; corner < NC; ++corner) {
-                long long off;
-                const float w = grid_corner_weight<D>(g, F, Fi, corner, base, off);
+                const float w = grid_corner_weight<D>(F, Fi, corner);
 #pragma unroll
                 for (int k = 0; k < NV; ++k) acc[corner][k] = __fadd_rn(acc[corner][k], __fmul_rn(w, v[k]));
             }
@@ -229,12 +255,11 @@ __global__ void __launch_bounds__(kGridThreads) grid_splat_kernel(PointSource sr
 #pragma unroll
             for (int corner = 0; corner < NC; ++corner) {
                 if (corner & ~hi_ok) continue;
-                long long off;
-                const float w = grid_corner_weight<D>(g, F, Fi, corner, base, off);
+                const float w = grid_corner_weight<D>(F, Fi, corner);
                 float c[NV];
 #pragma unroll
                 for (int k = 0; k < NV; ++k) c[k] = __fmul_rn(w, v[k]);
-                grid_add<VD>(g, off, c);
+                grid_add<VD>(g, base + grid_corner_offset<D>(g, corner), c);
             }
         }
     }
@@ -255,24 +280,36 @@ __global__ void __launch_bounds__(kGridThreads) grid_splat_kernel(PointSource sr
 // from the five values around x.  One thread per grid value; consecutive threads are
 // consecutive values, so every access is coalesced whatever the dimension.
 __device__ __forceinline__ float grid_pass_value(float left, float here, float right, uint32_t x, uint32_t len) {
-    const float t1 = x == 0 ? __fdiv_rn(here, 2.0f) : __fmul_rn(0.5f, __fadd_rn(left, here));
+    // (here / 2 and 0.5 * here round alike)
+    const float t1 = x == 0 ? __fmul_rn(0.5f, here) : __fmul_rn(0.5f, __fadd_rn(left, here));
     if (x == len - 1) return (float)__dmul_rn(0.5, __dadd_rn((double)t1, __dmul_rn(0.5, (double)here)));
     return __fmul_rn(0.5f, __fadd_rn(t1, __fmul_rn(0.5f, __fadd_rn(here, right))));
 }
 
-__global__ void __launch_bounds__(kGridThreads) grid_blur_kernel(GridArgs g, int j, const float* src,
-                                                                 float* dst, uint32_t total) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;   // grids hold < 2^30 values
+// ms, ml: floor(2^32 / stride) and floor(2^32 / len) (div_magic).  pairs: dimension 0 of a grid
+// splatted in pairs.
+__global__ void __launch_bounds__(kGridThreads) grid_blur_kernel(const float* src, float* dst, uint32_t total,
+                                                                 uint32_t s, uint32_t ms, uint32_t len, uint32_t ml,
+                                                                 int pairs) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;   // grids hold at most 2^30 values
     if (t >= total) return;
-    const uint32_t s = (uint32_t)g.stride[j];
-    const uint32_t len = (uint32_t)g.sizes[j];
-    const uint32_t x = (t / s) % len;
+    uint32_t rem, x;
+    div_magic(div_magic(t, s, ms, &rem), len, ml, &x);
     // old values at x-2 .. x+2 (those outside the row are never used)
     float o[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
         const int xx = (int)x + k - 2;
-        o[k] = (xx >= 0 && xx < (int)len) ? src[(int64_t)t + (int64_t)(k - 2) * s] : 0.0f;
+        o[k] = 0.0f;
+        if (xx < 0 || xx >= (int)len) continue;
+        const int64_t at = (int64_t)t + (int64_t)(k - 2) * s;
+        if (pairs) {   // s == 2: the cell's own two values, and the previous cell's for it
+            const int64_t cell = at >> 1, c = at & 1;
+            o[k] = src[4 * cell + c];
+            if (xx > 0) o[k] = __fadd_rn(o[k], src[4 * (cell - 1) + 2 + c]);
+        } else {
+            o[k] = src[at];
+        }
     }
     // first pass at x-1, x, x+1, then the second pass at x
     float p1[3];
@@ -285,82 +322,114 @@ __global__ void __launch_bounds__(kGridThreads) grid_blur_kernel(GridArgs g, int
 }
 
 template <int D, int VD>
-__global__ void __launch_bounds__(kGridThreads) grid_slice_kernel(PointSource src, unsigned bw, GridArgs g,
+__global__ void __launch_bounds__(kGridThreads) grid_slice_kernel(PointSource src, unsigned bshift, GridArgs g,
                                                                   OutView out) {
-    const uint32_t x = blockIdx.x * bw + threadIdx.x % bw;
-    const uint32_t y = blockIdx.y * (kGridThreads / bw) + threadIdx.x / bw;
+    constexpr int NV = VD > 0 ? VD : kGridMaxVd;
+    const int vd = VD > 0 ? VD : g.vd;
+    const uint32_t x = (blockIdx.x << bshift) + (threadIdx.x & ((1u << bshift) - 1u));
+    const uint32_t y = blockIdx.y * (kGridThreads >> bshift) + (threadIdx.x >> bshift);
     if (x >= (uint32_t)src.width || y >= (uint32_t)src.height) return;
     float p[D];
     load_position_xyt<D>(src, x, y, blockIdx.z, p);
     int I[D];
     float F[D], Fi[D];
     grid_cell<D>(g, p, I, F, Fi);
-    float acc[kGridMaxVd];
+    float acc[NV];
 #pragma unroll
-    for (int k = 0; k < kGridMaxVd; ++k) acc[k] = 0.0f;
-    long long base;
+    for (int k = 0; k < NV; ++k) acc[k] = 0.0f;
+    uint32_t base;
     unsigned hi_ok;
     const bool inside = grid_base<D>(g, I, base, hi_ok);
 #pragma unroll
     for (int corner = 0; corner < (1 << D); ++corner) {
         if (!inside || (corner & ~hi_ok)) continue;
-        long long off;
-        const float w = grid_corner_weight<D>(g, F, Fi, corner, base, off);
-        float c[kGridMaxVd];
+        const float w = grid_corner_weight<D>(F, Fi, corner);
+        const float* cell = g.grid + base + grid_corner_offset<D>(g, corner);
+        float c[NV];
         if constexpr (VD == 2) {
-            const float2 q = __ldg(reinterpret_cast<const float2*>(g.grid + off));
+            const float2 q = __ldg(reinterpret_cast<const float2*>(cell));
             c[0] = q.x, c[1] = q.y;
         } else if constexpr (VD == 4) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(g.grid + off));
+            const float4 q = __ldg(reinterpret_cast<const float4*>(cell));
             c[0] = q.x, c[1] = q.y, c[2] = q.z, c[3] = q.w;
         } else {
 #pragma unroll
-            for (int k = 0; k < kGridMaxVd; ++k) c[k] = k < g.vd ? g.grid[off + k] : 0.0f;
+            for (int k = 0; k < NV; ++k) c[k] = k < vd ? cell[k] : 0.0f;
         }
 #pragma unroll
-        for (int k = 0; k < kGridMaxVd; ++k)
-            if (k < g.vd) acc[k] = __fadd_rn(acc[k], __fmul_rn(w, c[k]));
+        for (int k = 0; k < NV; ++k)
+            if (k < vd) acc[k] = __fadd_rn(acc[k], __fmul_rn(w, c[k]));
     }
     float* o = out.base + (long long)blockIdx.z * out.tstride + (long long)y * out.ystride + x;
     float wsum = acc[0];
 #pragma unroll
-    for (int k = 0; k < kGridMaxVd; ++k) if (k == g.vd - 1) wsum = acc[k];
+    for (int k = 0; k < NV; ++k) if (k == vd - 1) wsum = acc[k];
 #pragma unroll
-    for (int k = 0; k < kGridMaxVd; ++k)
+    for (int k = 0; k < NV; ++k)
         if (k < out.channels) o[(long long)k * out.cstride] = out.normalize ? acc[k] / wsum : acc[k];
 }
 
 template <int D>
-void launch_minmax(const PointSource& s, uint32_t n, float sf, unsigned* mm, int sms, cudaStream_t st) {
-    uint64_t blocks = (n + kGridThreads - 1) / kGridThreads;
-    if (blocks > (uint64_t)sms * 8) blocks = (uint64_t)sms * 8;
-    if (blocks < 1) blocks = 1;
-    grid_minmax_kernel<D><<<(unsigned)blocks, kGridThreads, 0, st>>>(s, n, sf, mm);
+void launch_minmax(const PointSource& s, float sf, unsigned* mm, int sms, cudaStream_t st) {
+    const uint32_t pieces = ((uint32_t)s.width + kMinmaxPixels - 1) / kMinmaxPixels;
+    const uint32_t total = pieces * (uint32_t)s.height * (uint32_t)s.frames;   // at most the points
+    const uint32_t blocks = std::min(total, (uint32_t)sms * 8u);
+    grid_minmax_kernel<D><<<blocks, kGridThreads, 0, st>>>(s, sf, pieces, total, mm);
+}
+// Pixels of a run are summed in registers where the corner sums fit (2^d x vd <= 16), and
+// pairs halve the reductions of two values per cell (4K grey d=3: 66 M reductions of two floats
+// one by one 0.90 ms, runs 0.23 ms, runs in pairs 0.11).
+bool splat_in_pairs(int d, int vd, long long values) {
+    return vd == 2 && d <= 3 && values <= (1LL << 28);   // the pairs take twice the grid's memory
 }
 template <int D>
 void launch_splat(const PointSource& s, uint32_t n, const GridArgs& g, cudaStream_t st) {
     if (!n) return;
-    // runs of pixels summed in registers where the corner sums fit (2^d x vd <= 16)
-    if (g.vd == 2 && D <= 3) {
-        const PixelTiles t = pixel_tiles(s, 4);
-        grid_splat_kernel<D, 2, 4><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g);
-    } else if (g.vd == 4 && D <= 2) {
-        const PixelTiles t = pixel_tiles(s, 4);
-        grid_splat_kernel<D, 4, 4><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g);
-    } else {
-        const PixelTiles t = pixel_tiles(s, 1);
-        if (g.vd == 2) grid_splat_kernel<D, 2, 1><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g);
-        else if (g.vd == 4) grid_splat_kernel<D, 4, 1><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g);
-        else grid_splat_kernel<D, 0, 1><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g);
+    if constexpr (D <= 3) {
+        if (g.vd == 2) {
+            const PixelTiles t = pixel_tiles(s, 4);
+            if (g.pairs) grid_splat_kernel<D, 2, 4, true><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g);
+            else grid_splat_kernel<D, 2, 4, false><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g);
+            return;
+        }
     }
+    if constexpr (D <= 2) {
+        if (g.vd == 4) {
+            const PixelTiles t = pixel_tiles(s, 4);
+            grid_splat_kernel<D, 4, 4, false><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g);
+            return;
+        }
+    }
+    const PixelTiles t = pixel_tiles(s, 1);
+    if (g.vd == 2) grid_splat_kernel<D, 2, 1, false><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g);
+    else if (g.vd == 4) grid_splat_kernel<D, 4, 1, false><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g);
+    else grid_splat_kernel<D, 0, 1, false><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g);
 }
 template <int D>
 void launch_slice(const PointSource& s, uint32_t n, const GridArgs& g, const OutView& o, cudaStream_t st) {
     if (!n) return;
     const PixelTiles t = pixel_tiles(s, 1);
-    if (g.vd == 2) grid_slice_kernel<D, 2><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g, o);
-    else if (g.vd == 4) grid_slice_kernel<D, 4><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g, o);
-    else grid_slice_kernel<D, 0><<<t.grid, kGridThreads, 0, st>>>(s, t.bw, g, o);
+    if (g.vd == 2) grid_slice_kernel<D, 2><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g, o);
+    else if (g.vd == 4) grid_slice_kernel<D, 4><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g, o);
+    else grid_slice_kernel<D, 0><<<t.grid, kGridThreads, 0, st>>>(s, t.bshift, g, o);
+}
+
+// Bounds of the pixel-coordinate dimensions of s, folded into lo and hi: x * scale * scaleFactor,
+// with the kernels' roundings, never decreases (scale > 0) or increases from pixel to pixel.
+void coordinate_bounds(const PointSource& s, float sf, float* lo, float* hi, bool first) {
+    const int last[3] = {s.width - 1, s.height - 1, s.frames - 1};
+    int c = s.pos_channels;
+    for (int k = 0; k < 3; ++k) {
+        if (!((s.coord_mask >> k) & 1)) continue;
+        for (int end = 0; end < 2; ++end) {
+            volatile float p = (float)(uint32_t)(end ? last[k] : 0) * s.coord_scale[k];
+            volatile float q = p * sf;
+            const float v = q;
+            if ((first && end == 0) || v < lo[c] || !std::isfinite(v)) lo[c] = v;
+            if ((first && end == 0) || v > hi[c] || !std::isfinite(v)) hi[c] = v;
+        }
+        ++c;
+    }
 }
 
 #define PGPU_GRID_DISPATCH(d, call)          \
@@ -397,34 +466,46 @@ int run_grid(Engine& E, const LatticeJob& J, cudaStream_t st) {
     CUDA_TRY(cudaEventRecord(E.ev[0], st));
     CUDA_TRY(cudaMemsetAsync(mm, 0xFF, sizeof(unsigned) * d, st));
     CUDA_TRY(cudaMemsetAsync(mm + d, 0, sizeof(unsigned) * d, st));
-    PGPU_GRID_DISPATCH(d, launch_minmax<DD>(J.splat, J.n, sf, mm, E.sms, st));
-    if (!J.replay) PGPU_GRID_DISPATCH(d, launch_minmax<DD>(sl, nsl, sf, mm, E.sms, st));
+    if (J.splat.pos_channels) {
+        PGPU_GRID_DISPATCH(d, launch_minmax<DD>(J.splat, sf, mm, E.sms, st));
+        if (!J.replay) PGPU_GRID_DISPATCH(d, launch_minmax<DD>(sl, sf, mm, E.sms, st));
+    }
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(E.hstat, mm, sizeof(unsigned) * 2 * d, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
+    float lows[kGridMaxD], highs[kGridMaxD];
+    for (int i = 0; i < J.splat.pos_channels; ++i) {
+        lows[i] = unordered_float(E.hstat[i]);
+        highs[i] = unordered_float(E.hstat[d + i]);
+    }
+    coordinate_bounds(J.splat, sf, lows, highs, true);
+    if (!J.replay) coordinate_bounds(sl, sf, lows, highs, false);
 
     GridArgs g;
     memset(&g, 0, sizeof(g));
     g.vd = vd;
     g.sf = sf;
-    g.stride[0] = vd;
+    g.stride[0] = (uint32_t)vd;
+    long long cells = vd;   // values in the grid
     for (int i = 0; i < d; ++i) {
-        const float lo = unordered_float(E.hstat[i]), hi = unordered_float(E.hstat[d + i]);
+        const float lo = lows[i], hi = highs[i];
         if (!std::isfinite(lo) || !std::isfinite(hi))
             return fail(PGPU_ERR_ARGUMENT, "positions are not finite");
         g.minp[i] = lo;
         const float span = hi - lo;   // float subtraction, as maxPosition[i] - minPosition[i]
         g.sizes[i] = (int)(std::ceil(span) + 1);
-        g.stride[i + 1] = g.stride[i] * g.sizes[i];
-        if (g.sizes[i] < 1 || g.stride[i + 1] > kGridMaxCells)
+        cells *= g.sizes[i];
+        if (g.sizes[i] < 1 || cells > kGridMaxCells)
             return fail(PGPU_ERR_CAPACITY, "the grid would need more than %lld cells", kGridMaxCells);
+        g.stride[i + 1] = (uint32_t)cells;
     }
-    const long long cells = g.stride[d];
-    if ((rc = E.grid.ensure((size_t)cells * sizeof(float))) ||
+    g.pairs = splat_in_pairs(d, vd, cells) ? 1 : 0;
+    const size_t splat_values = (size_t)cells << g.pairs;
+    if ((rc = E.grid.ensure(splat_values * sizeof(float))) ||
         (rc = E.grid2.ensure((size_t)cells * sizeof(float))))
         return rc;
     g.grid = (float*)E.grid.p;
-    CUDA_TRY(cudaMemsetAsync(g.grid, 0, (size_t)cells * sizeof(float), st));
+    CUDA_TRY(cudaMemsetAsync(g.grid, 0, splat_values * sizeof(float), st));
     CUDA_TRY(cudaEventRecord(E.ev[1], st));
     PGPU_GRID_DISPATCH(d, launch_splat<DD>(J.splat, J.n, g, st));
     CUDA_TRY(cudaGetLastError());
@@ -436,7 +517,9 @@ int run_grid(Engine& E, const LatticeJob& J, cudaStream_t st) {
     int cur = 0;
     const unsigned blur_blocks = (unsigned)((cells + kGridThreads - 1) / kGridThreads);
     for (int j = 0; j < d; ++j, cur ^= 1)
-        grid_blur_kernel<<<blur_blocks, kGridThreads, 0, st>>>(g, j, bufs[cur], bufs[cur ^ 1], (uint32_t)cells);
+        grid_blur_kernel<<<blur_blocks, kGridThreads, 0, st>>>(
+            bufs[cur], bufs[cur ^ 1], (uint32_t)cells, g.stride[j], magic_of(g.stride[j]), (uint32_t)g.sizes[j],
+            magic_of((uint32_t)g.sizes[j]), j == 0 ? g.pairs : 0);
     g.grid = bufs[cur];
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaEventRecord(E.ev[4], st));

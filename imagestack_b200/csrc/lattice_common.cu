@@ -137,9 +137,6 @@ static uint32_t log2_of(uint32_t pow2) {
     while ((1u << k) < pow2) ++k;
     return k;
 }
-// floor(2^32 / d) for div_magic
-static uint32_t magic_of(uint32_t d) { return d <= 1 ? 0xFFFFFFFFu : (uint32_t)(0x100000000ull / d); }
-
 void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint32_t* splat,
                       uint32_t* tile, uint32_t* slice, uint32_t splat_threads, uint32_t tile_w) {
     const PointSource& q = s.src;

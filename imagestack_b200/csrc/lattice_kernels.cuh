@@ -87,7 +87,8 @@ struct Segment {
     uint32_t tile_xm, tile_fm, stile_xm, stile_fm;
 };
 
-// b / d with m = floor(2^32 / d) (2^32 - 1 for d = 1), for b < 2^31: the multiply-high is the
+inline uint32_t magic_of(uint32_t d) { return d <= 1 ? 0xFFFFFFFFu : (uint32_t)(0x100000000ull / d); }
+// b / d with m = magic_of(d) = floor(2^32 / d) (2^32 - 1 for d = 1), for b < 2^31: the multiply-high is the
 // quotient or one less.
 __device__ __forceinline__ uint32_t div_magic(uint32_t b, uint32_t d, uint32_t m, uint32_t* rem) {
     uint32_t q = __umulhi(b, m);
