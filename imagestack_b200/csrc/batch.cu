@@ -284,6 +284,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     const int forced = splat_forced();
     std::vector<Segment> segs(nseg), slsegs(B.replay ? 0 : nseg);
     uint64_t blocks = 0, tile_blocks = 0, slice_blocks = 0;
+    const int tile_px = tile_px_for(n_total);
     int tiled_count = 0;
     for (int k = 0; k < nseg; ++k) {
         const BatchItem& it = B.items[k];
@@ -296,7 +297,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
         const bool tiled = tile_splat_for(B, wide, forced, density[k], it.n);
         uint32_t nb_splat = 0, nb_tile = 0, nb_slice = 0;
         segment_geometry(sgm, B.replay ? it.splat : it.slice, tiled, &nb_splat, &nb_tile, &nb_slice,
-                         wide ? kSplatThreads : kDirectThreads, (uint32_t)B.tile_w);
+                         wide ? kSplatThreads : kDirectThreads, (uint32_t)B.tile_w, (uint32_t)tile_px);
         tiled_count += tiled ? 1 : 0;
         sgm.splat_base = (uint32_t)blocks;
         sgm.tile_base = (uint32_t)tile_blocks;
@@ -393,6 +394,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
 
         unsigned char* dmeta = (unsigned char*)E.meta.p;
         uint32_t* dM = (uint32_t*)dmeta + 1;
+        const Segment* host_segs = nseg <= kParamSegs && !graph ? segs.data() : nullptr;
         // where the splat accumulates
         void* rows0 = !vrows ? E.tvals.p : (homog || f32_rows) ? E.vf32.p : E.vv0.p;
         auto enqueue = [&](bool timed) -> int {
@@ -444,6 +446,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sa.seg_status = (unsigned*)(dmeta + L.segstat);
             sa.blocks = (uint32_t)blocks;
             sa.tile_blocks = (uint32_t)tile_blocks;
+            sa.tile_px = tile_px;
+            sa.host_segs = host_segs;
             sa.vcount = exact_order ? nullptr : dM;
             sa.seg_counts = (uint32_t*)(dmeta + L.counts);
             sa.vkey = E.vkey.p;
@@ -613,6 +617,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sl.rec = replay_w ? E.rec.p : nullptr;
             sl.svals = E.sval.p;
             sl.vd = vd;
+            sl.host_segs = host_segs;
             sl.rec_vtx = B.rec_vtx;
             sl.rec_w = B.rec_w;
             sl.seg_status = (unsigned*)(dmeta + L.segstat);

@@ -4,8 +4,8 @@
 
 #include "lattice_ops.h"
 
-// default tile splat tiles: PGPU_TILE_W pixels wide, kTilePixels / PGPU_TILE_W high (a
-// power of two up to kTilePixels; the autotuner also tries 32x8)
+// default tile splat tiles: PGPU_TILE_W pixels wide (a power of two; the autotuner also tries
+// 32), as many high as their kTileThreads * tile_px pixels allow
 #ifndef PGPU_TILE_W
 #define PGPU_TILE_W 16u
 #endif
@@ -138,7 +138,7 @@ static uint32_t log2_of(uint32_t pow2) {
     return k;
 }
 void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint32_t* splat,
-                      uint32_t* tile, uint32_t* slice, uint32_t splat_threads, uint32_t tile_w) {
+                      uint32_t* tile, uint32_t* slice, uint32_t splat_threads, uint32_t tile_w, uint32_t tile_px) {
     const PointSource& q = s.src;
     s.src.pos_is_val = q.pos.base == q.val.base && q.pos.ystride == q.val.ystride &&
                        q.pos.tstride == q.val.tstride && q.pos.cstride == q.val.cstride &&
@@ -146,15 +146,16 @@ void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint
     const uint32_t W = (uint32_t)s.src.width, H = (uint32_t)s.src.height, F = (uint32_t)s.src.frames;
     const uint64_t n = (uint64_t)W * H * F;
     if (tiled) {
-        // tile_w x (kTilePixels / tile_w) tiles (16x16 by default); a point list (one row) in runs of kTilePixels
+        // tile_w x (pixels / tile_w) tiles; a point list (one row) in runs
+        const uint32_t pixels = (uint32_t)kTileThreads * tile_px;
         const uint32_t tw = tile_w ? tile_w : (uint32_t)PGPU_TILE_W;
-        s.tile_w = (H == 1 && F == 1) ? (uint32_t)kTilePixels : std::min<uint32_t>(tw, pow2_at_least(W));
-        s.tile_h = (uint32_t)kTilePixels / s.tile_w;
+        s.tile_w = (H == 1 && F == 1) ? pixels : std::min<uint32_t>(tw, pow2_at_least(W));
+        s.tile_h = pixels / s.tile_w;
         s.tiles_x = (W + s.tile_w - 1) / s.tile_w;
         s.tiles_y = (H + s.tile_h - 1) / s.tile_h;
         s.tile_shift = log2_of(s.tile_w);
-        // 8 x 8 pixels per warp; a narrower image's tile width, or a run of a point list
-        s.warp_shift = s.tile_h == 1 ? log2_of((uint32_t)kWarpPixels) : std::min<uint32_t>(3u, s.tile_shift);
+        // 8x4 or 8x8 pixels per warp; a narrower image's tile width, or a run of a point list
+        s.warp_shift = s.tile_h == 1 ? log2_of(32u * tile_px) : std::min<uint32_t>(3u, s.tile_shift);
         s.tile_xm = magic_of(s.tiles_x);
         s.tile_fm = magic_of(s.tiles_x * s.tiles_y);
         *tile = s.tiles_x * s.tiles_y * F;

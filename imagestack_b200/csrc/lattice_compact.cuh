@@ -421,6 +421,8 @@ struct CompactSplatArgs {
     unsigned* seg_status;  // one status word per segment
     uint32_t blocks;       // direct splat blocks of the batch
     uint32_t tile_blocks;  // tile splat blocks of the batch
+    int tile_px;           // pixels per lane of the tile splat
+    const Segment* host_segs;   // host copies, nseg <= kParamSegs: pass them as parameters; or null
     // The vertices, numbered in the order the splat creates them (null with ft, whose vertices
     // are numbered afterwards, by first touch): the creator writes a vertex's key and slot,
     // marks its lower neighbours absent (nbr_init), and leaves the number at the slot.
@@ -484,12 +486,12 @@ __device__ __forceinline__ uint32_t reserve_numbers(const CompactSplatArgs& a, i
 }
 
 // ---------------------------------------------------------------------------------
-// tile splat: one block per 2D tile of kTilePixels pixels of one frame (d <= 7)
+// tile splat: one block per 2D tile of kTileThreads * NP pixels of one frame (d <= 7)
 // ---------------------------------------------------------------------------------
 // Neighbouring pixels land on the same lattice vertices (on the 4K d=5 bilateral the 384
 // (point, remainder) entries of 8x8 pixels touch about 78 distinct vertices), while the
 // direct splat pays a probe of the global table, a trip to L2 or DRAM, per entry.  Here each
-// warp takes 64 pixels of the block's tile (8x8), two per lane: it finds each
+// warp takes 32 or 64 pixels of the block's tile, one or two per lane: it finds each
 // vertex's entries in shared memory (phases A and B), inserts each distinct vertex into the
 // global table once (phase C), and then every lane adds its rows to the global rows with
 // fire-and-forget vector reductions and writes its replay records (phase D).  A vertex's
@@ -497,7 +499,7 @@ __device__ __forceinline__ uint32_t reserve_numbers(const CompactSplatArgs& a, i
 // reference's first insertion; the vertex set, keys and records equal the direct splat's,
 // only the order of the FP32 additions differs.
 //
-// The warps of a block do not wait for one another after the segment is loaded (but with
+// The warps of a block do not wait for one another after the start (but with
 // number_rows, for the vertices' numbers): the latency of one warp's probes hides behind
 // other warps' arithmetic.  The block's vertices are numbered by its last warp, with one
 // atomic: every vertex number of a batch comes from one counter, which takes about
@@ -514,31 +516,23 @@ __device__ __forceinline__ uint32_t reserve_numbers(const CompactSplatArgs& a, i
 // swaps: 12 shared-memory wavefronts per swap, 0.37 of the splat's 0.75 ms per 4K frame.)
 constexpr int kTileThreads = 128;
 constexpr int kTileWarps = kTileThreads / 32;
-#ifndef PGPU_TILE_PX
-#define PGPU_TILE_PX 2
-#endif
-constexpr int kTilePx = PGPU_TILE_PX;                   // pixels per lane
-constexpr int kWarpPixels = 32 * kTilePx;
-static_assert(kTileThreads * kTilePx == kTilePixels, "a block's warps cover its tile");
-#ifndef PGPU_TILE_CLAIM_BITS
-#define PGPU_TILE_CLAIM_BITS 10
-#endif
-constexpr int kTileClaimBits = PGPU_TILE_CLAIM_BITS;    // claim table entries per warp, log2
-#ifndef PGPU_TILE_MIN_BLOCKS_D5
-#define PGPU_TILE_MIN_BLOCKS_D5 8
-#endif
-static_assert((1 << kTileClaimBits) >= 2 * 8 * kWarpPixels, "the claims later list a warp's vertices and its new ones");
-__host__ __device__ constexpr int tile_min_blocks(int d) { return d <= 5 ? PGPU_TILE_MIN_BLOCKS_D5 : 6; }
+// Pixels per lane.  More pixels share more vertices (NP = 2: 8x8 pixels per warp, 78 vertices for
+// 64 pixels of a 4K frame; NP = 1: 8x4, 55 for 32), a small image needs the warps (tile_px_for).
+// Four pixels (16x8 per warp, 113 vertices for 128) leave too few warps: 0.66 ms per 4K frame
+// against 0.56.
+// claim table entries per warp, log2: they later list a warp's vertices and its new ones
+__host__ __device__ constexpr int tile_claim_bits(int np) { return np == 1 ? 9 : 10; }
+__host__ __device__ constexpr int tile_min_blocks(int d, int np) { return np == 1 ? (d <= 5 ? 12 : 8) : d <= 5 ? 8 : 6; }
 
 // Dynamic shared memory of a tile splat block; per warp: 8 bytes per entry, for the simplex
 // scratch, then the key, then (where the entry stands for a vertex) the vertex's row, and
 // the claims, which later list the vertices.  (The rows are not summed in shared memory:
 // float atomics there are compare-and-swap loops, and a variant that summed each tile's rows
 // before one global reduction per vertex took 2.1 ms per 4K frame against 0.73 ms.)
-__host__ __device__ constexpr size_t tile_warp_bytes(int d) {
-    return (size_t)(d + 1) * kWarpPixels * 8 + ((size_t)2 << kTileClaimBits);
+__host__ __device__ constexpr size_t tile_warp_bytes(int d, int np) {
+    return (size_t)(d + 1) * np * 32 * 8 + ((size_t)2 << tile_claim_bits(np));
 }
-__host__ __device__ constexpr size_t tile_smem_bytes(int d) { return tile_warp_bytes(d) * kTileWarps; }
+__host__ __device__ constexpr size_t tile_smem_bytes(int d, int np) { return tile_warp_bytes(d, np) * kTileWarps; }
 
 // first number of a block's new vertices, of which its warps have s_new
 __device__ __forceinline__ uint32_t number_block(const CompactSplatArgs& a, int kseg, const uint32_t* s_new) {
@@ -560,29 +554,34 @@ __device__ __forceinline__ void publish_list(const CompactSplatArgs& a, const ui
 }
 
 // claim of a key
-__device__ __forceinline__ uint32_t tile_claim(uint64_t k) { return ck_mix(k) >> (32 - kTileClaimBits); }
+template <int NP>
+__device__ __forceinline__ uint32_t tile_claim(uint64_t k) { return ck_mix(k) >> (32 - tile_claim_bits(NP)); }
 
-// Position and values of pixel (x, y, f).  The usual layout, as many guide channels as
-// positions but x and y, is read without asking per channel (BOTH: the guide is the image);
-// every other by load_point_xyt.
+// Position and values of pixel (x, y, f).  The usual layouts are read without asking per
+// channel: as many guide channels as positions but x and y (1, or 2 where the guide is the
+// image), or but x, y and t (3, 4); 0, any other, is read by load_point_xyt.
 template <int D, int VDP>
 __device__ __forceinline__ int point_layout(const PointSource& s) {
-    if (D < 3 || s.pos_channels != D - 2 || s.coord_mask != 3 || !s.homogeneous) return 0;
-    return s.pos_is_val && s.val_channels == D - 2 && D - 2 < VDP ? 2 : s.val_channels < VDP ? 1 : 0;
+    const int coords = s.coord_mask == 3 ? 2 : s.coord_mask == 7 ? 3 : 0;
+    if (coords == 0 || D <= coords || s.pos_channels != D - coords || !s.homogeneous) return 0;
+    const bool both = s.pos_is_val && s.val_channels == s.pos_channels && s.pos_channels < VDP;
+    if (!both && s.val_channels >= VDP) return 0;
+    return 2 * (coords - 2) + (both ? 2 : 1);
 }
-template <int D, int VDP, bool BOTH>
+template <int D, int VDP, int COORDS, bool BOTH>
 __device__ __forceinline__ void load_image_point(const PointSource& s, uint32_t x, uint32_t y, uint32_t f,
                                                  float (&p)[D], float (&v)[VDP]) {
-    constexpr int NC = D >= 3 ? D - 2 : 1;
+    constexpr int NC = D > COORDS ? D - COORDS : 1;
     const float* at = s.pos.base + ((long long)f * s.pos.tstride + (long long)y * s.pos.ystride + x);
     float ch[NC];
 #pragma unroll
     for (int k = 0; k < NC; ++k, at += s.pos.cstride) ch[k] = __ldg(at);
 #pragma unroll
     for (int k = 0; k < NC; ++k) p[k] = __fmul_rn(ch[k], s.pos_scale[k]);
-    if constexpr (D >= 3) {
-        p[D - 2] = __fmul_rn((float)x, s.coord_scale[0]);
-        p[D - 1] = __fmul_rn((float)y, s.coord_scale[1]);
+    if constexpr (D > COORDS) {
+        p[NC] = __fmul_rn((float)x, s.coord_scale[0]);
+        p[NC + 1] = __fmul_rn((float)y, s.coord_scale[1]);
+        if constexpr (COORDS == 3) p[NC + 2] = __fmul_rn((float)f, s.coord_scale[2]);
     }
     if constexpr (BOTH) {
 #pragma unroll
@@ -599,13 +598,11 @@ __device__ __forceinline__ void load_image_point(const PointSource& s, uint32_t 
 // are out of range): their weights, the list (in s_claim, after use) and number of their
 // vertices, each the entry that stands for it, and loc2, each entry's vertex (two entries to a
 // register).  The entry of remainder r of pixel k of a lane is e = b*32 + lane, b = k*(D+1) + r.
-template <int D>
-__device__ __forceinline__ uint32_t tile_vertices(const float (&pp)[kTilePx][D], const LatticeConsts& lc,
+template <int D, int NP>
+__device__ __forceinline__ uint32_t tile_vertices(const float (&pp)[NP][D], const LatticeConsts& lc,
                                                   unsigned* status, uint64_t* s_key, uint16_t* s_claim,
-                                                  unsigned lane, bool (&valid)[kTilePx],
-                                                  float (&bary)[kTilePx][D + 1],
-                                                  uint32_t (&loc2)[kTilePx * (D + 1) / 2 + 1]) {
-    constexpr int NP = kTilePx;
+                                                  unsigned lane, bool (&valid)[NP], float (&bary)[NP][D + 1],
+                                                  uint32_t (&loc2)[NP * (D + 1) / 2 + 1]) {
     // Phase A: simplices, keys and claims
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
@@ -634,7 +631,7 @@ __device__ __forceinline__ uint32_t tile_vertices(const float (&pp)[kTilePx][D],
             if (r > 0) ck_step<D>(key, code[D - (r - 1)], r - 1);
             const uint32_t e = (uint32_t)(k * (D + 1) + r) * 32 + lane;
             s_key[e] = key;
-            s_claim[tile_claim(key)] = (uint16_t)e;
+            s_claim[tile_claim<NP>(key)] = (uint16_t)e;
         }
     }
     __syncwarp();
@@ -650,7 +647,7 @@ __device__ __forceinline__ uint32_t tile_vertices(const float (&pp)[kTilePx][D],
             uint32_t c = 0;
             if (valid[k]) {
                 const uint64_t key = s_key[e];
-                c = s_claim[tile_claim(key)];
+                c = s_claim[tile_claim<NP>(key)];
                 if (s_key[c] != key) c = e;   // the claim went to another key
                 if (c == e) stands |= 1u << b;
             }
@@ -668,25 +665,34 @@ __device__ __forceinline__ uint32_t tile_loc(const uint32_t* loc2, int b) {
     return (b & 1) ? loc2[b >> 1] >> 16 : loc2[b >> 1] & 0xFFFFu;
 }
 
-template <int D, int VDP>
-__global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile_kernel(CompactSplatArgs a) {
+template <int D, int VDP, int NP, bool PARAM>
+__global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D, NP))
+compact_tile_kernel(CompactSplatArgs a, const __grid_constant__ SegSource<PARAM> ps) {
     using K = CompactKey<D>;
     static_assert(K::kOneWord, "the tile splat keeps 64-bit keys in shared memory");
-    constexpr int NP = kTilePx;
     constexpr unsigned kAll = 0xFFFFFFFFu;
     extern __shared__ __align__(16) unsigned char tile_smem[];
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint64_t* s_key = reinterpret_cast<uint64_t*>(tile_smem + warp * tile_warp_bytes(D));
+    uint64_t* s_key = reinterpret_cast<uint64_t*>(tile_smem + warp * tile_warp_bytes(D, NP));
     uint16_t* s_claim = reinterpret_cast<uint16_t*>(s_key + NP * (D + 1) * 32);
     uint16_t* s_list = s_claim;                           // the vertices of the warp's pixels, after the claims,
     uint16_t* s_made = s_claim + NP * (D + 1) * 32;       // and those that this warp created
     uint32_t* s_row = reinterpret_cast<uint32_t*>(s_key);   // a vertex's row, after its key: s_row[2*e]
-    __shared__ Segment sg;
+    __shared__ Segment s_sg[1];
     __shared__ uint32_t s_new[kTileWarps];   // vertices each warp created
     __shared__ uint32_t s_done, s_first;
-    const int kseg = segment_by<&Segment::tile_base>(a.segs, a.nseg, blockIdx.x);
     if (threadIdx.x == 0) s_done = 0;
-    load_segment(a.segs + kseg, sg);   // ends with a barrier
+    int kseg;
+    if constexpr (PARAM) {
+        kseg = 0;
+#pragma unroll
+        for (int k = 1; k < kParamSegs; ++k) kseg += k < a.nseg && ps.seg[k].tile_base <= blockIdx.x ? 1 : 0;
+        __syncthreads();
+    } else {
+        kseg = segment_by<&Segment::tile_base>(a.segs, a.nseg, blockIdx.x);
+        load_segment(a.segs + kseg, s_sg[0]);   // ends with a barrier
+    }
+    const Segment& sg = segment_ref<PARAM>(ps, kseg, s_sg[0]);
 
     unsigned* status = a.seg_status + kseg;
     uint64_t* tab = reinterpret_cast<uint64_t*>(a.keys) + sg.slot_base;
@@ -696,29 +702,30 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile
     const uint32_t ty = div_magic(bt, sg.tiles_x, sg.tile_xm, &tx);
     const uint32_t wsh = sg.warp_shift, wrow = sg.tile_shift - wsh;   // log2 of the warp's width, of warps per row
     const uint32_t x0 = (tx << sg.tile_shift) + ((warp & ((1u << wrow) - 1u)) << wsh);
-    const uint32_t y0 = ty * sg.tile_h + (warp >> wrow) * ((uint32_t)kWarpPixels >> wsh);
+    const uint32_t y0 = ty * sg.tile_h + (warp >> wrow) * ((uint32_t)(32 * NP) >> wsh);
     const uint32_t W = (uint32_t)sg.src.width, H = (uint32_t)sg.src.height;
 
-    // A lane's pixels are neighbours in a row.
     float v[NP][VDP], bary[NP][D + 1];
-    uint32_t gi[NP], count, loc2[kTilePx * (D + 1) / 2 + 1];
+    uint32_t gi[NP], count, loc2[NP * (D + 1) / 2 + 1];
     bool valid[NP];   // in the image, its keys in range
     {
         const int layout = point_layout<D, VDP>(sg.src);
         float pp[NP][D];
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
-            const uint32_t p = lane * NP + k;
+            const uint32_t p = lane * NP + k;   // a lane's pixels are neighbours
             const uint32_t px = x0 + (p & ((1u << wsh) - 1u)), py = y0 + (p >> wsh);
             valid[k] = px < W && py < H;
             gi[k] = sg.point_base + (f * H + py) * W + px;
             if (valid[k]) {
-                if (layout == 2) load_image_point<D, VDP, true>(sg.src, px, py, f, pp[k], v[k]);
-                else if (layout == 1) load_image_point<D, VDP, false>(sg.src, px, py, f, pp[k], v[k]);
+                if (layout == 2) load_image_point<D, VDP, 2, true>(sg.src, px, py, f, pp[k], v[k]);
+                else if (layout == 1) load_image_point<D, VDP, 2, false>(sg.src, px, py, f, pp[k], v[k]);
+                else if (layout == 4) load_image_point<D, VDP, 3, true>(sg.src, px, py, f, pp[k], v[k]);
+                else if (layout == 3) load_image_point<D, VDP, 3, false>(sg.src, px, py, f, pp[k], v[k]);
                 else load_point_xyt<D, VDP>(sg.src, px, py, f, pp[k], v[k]);
             }
         }
-        count = tile_vertices<D>(pp, a.lc, status, s_key, s_claim, lane, valid, bary, loc2);
+        count = tile_vertices<D, NP>(pp, a.lc, status, s_key, s_claim, lane, valid, bary, loc2);
     }
 
     // Phase C: each vertex into the global table; its batch slot replaces its key.  (One that
@@ -781,24 +788,31 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile
     __syncwarp();
 
     // Phase D: every lane's rows into its vertices' rows, and the replay record.  A lane's
-    // pixels often share a vertex (the same remainder of both): one reduction for the two.
-    static_assert(NP == 2, "a lane's two pixels");
+    // pixels often share a vertex (the same remainder of both): one reduction for them.
     float* acc = reinterpret_cast<float*>(a.rows);
     uint32_t rows[NP][D + 1];
 #pragma unroll
     for (int r = 0; r <= D; ++r) {
-        const uint32_t r0 = s_row[2 * tile_loc(loc2, r)], r1 = s_row[2 * tile_loc(loc2, D + 1 + r)];
-        rows[0][r] = r0, rows[1][r] = r1;
-        const bool both = valid[0] && valid[1] && r0 == r1;
-        float c0[VDP], c1[VDP];
+        float c[NP][VDP];
+        bool sends[NP];
 #pragma unroll
-        for (int i = 0; i < VDP; ++i) {
-            c0[i] = __fmul_rn(bary[0][r], v[0][i]);
-            c1[i] = __fmul_rn(bary[1][r], v[1][i]);
-            if (both) c0[i] = __fadd_rn(c0[i], c1[i]);
+        for (int k = 0; k < NP; ++k) {
+            rows[k][r] = s_row[2 * tile_loc(loc2, k * (D + 1) + r)];
+            sends[k] = valid[k];
+#pragma unroll
+            for (int i = 0; i < VDP; ++i) c[k][i] = __fmul_rn(bary[k][r], v[k][i]);
+#pragma unroll
+            for (int j = 0; j < k; ++j) {
+                const bool join = sends[k] && sends[j] && rows[j][r] == rows[k][r];
+#pragma unroll
+                for (int i = 0; i < VDP; ++i)
+                    if (join) c[j][i] = __fadd_rn(c[j][i], c[k][i]);
+                sends[k] = sends[k] && !join;
+            }
         }
-        if (valid[0]) atomic_add_row<VDP>(acc + (size_t)r0 * VDP, c0);
-        if (valid[1] && !both) atomic_add_row<VDP>(acc + (size_t)r1 * VDP, c1);
+#pragma unroll
+        for (int k = 0; k < NP; ++k)
+            if (sends[k]) atomic_add_row<VDP>(acc + (size_t)rows[k][r] * VDP, c[k]);
     }
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
@@ -817,7 +831,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile
     at = __shfl_sync(kAll, at, 0);
 #pragma unroll 1
     for (int w = 0; w < kTileWarps; ++w) {
-        const uint64_t* w_key = reinterpret_cast<const uint64_t*>(tile_smem + w * tile_warp_bytes(D));
+        const uint64_t* w_key = reinterpret_cast<const uint64_t*>(tile_smem + w * tile_warp_bytes(D, NP));
         publish_list<D>(a, reinterpret_cast<const uint16_t*>(w_key + NP * (D + 1) * 32) + NP * (D + 1) * 32,
                         reinterpret_cast<const uint32_t*>(w_key), s_new[w], at, lane);
         at += s_new[w];
@@ -830,15 +844,10 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile
 // d >= 8.  The probes of kAhead remainders are in flight together.
 // ---------------------------------------------------------------------------------
 constexpr int kDirectThreads = 128;
-#ifndef PGPU_DIRECT_MB
-#define PGPU_DIRECT_MB 6
-#endif
-#ifndef PGPU_DIRECT_AH
-#define PGPU_DIRECT_AH 2
-#endif
-__host__ __device__ constexpr int direct_min_blocks(int d) { return d <= 7 ? 6 : PGPU_DIRECT_MB; }
+// (d=16, 2M points: two probes in flight and 6 blocks per SM 4.30 ms, four and 4 blocks 4.48)
+__host__ __device__ constexpr int direct_min_blocks(int) { return 6; }
 template <int D>
-__host__ __device__ constexpr int direct_ahead() { return D <= 7 ? (D + 1 < 4 ? D + 1 : 4) : PGPU_DIRECT_AH; }
+__host__ __device__ constexpr int direct_ahead() { return D <= 7 ? (D + 1 < 4 ? D + 1 : 4) : 2; }
 __host__ __device__ constexpr size_t direct_smem_bytes(int d) { return (size_t)(d + 1) * kDirectThreads * 12; }
 
 template <int D, int VDP>
@@ -1031,21 +1040,16 @@ __device__ __forceinline__ void gather_row(const CompactNbrArgs& a, uint32_t slo
     else store_row<VDP, float, float>(reinterpret_cast<float*>(a.rows_out), v, r);
 }
 
-#ifndef PGPU_NBR_MB
-#define PGPU_NBR_MB 4
-#endif
+// Axes whose probes are in flight together, and blocks per SM: 64-bit keys, two axes and 6 blocks
+// (4K d=5: 0.123 ms; six axes and 3 blocks 0.146); 128-bit keys with tags, six and 4 (2M
+// points at d=16: 6.9 ms; four axes 7.2).
+__host__ __device__ constexpr int nbr_ahead(int d) { return d <= 7 ? 2 : 6; }
+__host__ __device__ constexpr int nbr_min_blocks(int d) { return d <= 7 ? 6 : 4; }
 template <int D>
-__global__ void __launch_bounds__(256, D <= 7 ? 3 : PGPU_NBR_MB) compact_neighbours_kernel(CompactNbrArgs a) {
+__global__ void __launch_bounds__(256, nbr_min_blocks(D)) compact_neighbours_kernel(CompactNbrArgs a) {
     using K = CompactKey<D>;
     using T = typename K::T;
-    // axes whose probes are in flight together
-#ifndef PGPU_NBR_AH
-#define PGPU_NBR_AH 6
-#endif
-#ifndef PGPU_NBR_MB
-#define PGPU_NBR_MB 4
-#endif
-    constexpr int AH = D <= 7 ? (D + 1) : PGPU_NBR_AH;
+    constexpr int AH = nbr_ahead(D);
     const uint32_t m = *a.nverts;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
         const T key = reinterpret_cast<const T*>(a.vkey)[v];
@@ -1131,14 +1135,15 @@ __device__ __forceinline__ void write_slice(const OutView& ov, int vd, uint32_t 
 
 // d <= 7: as the tile splat, a warp finds the vertices of 64 pixels first and looks each up once
 //
+constexpr int kTileSlicePx = 2;
 template <int D, int VDP>
-__global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile_slice_kernel(CompactSliceArgs a) {
+__global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D, 2)) compact_tile_slice_kernel(CompactSliceArgs a) {
     using K = CompactKey<D>;
-    constexpr int NP = kTilePx;
-    static_assert(kTilePixels == kSliceThreads, "a slice block's pixels");
+    constexpr int NP = kTileSlicePx;
+    static_assert(kTileThreads * NP == kSliceThreads, "a slice block's pixels");
     extern __shared__ __align__(16) unsigned char slice_smem[];
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint64_t* s_key = reinterpret_cast<uint64_t*>(slice_smem + warp * tile_warp_bytes(D));
+    uint64_t* s_key = reinterpret_cast<uint64_t*>(slice_smem + warp * tile_warp_bytes(D, NP));
     uint16_t* s_list = reinterpret_cast<uint16_t*>(s_key + NP * (D + 1) * 32);
     int* s_row = reinterpret_cast<int*>(s_key);
     __shared__ Segment sg;
@@ -1147,13 +1152,13 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile
     uint32_t bt, tx;
     const uint32_t fr = div_magic(blockIdx.x - sg.block_base, sg.stiles_x * sg.stiles_y, sg.stile_fm, &bt);
     const uint32_t ty = div_magic(bt, sg.stiles_x, sg.stile_xm, &tx);
-    const uint32_t wsh = sg.slice_th == 1 ? (kWarpPixels == 64 ? 6u : 5u) : min(3u, sg.slice_shift);
+    const uint32_t wsh = sg.slice_th == 1 ? 6u : min(3u, sg.slice_shift);   // 64 pixels: 8x8, or a run
     const uint32_t wrow = sg.slice_shift - wsh;
     const uint32_t x0 = (tx << sg.slice_shift) + ((warp & ((1u << wrow) - 1u)) << wsh);
-    const uint32_t y0 = ty * sg.slice_th + (warp >> wrow) * ((uint32_t)kWarpPixels >> wsh);
+    const uint32_t y0 = ty * sg.slice_th + (warp >> wrow) * ((uint32_t)(32 * NP) >> wsh);
     unsigned* status = a.seg_status + kseg;
     float bary[NP][D + 1];
-    uint32_t count, loc2[kTilePx * (D + 1) / 2 + 1];
+    uint32_t count, loc2[NP * (D + 1) / 2 + 1];
     bool valid[NP];
     {
         float pp[NP][D];
@@ -1164,7 +1169,7 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D)) compact_tile
             valid[k] = px < (uint32_t)sg.src.width && py < (uint32_t)sg.src.height;
             if (valid[k]) load_position_xyt<D>(sg.src, px, py, fr, pp[k]);
         }
-        count = tile_vertices<D>(pp, a.lc, status, s_key, s_list, lane, valid, bary, loc2);
+        count = tile_vertices<D, NP>(pp, a.lc, status, s_key, s_list, lane, valid, bary, loc2);
     }
     // a lattice whose splat failed is rerun by the host; its output may be its input, so
     // write nothing

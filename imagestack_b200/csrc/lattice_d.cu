@@ -20,6 +20,12 @@ int grid_cap(uint64_t work, int threads, int sms) {
     return (int)g;
 }
 
+SegSource<true> param_segs(const Segment* segs, int nseg) {
+    SegSource<true> p;
+    for (int k = 0; k < nseg; ++k) p.seg[k] = segs[k];
+    return p;
+}
+
 template <int VDP, typename Acc>
 void splat_t(const SplatArgs& a, cudaStream_t st) {
     if (a.blocks) splat_kernel<D, VDP, Acc><<<a.blocks, kSplatThreads, 0, st>>>(a);
@@ -42,8 +48,10 @@ void neighbours(const NbrArgs& a, uint32_t vmax, int sms, cudaStream_t st) {
 template <int VDP, typename A>
 void slice_t(const SliceArgs& a, cudaStream_t st) {
     if (!a.blocks) return;
-    if (a.rec)
-        slice_replay_kernel<D, VDP, A><<<a.blocks, kSliceThreads, 0, st>>>(a);
+    if (a.rec && a.host_segs)
+        slice_replay_kernel<D, VDP, A, true><<<a.blocks, kSliceThreads, 0, st>>>(a, param_segs(a.host_segs, a.nseg));
+    else if (a.rec)
+        slice_replay_kernel<D, VDP, A, false><<<a.blocks, kSliceThreads, 0, st>>>(a, SegSource<false>{});
     else
         slice_kernel<D, VDP, A><<<a.blocks, kSliceThreads, 0, st>>>(a);
 }
@@ -70,12 +78,27 @@ bool slice(const SliceArgs& a, int vdp, int payload, bool homog, cudaStream_t st
     return false;
 }
 
+template <int VDP, int NP>
+void compact_tile_t(const CompactSplatArgs& a, cudaStream_t st) {
+    if constexpr (CompactKey<D>::kOneWord) {
+        const size_t smem = tile_smem_bytes(D, NP);
+        if (a.host_segs)
+            compact_tile_kernel<D, VDP, NP, true><<<a.tile_blocks, kTileThreads, smem, st>>>(
+                a, param_segs(a.host_segs, a.nseg));
+        else
+            compact_tile_kernel<D, VDP, NP, false><<<a.tile_blocks, kTileThreads, smem, st>>>(a, SegSource<false>{});
+    }
+}
+
 template <int VDP>
 bool compact_splat_t(const CompactSplatArgs& a, cudaStream_t st) {
     if (a.blocks) compact_direct_kernel<D, VDP><<<a.blocks, kDirectThreads, direct_smem_bytes(D), st>>>(a);
     if constexpr (CompactKey<D>::kOneWord) {
-        if (a.tile_blocks)
-            compact_tile_kernel<D, VDP><<<a.tile_blocks, kTileThreads, tile_smem_bytes(D), st>>>(a);
+        if (a.tile_blocks) {
+            if (a.tile_px == 1) compact_tile_t<VDP, 1>(a, st);
+            else if (a.tile_px == 2) compact_tile_t<VDP, 2>(a, st);
+            else return false;
+        }
         return true;
     }
     return a.tile_blocks == 0;
@@ -102,7 +125,7 @@ template <int VDP>
 void compact_slice_t(const CompactSliceArgs& a, cudaStream_t st) {
     if (!a.blocks) return;
     if constexpr (CompactKey<D>::kOneWord)
-        compact_tile_slice_kernel<D, VDP><<<a.blocks, kTileThreads, tile_smem_bytes(D), st>>>(a);
+        compact_tile_slice_kernel<D, VDP><<<a.blocks, kTileThreads, tile_smem_bytes(D, kTileSlicePx), st>>>(a);
     else
         compact_slice_kernel<D, VDP><<<a.blocks, kSliceThreads, (size_t)(D + 1) * kSliceThreads * sizeof(uint2), st>>>(a);
 }

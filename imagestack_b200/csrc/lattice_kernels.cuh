@@ -135,6 +135,23 @@ __device__ __forceinline__ void load_segment(const Segment* g, Segment& s) {
     __syncthreads();
 }
 
+// Up to kParamSegs segments travel in the launch's parameters: their fields are then operands from
+// the constant bank, with no copy to shared memory, no barrier and no load before the first
+// pixel.  (A captured launch would keep its parameters, so graphs read the segment table.)
+constexpr int kParamSegs = 4;
+template <bool PARAM>
+struct SegSource {
+    Segment seg[kParamSegs];
+};
+template <>
+struct SegSource<false> {};
+
+template <bool PARAM>
+__device__ __forceinline__ const Segment& segment_ref(const SegSource<PARAM>& ps, int k, const Segment& shared) {
+    if constexpr (PARAM) return ps.seg[k];
+    else return shared;
+}
+
 struct SplatArgs {
     const Segment* segs;
     int nseg;
@@ -267,6 +284,7 @@ struct SliceArgs {
     float* rec_w;               // optional weights
     unsigned* seg_status;
     uint32_t blocks;
+    const Segment* host_segs = nullptr;   // host copies, nseg <= kParamSegs: pass them as parameters
 };
 
 // ---------------------------------------------------------------------------------
@@ -395,7 +413,8 @@ __device__ __forceinline__ double acc_add(double a, double b) { return __dadd_rn
 // Remainders 2j and 2j+1 of point i are the four words (row, weight, row, weight) at
 // [j][i]; the last of an odd number of remainders is two words behind them.  A warp's
 // accesses are then runs of 16 bytes per lane: 3 stores and 3 loads per point at d = 5
-// instead of 12 each of four bytes.
+// instead of 12 each of four bytes.  Written once and read once, it passes L2 first, ahead of
+// the table and the rows.
 // ---------------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ void store_record(void* rec, uint32_t n_total, uint32_t i, const uint32_t (&row)[D + 1],
@@ -403,10 +422,10 @@ __device__ __forceinline__ void store_record(void* rec, uint32_t n_total, uint32
     uint4* pairs = reinterpret_cast<uint4*>(rec);
 #pragma unroll
     for (int j = 0; j < (D + 1) / 2; ++j)
-        pairs[(size_t)j * n_total + i] = make_uint4(row[2 * j], __float_as_uint(w[2 * j]), row[2 * j + 1],
-                                                    __float_as_uint(w[2 * j + 1]));
+        __stcs(pairs + (size_t)j * n_total + i, make_uint4(row[2 * j], __float_as_uint(w[2 * j]), row[2 * j + 1],
+                                                           __float_as_uint(w[2 * j + 1])));
     if constexpr (D % 2 == 0)
-        reinterpret_cast<uint2*>(pairs + (size_t)(D / 2) * n_total)[i] = make_uint2(row[D], __float_as_uint(w[D]));
+        __stcs(reinterpret_cast<uint2*>(pairs + (size_t)(D / 2) * n_total) + i, make_uint2(row[D], __float_as_uint(w[D])));
 }
 template <int D>
 __device__ __forceinline__ void load_record(const void* rec, uint32_t n_total, uint32_t i, int (&row)[D + 1],
@@ -428,10 +447,6 @@ __device__ __forceinline__ void load_record(const void* rec, uint32_t n_total, u
 // splat
 // ---------------------------------------------------------------------------------
 constexpr int kSplatThreads = 256;
-#ifndef PGPU_TILE_PX
-#define PGPU_TILE_PX 2
-#endif
-constexpr int kTilePixels = 128 * PGPU_TILE_PX;        // pixels of a tile splat block (lattice_compact.cuh)
 // Tuning (measured on the 4K d=5 and d=3 bilaterals and the 2M-point d=16 transform): the
 // splat is latency bound, so resident warps matter more than a few spilled registers —
 // 6 blocks of 256 per SM up to d=5 (40 registers; 0.94 -> 0.77 ms at 4K d=5), 4 for d=6,
@@ -1090,11 +1105,20 @@ __global__ void __launch_bounds__(kSliceThreads, slice_min_blocks(D)) slice_kern
 // Replay slice from the splat's records of slots and weights (src/Permutohedral.h:418-427:
 // the reference replays its recorded offsets and weights the same way): a gather of d+1 rows
 // per point with no simplex to recompute.  A block is a slice_tw x slice_th tile of one frame.
-template <int D, int VDP, typename A>
-__global__ void __launch_bounds__(kSliceThreads) slice_replay_kernel(SliceArgs a) {
-    __shared__ Segment sg;
-    const int kseg = segment_of_block(a.segs, a.nseg, blockIdx.x);
-    load_segment(a.segs + kseg, sg);
+template <int D, int VDP, typename A, bool PARAM>
+__global__ void __launch_bounds__(kSliceThreads) slice_replay_kernel(SliceArgs a,
+                                                                     const __grid_constant__ SegSource<PARAM> ps) {
+    __shared__ Segment s_sg[1];
+    int kseg;
+    if constexpr (PARAM) {
+        kseg = 0;
+#pragma unroll
+        for (int k = 1; k < kParamSegs; ++k) kseg += k < a.nseg && ps.seg[k].block_base <= blockIdx.x ? 1 : 0;
+    } else {
+        kseg = segment_of_block(a.segs, a.nseg, blockIdx.x);
+        load_segment(a.segs + kseg, s_sg[0]);
+    }
+    const Segment& sg = segment_ref<PARAM>(ps, kseg, s_sg[0]);
     uint32_t bt, tx;
     const uint32_t fr = div_magic(blockIdx.x - sg.block_base, sg.stiles_x * sg.stiles_y, sg.stile_fm, &bt);
     const uint32_t ty = div_magic(bt, sg.stiles_x, sg.stile_xm, &tx);

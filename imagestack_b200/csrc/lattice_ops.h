@@ -44,7 +44,13 @@ const DimOps* dim_ops(int d);
 // sliced, are set): the direct-splat blocks (of splat_threads points) or, when `tiled`, the tile-splat tiles, and
 // the slice tiles.  Returns the blocks of each launch through *splat, *tile and *slice.
 void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint32_t* splat,
-                      uint32_t* tile, uint32_t* slice, uint32_t splat_threads, uint32_t tile_w = 0);
+                      uint32_t* tile, uint32_t* slice, uint32_t splat_threads, uint32_t tile_w = 0, uint32_t tile_px = 2);
+
+// pixels per lane of the tile splat for `pixels` pixels in all: one where two would leave the
+// GPU's SMs less than a block of 128 threads each or little more (64x64: splat 26.6 us with
+// two, 20.5 with one; 512x512: 37.7 and 39.8)
+inline int tile_px_for(uint64_t pixels) { return pixels <= (1u << 17) ? 1 : 2; }
+
 
 void launch_mark(const uint32_t* ft, uint32_t cap, uint32_t* bitmap, int sms, cudaStream_t st);
 // per-segment vertex counts from the first-touch bitmap and its prefix popcount
