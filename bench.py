@@ -44,12 +44,8 @@ def workload(payload):
 
 
 L2_BYTES = 126 * 1024 * 1024
-# launches of one lattice besides the blur's: tile splat, neighbours, replay slice, and the
-# list-ordered compaction where rows stay in slot space
-
-
-def kernels_per_lattice(vertex_rows):
-    return 3 if vertex_rows else 4
+# launches of one lattice besides the blur's: clear, tile splat, neighbours, replay slice
+KERNELS_PER_LATTICE = 4
 TUNE_MAX_CALLS = 24       # at most this many calls for the autotuner to finish a shape
 
 
@@ -830,7 +826,7 @@ def run_ours(args):
                     "copies_alone": copies,
                     "one_call_per_step_mpix_s": round(e2e_sync, 2),
                     "autotuner_calls": e2e_tune},
-            "gpu_launches": args.steps * (kernels_per_lattice(stage[-1]["vertex_rows"]) + passes),
+            "gpu_launches": args.steps * (KERNELS_PER_LATTICE + passes),
             "autotuned": {"load_factor": round(stage[-1]["load_factor"], 3),
                           "blur_pairs": bool(stage[-1]["blur_pairs"]),
                           "blur_grid": "one vertex per thread" if stage[-1]["blur_grid"]

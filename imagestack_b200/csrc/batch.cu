@@ -400,17 +400,29 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
         auto enqueue = [&](bool timed) -> int {
             // the lattice's time (and so the autotuner's) includes clearing its tables
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[6], st));
-            CUDA_TRY(cudaMemcpyAsync(dmeta + L.slotbase, h + L.slotbase, L.total - L.slotbase,
-                                     cudaMemcpyHostToDevice, st));
-            CUDA_TRY(cudaMemsetAsync(dmeta, 0, L.slotbase, st));
-            CUDA_TRY(cudaMemsetAsync(E.key0.p, 0xFF, cap_total * (wide ? 16 : kb), st));
-            CUDA_TRY(cudaMemsetAsync(rows0, 0, cap_total * vdp * accb, st));
-            if (vrows) CUDA_TRY(cudaMemsetAsync(E.slot2vtx.p, 0xFF, cap_total * 4, st));
+            ClearArgs cl;
+            cl.count = 0;
+            cl.meta_n = 0;
+            cl.meta = (uint4*)(dmeta + L.slotbase);
+            // capacities are multiples of 32, so every region is whole 16-byte words
+            cl.add(dmeta, L.slotbase, 0u);
+            cl.add(E.key0.p, cap_total * (wide ? 16 : kb), 0xFFFFFFFFu);
+            cl.add(rows0, cap_total * vdp * accb, 0u);
+            if (vrows) cl.add(E.slot2vtx.p, cap_total * 4, 0xFFFFFFFFu);
+            if (use_tags) cl.add(E.tags.p, cap_total, 0u);
+            const size_t mb = L.total - L.slotbase;
+            // a captured pass reads its metadata when it is replayed, from the pinned buffer
+            if (!graph && mb <= sizeof(cl.words)) {
+                memcpy(cl.words, h + L.slotbase, mb);
+                cl.meta_n = (uint32_t)(mb / 16);
+            } else {
+                CUDA_TRY(cudaMemcpyAsync(dmeta + L.slotbase, h + L.slotbase, mb, cudaMemcpyHostToDevice, st));
+            }
+            launch_clear(cl, E.sms, st);
             if (exact_order) {
                 CUDA_TRY(cudaMemsetAsync(E.ft.p, 0xFF, cap_total * 4, st));
                 CUDA_TRY(cudaMemsetAsync(E.bitmap.p, 0, (size_t)nwords * 4, st));
             }
-            if (use_tags) CUDA_TRY(cudaMemsetAsync(E.tags.p, 0, cap_total, st));
             if (timed) CUDA_TRY(cudaEventRecord(E.ev[0], st));
 
             if (wide) {

@@ -12,6 +12,29 @@
 
 namespace pgpu {
 
+// Clears a pass's tables and writes its metadata: one launch in place of a copy and three to
+// five memsets, each of which small passes waited out.
+__global__ void __launch_bounds__(256) clear_kernel(const __grid_constant__ ClearArgs a) {
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    if (first < a.meta_n) a.meta[first] = a.words[first];
+#pragma unroll
+    for (int r = 0; r < ClearArgs::kRegions; ++r) {
+        if (r >= a.count) break;
+        uint4* const p = a.p[r];
+        const uint64_t n = a.n[r];
+        const uint4 v = make_uint4(a.value[r], a.value[r], a.value[r], a.value[r]);
+        for (uint64_t i = first; i < n; i += step) p[i] = v;
+    }
+}
+
+void launch_clear(const ClearArgs& a, int sms, cudaStream_t st) {
+    uint64_t most = a.meta_n;
+    for (int r = 0; r < a.count; ++r) most = std::max(most, a.n[r]);
+    const uint64_t blocks = std::min<uint64_t>((most + 255) / 256, (uint64_t)sms * 8);
+    if (blocks) clear_kernel<<<(unsigned)blocks, 256, 0, st>>>(a);
+}
+
 __global__ void mark_kernel(const uint32_t* __restrict__ ft, uint32_t cap, uint32_t* bitmap) {
     for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < cap; s += gridDim.x * blockDim.x) {
         const uint32_t f = ft[s];

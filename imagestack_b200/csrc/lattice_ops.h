@@ -52,6 +52,27 @@ void segment_geometry(Segment& s, const PointSource& slice_src, bool tiled, uint
 inline int tile_px_for(uint64_t pixels) { return pixels <= (1u << 17) ? 1 : 2; }
 
 
+// What a pass clears before its splat, and the batch's description where it is small enough
+// to travel with the launch.
+struct ClearArgs {
+    static constexpr int kRegions = 5;
+    static constexpr size_t kMetaBytes = 1024;
+    uint4* p[kRegions];
+    uint64_t n[kRegions];          // 16-byte words
+    uint32_t value[kRegions];      // of every 32-bit word
+    uint4* meta;
+    uint32_t meta_n;               // 16-byte words of words[]
+    int count;
+    uint4 words[kMetaBytes / 16];
+    void add(void* q, uint64_t bytes, uint32_t v) {
+        if (!bytes) return;
+        p[count] = (uint4*)q;
+        n[count] = bytes / 16;
+        value[count++] = v;
+    }
+};
+void launch_clear(const ClearArgs& a, int sms, cudaStream_t st);
+
 void launch_mark(const uint32_t* ft, uint32_t cap, uint32_t* bitmap, int sms, cudaStream_t st);
 // per-segment vertex counts from the first-touch bitmap and its prefix popcount
 void launch_segment_counts(const uint32_t* bitmap, const uint32_t* offs, uint32_t nwords,
