@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "engine.h"
+#include "host_copy.h"
 
 namespace pgpu {
 
@@ -51,6 +52,8 @@ void Engine::drop_graphs() {
 void Engine::shutdown() {
     if (device >= 0) cudaSetDevice(device);
     drain_async(*this);
+    delete copier;
+    copier = nullptr;
     for (auto& pb : pinned_free) cudaFreeHost(pb.first);
     pinned_free.clear();
     if (stream) cudaStreamSynchronize(stream);

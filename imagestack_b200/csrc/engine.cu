@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "engine.h"
+#include "host_copy.h"
 
 namespace pgpu {
 
@@ -299,17 +300,48 @@ int copy_view(const pgpu_image& src, const pgpu_image& dst, int channels, cudaMe
     return PGPU_OK;
 }
 
-int upload(Engine& E, DevBuf& buf, const pgpu_image& host, pgpu_image* dev, cudaStream_t st) {
+int copy_views(Engine& E, const std::vector<ViewCopy>& views, cudaMemcpyKind kind, cudaStream_t st) {
+    std::vector<HostPiece> pieces;
+    size_t bytes = 0;
+    std::vector<const ViewCopy*> direct;
+    for (const ViewCopy& v : views) {
+        const pgpu_image& s = v.src;
+        const void* host = kind == cudaMemcpyHostToDevice ? s.base : v.dst.base;
+        const size_t plane = sizeof(float) * (size_t)s.width * s.height;
+        if (s.ystride != s.width || v.dst.ystride != v.dst.width || !HostCopier::pageable(host)) {
+            direct.push_back(&v);
+        } else if (is_dense(s) && is_dense(v.dst)) {
+            pieces.push_back({(char*)v.dst.base, (const char*)s.base, plane * s.frames * v.channels});
+            bytes += pieces.back().bytes;
+        } else {
+            for (int c = 0; c < v.channels; ++c)
+                for (int t = 0; t < s.frames; ++t)
+                    pieces.push_back({(char*)(v.dst.base + c * v.dst.cstride + t * v.dst.tstride),
+                                      (const char*)(s.base + c * s.cstride + t * s.tstride), plane});
+            bytes += plane * s.frames * v.channels;
+        }
+    }
+    // below this the driver queues a copy without its staging buffer; from 80 KB on the
+    // helpers were faster at every size (48x48 Gauss transform 0.198 -> 0.174 ms)
+    constexpr size_t kStagedBytes = 64 << 10;
+    if (bytes < kStagedBytes || !HostCopier::available()) {
+        for (const HostPiece& p : pieces) CUDA_TRY(cudaMemcpyAsync(p.dst, p.src, p.bytes, kind, st));
+    } else {
+        if (!E.copier) E.copier = new HostCopier(E.device);
+        CUDA_TRY(E.copier->copy(pieces, kind, st));
+    }
+    for (const ViewCopy* v : direct)
+        if (int rc = copy_view(v->src, v->dst, v->channels, kind, st)) return rc;
+    return PGPU_OK;
+}
+
+// device memory for an image of host memory, dense
+int stage(DevBuf& buf, const pgpu_image& host, pgpu_image* dev) {
     const size_t n = (size_t)host.width * host.height * host.frames * host.channels;
     int rc = buf.ensure(n * sizeof(float));
     if (rc) return rc;
-    (void)E;
     *dev = dense_like(host, (float*)buf.p, host.channels);
-    return copy_view(host, *dev, host.channels, cudaMemcpyHostToDevice, st);
-}
-
-int download(const pgpu_image& dev, const pgpu_image& host, int channels, cudaStream_t st) {
-    return copy_view(dev, host, channels, cudaMemcpyDeviceToHost, st);
+    return PGPU_OK;
 }
 
 PlanarView planar(const pgpu_image& v) { return PlanarView{v.base, v.ystride, v.tstride, v.cstride}; }
@@ -880,9 +912,12 @@ int pgpu_gauss_transform(const pgpu_image* slice, const pgpu_image* splat, const
     const bool replay = !slice || same_view(*slice, *splat);
     pgpu_image dsplat, dvals, dslice, dout;
     int rc;
-    if ((rc = upload(E, E.img_a, *splat, &dsplat, S.st))) return rc;
-    if ((rc = upload(E, E.img_b, *values, &dvals, S.st))) return rc;
-    if (!replay && (rc = upload(E, E.img_c, *slice, &dslice, S.st))) return rc;
+    if ((rc = stage(E.img_a, *splat, &dsplat)) || (rc = stage(E.img_b, *values, &dvals)) ||
+        (!replay && (rc = stage(E.img_c, *slice, &dslice))))
+        return rc;
+    std::vector<ViewCopy> in = {{*splat, dsplat, splat->channels}, {*values, dvals, values->channels}};
+    if (!replay) in.push_back({*slice, dslice, slice->channels});
+    if ((rc = copy_views(E, in, cudaMemcpyHostToDevice, S.st))) return rc;
     const pgpu_image& sl = replay ? *splat : *slice;
     if ((rc = E.img_d.ensure(sizeof(float) * (size_t)sl.width * sl.height * sl.frames * values->channels)))
         return rc;
@@ -890,7 +925,7 @@ int pgpu_gauss_transform(const pgpu_image* slice, const pgpu_image* splat, const
     rc = gauss_transform_device(E, replay ? nullptr : &dslice, dsplat, dvals, sigmas, n_sigmas, dout,
                                 opt.payload, opt.load_factor, S.st, opt.method);
     if (rc) return rc;
-    if ((rc = download(dout, *out, values->channels, S.st))) return rc;
+    if ((rc = copy_views(E, {{dout, *out, values->channels}}, cudaMemcpyDeviceToHost, S.st))) return rc;
     CUDA_TRY(cudaStreamSynchronize(S.st));
     return PGPU_OK;
 }
@@ -910,13 +945,15 @@ int pgpu_joint_bilateral(pgpu_image* im, const pgpu_image* ref, float filter_wid
     const bool same = same_view(*im, *ref);
     pgpu_image dim, dref;
     int rc;
-    if ((rc = upload(E, E.img_a, *im, &dim, S.st))) return rc;
+    if ((rc = stage(E.img_a, *im, &dim)) || (!same && (rc = stage(E.img_b, *ref, &dref)))) return rc;
+    std::vector<ViewCopy> in = {{*im, dim, im->channels}};
     if (same) dref = dim;
-    else if ((rc = upload(E, E.img_b, *ref, &dref, S.st))) return rc;
+    else in.push_back({*ref, dref, ref->channels});
+    if ((rc = copy_views(E, in, cudaMemcpyHostToDevice, S.st))) return rc;
     rc = joint_bilateral_device(E, dim, dref, filter_width, filter_height, filter_frames, color_sigma,
                                 opt.payload, opt.load_factor, S.st, opt.method);
     if (rc) return rc;
-    if ((rc = download(dim, *im, im->channels, S.st))) return rc;
+    if ((rc = copy_views(E, {{dim, *im, im->channels}}, cudaMemcpyDeviceToHost, S.st))) return rc;
     CUDA_TRY(cudaStreamSynchronize(S.st));
     return PGPU_OK;
 }

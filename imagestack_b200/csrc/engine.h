@@ -47,6 +47,7 @@ struct DevBuf {
     ~DevBuf();
 };
 
+class HostCopier;    // host_copy.h
 struct AsyncBatch;   // a host-memory batch queued by pgpu_bilateral_batch_submit (engine.cu)
 
 struct Engine {
@@ -77,6 +78,7 @@ struct Engine {
     unsigned* hstat = nullptr;
     cudaEvent_t ev[8] = {};
     cudaEvent_t join_ev[2] = {};   // ordering against the legacy default stream
+    HostCopier* copier = nullptr;   // its threads and pinned buffers, from the first large copy on
     // host-memory batches: uploads and downloads overlap the lattices on these streams
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaEvent_t pipe_ev[9] = {};   // per device slot (3): uploaded, filtered, downloaded
@@ -129,6 +131,13 @@ bool is_dense(const pgpu_image& v);
 pgpu_image dense_like(const pgpu_image& v, float* base, int channels);
 int copy_view(const pgpu_image& src, const pgpu_image& dst, int channels, cudaMemcpyKind kind,
               cudaStream_t st);
+// One image to copy, and copies of several images between host and device memory that do
+// not wait for one another (engine.cu); E is the calling thread's for the call.
+struct ViewCopy {
+    pgpu_image src, dst;
+    int channels;
+};
+int copy_views(Engine& E, const std::vector<ViewCopy>& views, cudaMemcpyKind kind, cudaStream_t st);
 PlanarView planar(const pgpu_image& v);
 OutView outview(const pgpu_image& v, int channels, int normalize);
 

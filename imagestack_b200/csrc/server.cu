@@ -156,14 +156,17 @@ public:
         clear_error();
         const cudaStream_t st = E.stream;
         size_t floats = 0;
+        size_t out_floats = 0;
         for (Req* q : batch) {
             const pgpu_request& r = q->r;
-            floats += (size_t)q->n * (r.in.channels + q->out_channels +
-                                      (r.kind == PGPU_REQ_BILATERAL ? 0 : r.ref.channels));
+            floats += (size_t)q->n * (r.in.channels + (r.kind == PGPU_REQ_BILATERAL ? 0 : r.ref.channels));
+            out_floats += (size_t)q->n * q->out_channels;
         }
         int rc;
-        if ((rc = E.img_a.ensure(floats * sizeof(float)))) return rc;
+        if ((rc = E.img_a.ensure((floats + out_floats) * sizeof(float)))) return rc;
+        // inputs first, then outputs: those of several small requests travel as one copy
         float* p = (float*)E.img_a.p;
+        float* pout = p + floats;
         BatchJob B;
         B.d = batch[0]->d;
         B.vd = batch[0]->vd;
@@ -173,21 +176,23 @@ public:
         B.replay = true;
         B.items.resize(batch.size());
         std::vector<pgpu_image> dout(batch.size());
+        std::vector<ViewCopy> in, back;
         volatile float one = 1.0f;
         for (size_t k = 0; k < batch.size(); ++k) {
             const Req* q = batch[k];
             const pgpu_request& r = q->r;
             pgpu_image din = dense_like(r.in, p, r.in.channels);
             p += (size_t)q->n * r.in.channels;
-            if ((rc = copy_view(r.in, din, r.in.channels, cudaMemcpyHostToDevice, st))) return rc;
+            in.push_back({r.in, din, r.in.channels});
             pgpu_image dpos = din;
             if (r.kind != PGPU_REQ_BILATERAL) {
                 dpos = dense_like(r.ref, p, r.ref.channels);
                 p += (size_t)q->n * r.ref.channels;
-                if ((rc = copy_view(r.ref, dpos, r.ref.channels, cudaMemcpyHostToDevice, st))) return rc;
+                in.push_back({r.ref, dpos, r.ref.channels});
             }
-            dout[k] = dense_like(r.out, p, q->out_channels);
-            p += (size_t)q->n * q->out_channels;
+            dout[k] = dense_like(r.out, pout, q->out_channels);
+            pout += (size_t)q->n * q->out_channels;
+            back.push_back({dout[k], r.out, q->out_channels});
             BatchItem& it = B.items[k];
             PointSource& s = it.splat;
             memset(&s, 0, sizeof(s));
@@ -215,10 +220,9 @@ public:
         }
         // The lattices follow the uploads on this worker's stream; the other workers'
         // copies and lattices run on theirs at the same time.
-        if ((rc = run_batch(E, B, st))) return rc;
-        for (size_t k = 0; k < batch.size(); ++k)
-            if ((rc = copy_view(dout[k], batch[k]->r.out, batch[k]->out_channels, cudaMemcpyDeviceToHost, st)))
-                return rc;
+        if ((rc = copy_views(E, in, cudaMemcpyHostToDevice, st)) || (rc = run_batch(E, B, st)) ||
+            (rc = copy_views(E, back, cudaMemcpyDeviceToHost, st)))
+            return rc;
         CUDA_TRY(cudaStreamSynchronize(st));
         return PGPU_OK;
     }

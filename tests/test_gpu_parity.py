@@ -453,3 +453,27 @@ def test_batch_with_images_out_of_the_compact_keys_range(gpu, payload, tol):
         gpu.bilateral_batch(out, fw, cs, payload=payload)
         for a, b in zip(out, expect):
             assert rel_err(a, b, floor_frac=1e-2) <= tol
+
+
+@pytest.mark.parametrize("rows", [slice(None), slice(3, -2)])      # dense, a range of rows
+@pytest.mark.parametrize("w,h", [(64, 81), (64, 90), (411, 218), (1023, 1130)])
+def test_host_copies_in_chunks_match_device_memory(gpu, w, h, rows):
+    """Images in pageable memory, below and above the size from which several threads copy
+    them, in one chunk, in chunks of the smallest and of the largest size with remainders;
+    pinned memory; and the rows around a range of rows stay as they were."""
+    import torch
+    big = synth.image(w, h, 3, rects=8, seed=w + h)
+    expect = torch.from_numpy(big[:, rows].copy()).cuda()
+    gpu.Bilateral.apply(expect, 9.0, 9.0, 0.0, 0.15)
+    expect = expect.cpu().numpy()
+    pinned = torch.from_numpy(big.copy()).pin_memory().numpy()
+    for work in (big.copy(), pinned):
+        gpu.Bilateral.apply(work[:, rows], 9.0, 9.0, 0.0, 0.15)
+        assert rel_err(work[:, rows], expect) <= RTOL_FP32
+        outside = np.ones(h, bool)
+        outside[rows] = False
+        np.testing.assert_array_equal(work[:, outside], big[:, outside])
+    out = gpu.GaussTransform.apply(None, big[:, rows], big[:2, rows], [0.2, 0.2, 0.2])
+    dev = torch.from_numpy(big[:, rows].copy()).cuda()
+    ref = gpu.GaussTransform.apply(None, dev, dev[:2].contiguous(), [0.2, 0.2, 0.2])
+    assert rel_err(out, ref.cpu().numpy()) <= RTOL_FP32
