@@ -263,6 +263,7 @@ struct BlurArgs {
     const uint32_t* dst_map;    // row index of vertex v in dst (vertex -> slot); null: v
     int wc;                     // homogeneous weight channel (homogeneous rows only)
     int products = 0;           // homogeneous rows written as plain products (the last pass)
+    int chained = 0;            // follows another pass directly on the stream
 };
 
 // Slice segments are the splat's for the replay slice; for a slice at other positions
@@ -957,6 +958,10 @@ __global__ void blur_kernel(BlurArgs a) {
     const PS* src = reinterpret_cast<const PS*>(a.src);
     PD* dst = reinterpret_cast<PD*>(a.dst);
     const uint32_t m = *a.nverts;
+    // A pass after another is launched while that one drains, and waits here for its rows;
+    // only the count, which no pass writes, is read before.
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t vtx = blockIdx.x * blockDim.x + threadIdx.x; vtx < m; vtx += stride * ILP) {
         A out[VDP];
