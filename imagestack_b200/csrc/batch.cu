@@ -209,6 +209,22 @@ MetaLayout layout(int nseg, bool slice_segs) {
 
 size_t batch_meta_bytes(int nseg) { return layout(nseg, false).total; }
 
+// Whether two axes per blur pass are faster than one, by the vertices and points expected.
+// A pair saves a pass over memory; it reads nine rows and two more pairs of neighbours in
+// places of their own where two passes read three rows each.  Blur, pairs against single:
+// - few vertices, where launches count: 64x64 (3.5 k) 13 us, 15; 512x512 sigma 8 (142 k) 20,
+//   21; from 200 k on single is faster: 256x256 sigma 4 (211 k) 26, 24; 4K sigma 32 (539 k)
+//   56, 44; 4K sigma 16 (1.5 M) 126, 102; video d=6 (1.4 M) 130, 108; d=8 (3.5 M) 346, 347;
+// - rows beyond L2 (over 3.5 M) whose neighbours are near in memory: 4K sigmas 4 and 0.3
+//   (3.9 M, 0.47 per point) 255, 281; 4 and 0.1 (10.9 M, 1.3 per point) 880, 925;
+// - and far apart: 4K sigmas 4 and 0.05 (25.6 M, 3.1 per point) 3256, 2577; 8 and 0.05 (12.2 M,
+//   1.47 per point) 1156, 1086; d=16, 2M points (15.4 M) 6833, 5787.
+// 16-bit rows: 256 images (9.3 M) 5.40 ms in all, 5.43.
+static bool pairs_pay(int d, int payload, double vertices, uint64_t points) {
+    if (payload != kPayloadF32 || vertices < 2e5) return true;
+    return vertices > 3.5e6 && d < 10 && vertices < 1.4 * (double)points;
+}
+
 // Queue one pass over the batch on st, its metadata staged in the pinned buffer h (E.hmeta
 // when null); *ps receives what finish_pass needs once the stream has run it.  timed: CUDA
 // events around every stage (read by finish_pass).
@@ -326,11 +342,14 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     // rows (16-bit payloads: FP32 rows, homogeneous ones normalised by the neighbour
     // search, once per vertex) and the slice reads rows by vertex index.
     const bool vrows = vertex_rows_wanted(B) && !wide && tiled_count == nseg;
+    double expected = 0;   // vertices
+    for (int k = 0; k < nseg; ++k) expected += (double)cap[k] * load / 1.3;
     // PGPU_BLUR=pairs or =single in the environment overrides the blur pairing (tests)
     const char* blur_mode = std::getenv("PGPU_BLUR");
     const bool blur_pairs = blur_mode && !strcmp(blur_mode, "pairs") ? true
                           : blur_mode && !strcmp(blur_mode, "single") ? false
-                                                                       : B.blur_pairs;
+                                                                       : B.blur_pairs >= 0 ? B.blur_pairs != 0
+                                                                       : pairs_pay(d, B.payload, expected, n_total);
     // one neighbour lookup per axis (the splat's creators or the compaction mark the pairs
     // absent first); PGPU_NBR=half or =both in the environment overrides the job's choice
     const char* nbr_mode = std::getenv("PGPU_NBR");

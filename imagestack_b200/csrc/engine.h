@@ -165,7 +165,7 @@ struct BatchJob {
     bool replay = true;    // slice at the splat points
     bool use_graph = false;   // capture / replay the launch sequence as a CUDA graph
     bool autotune = false;    // pick load factor and blur pairing per batch shape
-    bool blur_pairs = true;   // blur two axes per launch
+    int blur_pairs = -1;   // blur two axes per launch (1), one (0), as pairs_pay says (-1)
     int blur_grid = 0;        // 0: 16 blocks per SM striding over the vertices, 1: one vertex per
                               // thread, 2: as 0 with two vertices per iteration (one-axis passes)
     int splat = 0;            // 0: the tile splat where vertices are shared, 1: direct only

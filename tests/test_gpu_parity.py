@@ -477,3 +477,17 @@ def test_host_copies_in_chunks_match_device_memory(gpu, w, h, rows):
     dev = torch.from_numpy(big[:, rows].copy()).cuda()
     ref = gpu.GaussTransform.apply(None, dev, dev[:2].contiguous(), [0.2, 0.2, 0.2])
     assert rel_err(out, ref.cpu().numpy()) <= RTOL_FP32
+
+
+@pytest.mark.parametrize("mode", ["pairs", "single"])
+@pytest.mark.parametrize("d", [9, 10, 13, 16])
+def test_blur_passes_match_the_oracle_in_many_dimensions(gpu, monkeypatch, mode, d):
+    """Axes in pairs and one by one, of odd and even numbers of axes."""
+    monkeypatch.setenv("PGPU_BLUR", mode)
+    rng = np.random.default_rng(d)
+    n = 1211
+    pos = (rng.integers(0, 4, (n, 1)) * 1.5 + rng.normal(0, 0.3, (n, d))).astype(np.float32)
+    val = rng.uniform(0, 1, (n, 4)).astype(np.float32)
+    planar = lambda a: np.ascontiguousarray(a.T).reshape(a.shape[1], 1, n)
+    out = gpu.GaussTransform.apply(None, planar(pos), planar(val), [1.0] * d)
+    assert rel_err(out.reshape(-1, n).T, oracle.oracle_lattice(pos, val).out) <= RTOL_FP32
