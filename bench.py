@@ -110,6 +110,20 @@ def stage_bytes(N, M, d=D, C=3, p=4, vdp=4, vertex_rows=False, nbr_half=False):
             "blur": int(blur), "slice": int(slice_)}
 
 
+def moved_bytes(N, M, d=D, C=3, p=4, vdp=4, vertex_rows=False, nbr_half=False):
+    """stage_bytes with what compact keys change (d <= 7): keys of 8 bytes, which the splat's
+    creators also write in vertex order with both index maps and, for the one-lookup search,
+    the vertex's absent lower neighbours; no compaction, the neighbour search gathers slot
+    rows."""
+    axes = d + 1
+    b = stage_bytes(N, M, d, C, p, vdp, vertex_rows, nbr_half)
+    lookups = axes if nbr_half else 2 * axes
+    b["splat"] = N * C * 4 + N * axes * 8 + M * (8 + 4 * vdp) + M * (8 + 8) + (M * 4 * axes if nbr_half else 0)
+    b["compact"] = 0
+    b["neighbours"] = M * 8 + lookups * M * 8 + axes * M * 8 + (0 if vertex_rows else M * (4 + 4 * vdp + p * vdp))
+    return b
+
+
 def ncu_traffic():
     """DRAM bytes of each stage for one 3840x2160 frame, from the committed ncu summary."""
     path = os.path.join(ROOT, "profiles", "dram_traffic_bilateral_4k_frame.txt")
@@ -739,12 +753,12 @@ def run_ours(args):
         plain_stages = {k: round(statistics.mean(s[k] for s in plain_stage), 4)
                         for k in ("ms_splat", "ms_compact", "ms_neighbours", "ms_blur",
                                   "ms_slice", "ms_total")}
-        # Algorithmic bytes of each stage (stage_bytes: formulas that follow the kernels),
+        # Algorithmic bytes of each stage (moved_bytes: formulas that follow the kernels),
         # for all frames of the batch and M = the measured vertices of the batch
         p = {"fp32": 4, "fp16": 2, "bf16": 2, "fp64": 8}[args.payload]
         N = FRAMES_PER_STEP * n
         passes = blur_launches(D, bool(stage[-1]["blur_pairs"]))
-        sb = stage_bytes(N, M, p=p, vertex_rows=bool(stage[-1]["vertex_rows"]),
+        sb = moved_bytes(N, M, p=p, vertex_rows=bool(stage[-1]["vertex_rows"]),
                          nbr_half=bool(stage[-1]["nbr_half"]))
         splat_bytes = sb["splat"]
         achieved = splat_bytes / (splat_ms / 1e3) / 1e9
@@ -833,7 +847,7 @@ def run_ours(args):
                                        else "16 blocks per SM, striding",
                           "splat": "tile" if stage[-1]["tiled"] else "direct",
                           "rows": "vertex-ordered by the splat" if stage[-1]["vertex_rows"]
-                                  else "slot space + compaction",
+                                  else "slot space",
                           "neighbour_lookups_per_axis": 1 if stage[-1]["nbr_half"] else 2,
                           "tiles": "%dx%d" % (stage[-1]["tile_w"], 256 // max(1, stage[-1]["tile_w"])),
                           "calls": tune_calls,

@@ -350,7 +350,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
                           : blur_mode && !strcmp(blur_mode, "single") ? false
                                                                        : B.blur_pairs >= 0 ? B.blur_pairs != 0
                                                                        : pairs_pay(d, B.payload, expected, n_total);
-    // one neighbour lookup per axis (the splat's creators or the compaction mark the pairs
+    // one neighbour lookup per axis (whoever numbers a vertex marks its down neighbours
     // absent first); PGPU_NBR=half or =both in the environment overrides the job's choice
     const char* nbr_mode = std::getenv("PGPU_NBR");
     const bool nbr_half = nbr_mode && !strcmp(nbr_mode, "half") ? true
@@ -822,15 +822,15 @@ static int run_batch_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     return finish_pass(E, B, ps, failed, cap_next);
 }
 
-// Autotuner: coordinate descent over six knobs, starting from load 0.5, the tile splat,
-// slot-space rows, two neighbour lookups, blur axes in pairs and the capped blur grid.
+// Autotuner: coordinate descent over seven knobs, starting from load 0.5, the tile splat,
+// slot-space rows, one neighbour lookup, blur axes in pairs and the capped blur grid.
 // Each knob's options are tried with the best setting found so far for the other knobs,
 // each twice (the faster time counts: the first call of a shape also learns its vertex
 // ratio), by the device time of what the knob changes (knob_time):
 //   0. hash-table load factor 0.5 / 0.35 / 0.7;
 //   1. splat: the tile splat wherever the learned vertex density allows it, or the direct
 //      splat for every image;
-//   2. rows: in slot space with a compaction into vertex order, or numbered by the tile
+//   2. rows: in slot space, gathered by the neighbour search, or numbered by the tile
 //      splat as it creates the vertices, in vertex order from the start (where every image
 //      of the batch takes the tile splat);
 //   3. neighbour search: one lookup per axis (n1), the other pair entry written by the
@@ -840,7 +840,7 @@ static int run_batch_pass(Engine& E, const BatchJob& B, cudaStream_t st,
 //      second, as a pair rounds them, so the results are the same bit for bit);
 //   5. blur grid: 16 blocks per SM striding over the vertices, one vertex per thread, or
 //      (one-axis passes) 16 blocks per SM with two vertices per iteration;
-//   6. tile splat tiles (the blocks per image): 16x16 or 32x8 pixels (splat time).
+//   6. tile splat tiles (the blocks per image): 16 or 32 pixels wide (splat time).
 // Keys, vertex order and FP32/FP64 results do not depend on the choice.
 constexpr float kTuneLoads[] = {0.5f, 0.35f, 0.7f};
 constexpr int kTuneKnobs = 7;

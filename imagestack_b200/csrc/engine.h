@@ -57,7 +57,7 @@ struct Engine {
     std::mutex mu;
     // hash table (slot space)
     DevBuf key0, keyn, tvals, ft, slot2vtx;
-    // compaction
+    // numbering of dumps, and of int16-lane lattices
     DevBuf bitmap, offs, partials;
     // vertex space (vkey: compact keys, vkey0/vkeyn: int16-lane keys)
     DevBuf vkey, vkey0, vkeyn, vv0, vv1, nbr;
@@ -66,7 +66,7 @@ struct Engine {
     DevBuf sval;       // filtered rows in slot space, arithmetic type, read by the slice
     DevBuf rec;        // row and weight of every (point, remainder), recorded by the splat
     DevBuf grid, grid2;   // the dense grid of the grid method, and its blur's second buffer
-    DevBuf tags;       // one tag byte per hash slot (compaction -> neighbour lookups)
+    DevBuf tags;       // one tag byte per hash slot (multi-word keys: splat -> neighbour lookups)
     DevBuf vlist;      // slots in the order the splat created them (the vertex list)
     DevBuf dstat;
     // batch metadata: statuses, counts, segment tables (device copy of hmeta)
@@ -169,7 +169,7 @@ struct BatchJob {
     int blur_grid = 0;        // 0: 16 blocks per SM striding over the vertices, 1: one vertex per
                               // thread, 2: as 0 with two vertices per iteration (one-axis passes)
     int splat = 0;            // 0: the tile splat where vertices are shared, 1: direct only
-    bool slot_rows = true;    // rows in slot space with a compaction; false: the tile splat
+    bool slot_rows = true;    // rows in slot space; false: the tile splat
                               // numbers vertices and fills vertex-ordered rows where it can
     int nbr_half = 1;         // one neighbour lookup per axis (1) or two (0)
     bool wide = false;        // int16-lane keys (a lattice whose keys do not fit compact keys)
@@ -196,7 +196,7 @@ struct PassState {
     uint64_t n_total = 0, cap_total = 0;
     int timed = 0;   // 0: no events, 1: events around every stage, 2: around a graph
     int nbr_half = 0;   // the neighbour search looked up one direction per axis
-    int vertex_rows = 0;   // the splat filled vertex-ordered rows (no compaction)
+    int vertex_rows = 0;   // the splat filled vertex-ordered rows
     int blur_pairs = 1;    // blur axes fused in pairs
     int tile_w = 16;       // tile splat tile width
 };

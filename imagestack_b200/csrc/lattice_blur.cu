@@ -38,7 +38,7 @@ void blur_t(const BlurArgs& a, bool pair, int blocks, int ilp, cudaStream_t st) 
     else blur_launch(blur_kernel<VDP, PS, PD, HOMOG, false, 1>, a, blocks, st);
 }
 
-// 16-bit payload P: rows are P between passes, FP32 when read from the compaction
+// 16-bit payload P: rows are P between passes, FP32 when read from the splat
 // (homogeneous lattices) or written for the slice (last pass)
 template <int VDP, typename P, bool HOMOG>
 void blur_16(const BlurArgs& a, bool src_f32, bool dst_acc, bool pair, int blocks,

@@ -1,5 +1,6 @@
-// Kernels that do not depend on the number of position dimensions: first-touch
-// marking, the prefix popcount that numbers the vertices, compaction and the blur.
+// Kernels that do not depend on the number of position dimensions: clearing a pass's tables,
+// first-touch marking, the prefix popcount that numbers the vertices of parity dumps, and the
+// compaction of the int16-lane lattices.
 #include <algorithm>
 
 #include "lattice_ops.h"

@@ -1,4 +1,7 @@
-// Kernels of the permutohedral-lattice Gauss transform (sm_100a).
+// Kernels of the permutohedral-lattice Gauss transform (sm_100a): the blur and the replay
+// slice of every lattice, and the whole pipeline on int16-lane keys, which runs where compact
+// keys (lattice_compact.cuh, the main path) do not: keys out of their range, FP64 rows, the
+// allocation-free entry point.
 //
 // Pipeline for one lattice (one image, or one segment of a batch):
 //   splat      one thread per point: positions from the planar images, elevation and
@@ -928,7 +931,7 @@ __device__ __forceinline__ void blurred_row(const PS* src, const int* nbr, size_
 }
 
 // PS/PD: row types read and written.  They differ for the first pass of a homogeneous
-// 16-bit lattice (FP32 rows from the compaction) and for the last pass of a 16-bit
+// 16-bit lattice (normalised FP32 rows) and for the last pass of a 16-bit
 // lattice (FP32 rows in slot space for the slice).  A fused pair computes the first
 // axis's rows in registers with the same arithmetic a separate pass would store, so in
 // FP32 it is bit-identical to two passes.

@@ -100,7 +100,7 @@ struct BlurPlan {
     size_t nbr_stride;
     const uint32_t* nverts;
     uint32_t vmax;
-    const void* src;       // the compaction's rows in vertex order
+    const void* src;       // the rows in vertex order
     void* bufs[2];
     void* f32buf = nullptr;   // FP32 rows (16-bit payloads, one axis per pass)
     void* sval;

@@ -83,8 +83,8 @@ typedef struct pgpu_stats {
                               vertex per thread, 2 as 0 with two vertices per iteration */
     int tuned;             /* autotuner: 0 off, 1 this call was one of its trials, 2 its choice */
     int nbr_half;          /* 1: one neighbour lookup per axis (the other pair entry scattered) */
-    int vertex_rows;       /* 1: the splat numbered vertices and filled vertex-ordered rows (no compaction) */
-    int tile_w;            /* tile splat tile width in pixels (tiles of 256 pixels) */
+    int vertex_rows;       /* 1: the splat numbered vertices and filled vertex-ordered rows */
+    int tile_w;            /* tile splat tile width in pixels (of 256 pixels; 128 for small images) */
 } pgpu_stats;
 
 /* Fill *opt with the defaults. */
@@ -133,9 +133,9 @@ int pgpu_bilateral(pgpu_image *im, float filter_width, float filter_height,
  * opt->flags & PGPU_FLAG_AUTOTUNE lets the first calls of each batch shape (the number
  * of images, the point count to a power of two, d, the payload) try candidate settings
  * one knob at a time — hash-table load factor 0.5, 0.35 or 0.7, the tile splat where it
- * applies or the direct splat for every image, rows compacted from hash-slot space or
+ * applies or the direct splat for every image, rows in hash-slot space or
  * numbered in vertex order by the splat, one or two neighbour lookups per axis, blur axes
- * fused in pairs or one per pass, the blur's launch shape, 16x16 or 32x8 splat tiles —
+ * fused in pairs or one per pass, the blur's launch shape, splat tiles 16 or 32 pixels wide —
  * and keeps the fastest for later calls of that shape (opt->load_factor is then unused);
  * results do not depend on the choice beyond the FP32 tolerance. */
 #define PGPU_FLAG_GRAPH 1
