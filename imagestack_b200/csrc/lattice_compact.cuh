@@ -302,27 +302,39 @@ __device__ __forceinline__ int ck_find(const typename CompactKey<D>::T* tab, uin
 // a slot's tag: odd, from hash bits that the home sector does not use
 __device__ __forceinline__ uint8_t ck_tag(uint32_t mix) { return (uint8_t)(ck_fold(mix) | 1u); }
 
+// Of eight slots' tags (slot 0's the low byte), those from slot `first` on that may be `tag`, up to
+// the first empty slot: the top bit of each one's byte, counted from slot `first`.  Every tag that
+// matches is among them (a byte next above one may be too, the key decides); slots behind the
+// eight never are.  *end: one of them is empty.
+__host__ __device__ __forceinline__ uint64_t tag_matches(uint64_t word, uint32_t first, uint8_t tag, bool* end) {
+    constexpr uint64_t kOnes = 0x0101010101010101ull, kTops = 0x8080808080808080ull;
+    const uint32_t sh = first * 8u;
+    // behind the word's end, bytes that are not empty
+    const uint64_t x = sh ? (word >> sh) | (0x0202020202020202ull << (64u - sh)) : word;
+    const uint64_t empty = (x - kOnes) & ~x & kTops;   // lowest set: the first zero byte
+    const uint64_t y = x ^ (tag * kOnes);
+    uint64_t match = (y - kOnes) & ~y & kTops & (~0ull >> sh);
+    if (empty) match &= (empty & (0 - empty)) - 1;
+    *end = empty != 0;
+    return match;
+}
+
 // the slot of a 128-bit key by the slots' tags, from slot s (a sector's first) on; word: the
 // eight tags that hold s's.  -1 if absent.  Slots of a sector fill in order, so tags behind the
-// first empty one are not the key's.
+// first empty one are not the key's.  (As many slots as ck_insert tries: kMaxProbe, from s on,
+// lie in one word more than kMaxProbe / 8 where s is not a word's first.)
 __device__ __forceinline__ int ck_find_tagged(const uint4* tab, const uint64_t* tags, uint32_t cap, const uint4& key,
                                               uint32_t s, uint64_t word) {
-    constexpr uint64_t kOnes = 0x0101010101010101ull, kTops = 0x8080808080808080ull;
-    const uint64_t tag = ck_tag(ck_mix(key)) * kOnes;
+    const uint8_t tag = ck_tag(ck_mix(key));
 #pragma unroll 1
-    for (int probe = 0; probe < kMaxProbe / 8; ++probe) {
-        const uint32_t sh = (s & 7u) * 8u;
-        // tags from s on, low byte first; behind the word's end, neither empty nor any key's
-        const uint64_t x = sh ? (word >> sh) | (0x0202020202020202ull << (64u - sh)) : word;
-        const uint64_t empty = (x - kOnes) & ~x & kTops;   // lowest set: the first zero byte
-        const uint64_t y = x ^ tag;
-        uint64_t match = (y - kOnes) & ~y & kTops;         // bytes equal to the tag (and perhaps some above)
-        if (empty) match &= (empty & (0 - empty)) - 1;
+    for (int probe = 0; probe <= kMaxProbe / 8; ++probe) {
+        bool end;
+        uint64_t match = tag_matches(word, s & 7u, tag, &end);
         for (; match; match &= match - 1) {
             const uint32_t at = s + ((uint32_t)(__ffsll((long long)match) - 1) >> 3);
             if (words_equal(__ldg(tab + at), key)) return (int)at;
         }
-        if (empty) return -1;
+        if (end) return -1;
         s = (s | 7u) + 1u;
         if (s >= cap) s = 0;
         word = __ldg(tags + (s >> 3));
