@@ -33,11 +33,15 @@ struct CompactKey {
     static constexpr int kPerWord = (D + 3) / 4;      // 128-bit keys: fields per 32-bit word
     static constexpr int kFieldBits = kOneWord ? ((63 - kRemBits) / D < 16 ? (63 - kRemBits) / D : 16)
                                       : kPerWord == 2 ? 14 : kPerWord == 3 ? 9 : 7;
-    // largest quotient of a point: room for its remainders' steps and their neighbours, and
-    // coordinates clear of the int16 range's ends, where the reference's short keys wrap
-    static constexpr int kMaxField = (1 << (kFieldBits - 1)) - 2;
+    // Largest quotient of a greedy point.  The walk back onto the hyperplane moves it by one, a
+    // remainder's step lowers it by one and a neighbour lies one further either way, and all of
+    // these have to stay inside the field: a carry would make another vertex's key of it.
+    // And coordinates stay clear of the int16 range's ends, where the reference's short keys wrap.
+    static constexpr int kMaxField = (1 << (kFieldBits - 1)) - 3;
     static constexpr int kMaxAbs = 32767 / (D + 1) - 2;
     static constexpr int kMaxQ = kMaxAbs < kMaxField ? kMaxAbs : kMaxField;
+    static_assert(kMaxQ + 3 <= (1 << (kFieldBits - 1)) && kMaxQ + 2 < (1 << (kFieldBits - 1)),
+                  "the neighbours of a point's vertices fit the fields");
     __host__ __device__ static constexpr int word(int i) { return kOneWord ? 0 : i / kPerWord; }
     __host__ __device__ static constexpr int shift(int i) {
         return kOneWord ? kRemBits + i * kFieldBits : (i % kPerWord) * kFieldBits;

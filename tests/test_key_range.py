@@ -1,0 +1,105 @@
+"""Lattices whose keys lie at the ends of what a compact key's fields hold, and beyond: the
+results have to be those of the reference's int16 keys wherever the positions lie."""
+import numpy as np
+import pytest
+
+import oracle
+from test_gpu_parity import RTOL_FP32, rel_err
+
+pytestmark = pytest.mark.gpu
+
+# bits of a quotient's field by d (64-bit keys to d = 7, 128 above), and the quotients where
+# compact keys end
+FIELD_BITS = {5: 12, 6: 10, 7: 8, 9: 9, 12: 9, 13: 7, 15: 7, 16: 7}
+
+
+def elevation(d):
+    """The linear map of positions to the lattice's d+1 coordinates (src/Permutohedral.h:293-299)."""
+    sf = np.empty(64, np.float32)
+    oracle._load_oracle().lo_scale_factors(d, sf)
+    e = np.zeros((d + 1, d))
+    e[d, d - 1] = -d * sf[d - 1]
+    for i in range(d - 1, 0, -1):
+        e[i] = e[i + 1]
+        e[i, i - 1] -= i * sf[i - 1]
+        e[i, i] += (i + 2) * sf[i]
+    e[0] = e[1]
+    e[0, 0] += 2 * sf[0]
+    return e
+
+
+def positions(coords):
+    """Positions whose lattice coordinates are `coords` (rows of d+1 numbers of sum zero)."""
+    d = coords.shape[1] - 1
+    return np.ascontiguousarray((coords @ np.linalg.pinv(elevation(d)).T).astype(np.float32))
+
+
+def check(gpu, pos, val):
+    ref = oracle.oracle_lattice(pos, val)
+    got = gpu.lattice_dump(pos, val)
+    for k in ("keys", "replay_vtx", "replay_w"):
+        np.testing.assert_array_equal(got[k], getattr(ref, k))
+    for k in ("splat", "blur", "out"):
+        assert rel_err(got[k], getattr(ref, k)) <= RTOL_FP32
+
+
+@pytest.mark.parametrize("step", [-1, 0, 1, 2])
+@pytest.mark.parametrize("d", sorted(FIELD_BITS))
+def test_quotients_at_the_ends_of_the_fields(gpu, d, step):
+    """Points whose greedy quotients are the largest a compact key takes, and one or two
+    more, along every coordinate and at both ends."""
+    rng = np.random.default_rng(10 * d + step)
+    top = (1 << (FIELD_BITS[d] - 1)) - 3 + step
+    q = np.zeros((2 * (d + 1), d + 1))
+    for i in range(d + 1):
+        q[2 * i, i], q[2 * i, (i + 1) % (d + 1)] = top, -top
+        q[2 * i + 1, i], q[2 * i + 1, (i + 2) % (d + 1)] = -top, top
+    off = rng.uniform(-0.9, 0.9, (20, 2 * (d + 1), d + 1)) * (d + 1)
+    coords = (q * (d + 1) + off - off.mean(2, keepdims=True)).reshape(-1, d + 1)
+    val = rng.uniform(0, 1, (len(coords), 4)).astype(np.float32)
+    check(gpu, positions(coords), val)
+
+
+def points_around(c, r, i, rank_i, rng, n):
+    """n points of simplices that have vertex c (d+1 coordinates, remainder r), coordinate i
+    of rank rank_i in them (src/Permutohedral.h:367-369)."""
+    d = len(c) - 1
+    coords = np.empty((n, d + 1))
+    for k in range(n):
+        rank = rng.permutation(d + 1)
+        j = int(np.flatnonzero(rank == rank_i)[0])
+        rank[j], rank[i] = rank[i], rank_i
+        step = np.array([np.where(rank <= d - s, s, s - (d + 1)) for s in range(d + 1)])
+        coords[k] = c - step[r] + rng.dirichlet(np.ones(d + 1)) @ step
+    return positions(coords)
+
+
+@pytest.mark.parametrize("mode,ends", [
+    # neighbour down of remainder 1, quotient 63: quotient 64 would carry into remainder 16
+    ("both", ((1, 63, -56, 15), (16, -64, 56, 1))),
+    # neighbour up of remainder 15, quotient -64: quotient -65 would borrow from remainder 16
+    ("half", ((15, -64, 56, 2), (0, 63, -56, 16))),
+])
+def test_no_neighbour_across_a_field_of_sixteen_dimensions(gpu, monkeypatch, mode, ends):
+    """Two far points with a vertex each whose keys differ by what a carry out of coordinate
+    11's 7-bit field would make of the first one's neighbour along that axis."""
+    monkeypatch.setenv("PGPU_NBR", mode)
+    d, i = 16, 11
+    rng = np.random.default_rng(1)
+    e = elevation(d)
+    pos = []
+    for r, q_i, q_d, rank_i in ends:
+        q = np.zeros(d + 1)
+        q[i], q[d] = q_i, q_d
+        q[:int(q.sum() + r)] = -1   # the coordinates' sum is zero
+        c = q * (d + 1) + r
+        assert c.sum() == 0
+        p = points_around(c, r, i, rank_i, rng, 4000)
+        keys, _ = oracle.oracle_simplex(p)
+        has = (keys[:, r] == c[:d]).all(1)
+        # the greedy point's quotients are 62 at most
+        has &= np.abs(np.rint(p.astype(np.float64) @ e.T / (d + 1))).max(1) <= 62
+        assert has.sum() >= 3
+        pos.append(p[has][:3])
+    pos = np.concatenate(pos)
+    check(gpu, pos, rng.uniform(0.5, 1, (len(pos), 4)).astype(np.float32))
