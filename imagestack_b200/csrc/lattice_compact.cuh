@@ -15,7 +15,9 @@
 //    a few 32-bit multiplies.
 // Quotients reach about 0.75 of a position in sigmas, so fields hold images thousands of
 // sigmas across at d <= 5 and hundreds at d = 6 and 7.  A point whose keys do not fit sets
-// kStatusWide, and the host runs the lattice again on the int16-lane keys.
+// kStatusWide in the splat, before anything is written, and the host runs the lattice again on
+// the int16-lane keys.  A slice at other positions asks for no rerun: a position out of the
+// fields' range takes the int16 arithmetic on its own (slice_far_point).
 #pragma once
 
 #include <type_traits>
@@ -611,7 +613,7 @@ __device__ __forceinline__ void load_image_point(const PointSource& s, uint32_t 
 }
 
 // Phases A and B of a warp's pixels (positions pp; valid: in the image, cleared where the keys
-// are out of range): their weights, the list (in s_claim, after use) and number of their
+// are out of range, and kStatusWide set unless status is null): their weights, the list (in s_claim, after use) and number of their
 // vertices, each the entry that stands for it, and loc2, each entry's vertex (two entries to a
 // register).  The entry of remainder r of pixel k of a lane is e = b*32 + lane, b = k*(D+1) + r.
 template <int D, int NP>
@@ -626,7 +628,7 @@ __device__ __forceinline__ uint32_t tile_vertices(const float (&pp)[NP][D], cons
         uint2* scr = reinterpret_cast<uint2*>(s_key + k * (D + 1) * 32 + lane);
         int q[D + 1];
         if (!compact_simplex<D>(pp[k], lc, q, scr, 32)) {
-            atomicOr(status, kStatusWide);
+            if (status) atomicOr(status, kStatusWide);
             valid[k] = false;
             continue;
         }
@@ -1149,11 +1151,74 @@ __device__ __forceinline__ void write_slice(const OutView& ov, int vd, uint32_t 
         if (k < ov.channels) o[(long long)k * ov.cstride] = ov.normalize ? acc[k] / wsum : acc[k];
 }
 
+// A vertex's key from its int16 coordinates; false where they are no compact key
+template <int D>
+__device__ __forceinline__ bool ck_from_coords(const int (&k)[D], typename CompactKey<D>::T& key) {
+    using K = CompactKey<D>;
+    constexpr int kHalf = 1 << (K::kFieldBits - 1);
+    const int r = ((k[0] % (D + 1)) + D + 1) % (D + 1);
+    int q[D + 1];
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+        q[i] = (k[i] - r) / (D + 1);
+        ok = ok && q[i] * (D + 1) + r == k[i] && q[i] >= -kHalf && q[i] < kHalf;
+    }
+    key = ck_first<D>(q);
+    if constexpr (K::kOneWord) {
+        key += (uint64_t)r;
+    } else {
+        key.w += (uint32_t)(r & 15) << 28;
+        if (D >= 16) key.z += (uint32_t)(r >> 4) << 28;
+    }
+    return ok;
+}
+
+// The slice of a position whose greedy point does not fit a compact key: the reference's int16
+// simplex (compute_simplex; a position beyond int16 sets kStatusKeyRange, which fails the
+// call), and each vertex on its own.  All vertices of the splat are compact keys, so one that
+// is none was never created and contributes zero.  (Deciding this here, and not by a rerun of
+// the lattice, matters beyond time: other blocks have written by now, and the output may be
+// one of the inputs.)  Rare, so kept out of the callers' registers.
+template <int D, int VDP>
+__device__ __noinline__ void slice_far_point(const CompactSliceArgs& a, const Segment& sg, uint32_t x, uint32_t y,
+                                             uint32_t f, unsigned* status, float (&acc)[VDP]) {
+    using K = CompactKey<D>;
+    using T = typename K::T;
+    constexpr int B = K::kBucket;
+    float p[D];
+    load_position_xyt<D>(sg.src, x, y, f, p);
+    float delta[D + 1];
+    unsigned char coord[D + 1];
+    Simplex<D> sx;
+    compute_simplex<D>(p, a.lc, sx, status, SimplexScratch{delta, coord, 1, 1});
+    const T* tab = reinterpret_cast<const T*>(a.keys) + sg.slot_base;
+    const uint32_t sectors = sg.cap / B;
+#pragma unroll
+    for (int k = 0; k < VDP; ++k) acc[k] = 0.0f;
+#pragma unroll 1
+    for (int r = 0; r <= D; ++r) {
+        int kc[D];
+        vertex_coords<D>(sx, r, kc);
+        T key;
+        if (!ck_from_coords<D>(kc, key)) continue;
+        const uint32_t b = __umulhi(ck_fold(ck_mix(key)), sectors);
+        T in[B];
+        read_sector(tab + (size_t)b * B, in);
+        const int s = ck_find<D>(tab, sectors, key, b, in);
+        if (s < 0) continue;
+        float row[VDP];
+        load_row<VDP, float, float>(a.rows + (size_t)sg.slot_base * VDP, s, row);
+#pragma unroll
+        for (int k = 0; k < VDP; ++k) acc[k] = acc_add(acc[k], sx.bary[r] * row[k]);
+    }
+}
+
 // d <= 7: as the tile splat, a warp finds the vertices of 64 pixels first and looks each up once
-//
 constexpr int kTileSlicePx = 2;
 template <int D, int VDP>
-__global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D, 2)) compact_tile_slice_kernel(CompactSliceArgs a) {
+__global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D, 2)) compact_tile_slice_kernel(
+    const __grid_constant__ CompactSliceArgs a) {
     using K = CompactKey<D>;
     constexpr int NP = kTileSlicePx;
     static_assert(kTileThreads * NP == kSliceThreads, "a slice block's pixels");
@@ -1185,11 +1250,11 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D, 2)) compact_t
             valid[k] = px < (uint32_t)sg.src.width && py < (uint32_t)sg.src.height;
             if (valid[k]) load_position_xyt<D>(sg.src, px, py, fr, pp[k]);
         }
-        count = tile_vertices<D, NP>(pp, a.lc, status, s_key, s_list, lane, valid, bary, loc2);
+        count = tile_vertices<D, NP>(pp, a.lc, nullptr, s_key, s_list, lane, valid, bary, loc2);
     }
     // a lattice whose splat failed is rerun by the host; its output may be its input, so
-    // write nothing
-    if (__ldcg(status) & kStatusFailed) return;
+    // write nothing (the warp decides as one: its lanes look up each other's vertices)
+    if (__any_sync(0xFFFFFFFFu, (__ldcg(status) & kStatusFailed) != 0)) return;
     const uint64_t* tab = reinterpret_cast<const uint64_t*>(a.keys) + sg.slot_base;
     const uint32_t sectors = sg.cap / K::kBucket;
 #pragma unroll 1
@@ -1205,8 +1270,15 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D, 2)) compact_t
     const float* rows = a.rows + (size_t)sg.slot_base * VDP;
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
-        if (!valid[k]) continue;
+        const uint32_t p = lane * NP + k;
+        const uint32_t px = x0 + (p & ((1u << wsh) - 1u)), py = y0 + (p >> wsh);
         float acc[VDP];
+        if (!valid[k]) {
+            if (px >= (uint32_t)sg.src.width || py >= (uint32_t)sg.src.height) continue;
+            slice_far_point<D, VDP>(a, sg, px, py, fr, status, acc);
+            write_slice<VDP>(sg.out, a.vd, px, py, fr, acc);
+            continue;
+        }
 #pragma unroll
         for (int i = 0; i < VDP; ++i) acc[i] = 0.0f;
 #pragma unroll
@@ -1218,13 +1290,12 @@ __global__ void __launch_bounds__(kTileThreads, tile_min_blocks(D, 2)) compact_t
 #pragma unroll
             for (int i = 0; i < VDP; ++i) acc[i] = acc_add(acc[i], bary[k][r] * row[i]);
         }
-        const uint32_t p = lane * NP + k;
-        write_slice<VDP>(sg.out, a.vd, x0 + (p & ((1u << wsh) - 1u)), y0 + (p >> wsh), fr, acc);
+        write_slice<VDP>(sg.out, a.vd, px, py, fr, acc);
     }
 }
 
 template <int D, int VDP>
-__global__ void __launch_bounds__(kSliceThreads) compact_slice_kernel(CompactSliceArgs a) {
+__global__ void __launch_bounds__(kSliceThreads) compact_slice_kernel(const __grid_constant__ CompactSliceArgs a) {
     using K = CompactKey<D>;
     using T = typename K::T;
     constexpr int AH = direct_ahead<D>();
@@ -1240,21 +1311,22 @@ __global__ void __launch_bounds__(kSliceThreads) compact_slice_kernel(CompactSli
     const uint32_t py = ty * sg.slice_th + (threadIdx.x >> sg.slice_shift);
     if (px >= (uint32_t)sg.src.width || py >= (uint32_t)sg.src.height) return;
     unsigned* status = a.seg_status + kseg;
-    float p[D];
-    load_position_xyt<D>(sg.src, px, py, fr, p);
-    int q[D + 1];
-    if (!compact_simplex<D>(p, a.lc, q, scr, kSliceThreads)) {
-        atomicOr(status, kStatusWide);
-        return;
-    }
     // a lattice whose splat failed is rerun by the host; its output may be its input, so
     // write nothing
     if (__ldcg(status) & kStatusFailed) return;
+    float p[D];
+    load_position_xyt<D>(sg.src, px, py, fr, p);
+    int q[D + 1];
+    float acc[VDP];
+    if (!compact_simplex<D>(p, a.lc, q, scr, kSliceThreads)) {
+        slice_far_point<D, VDP>(a, sg, px, py, fr, status, acc);
+        write_slice<VDP>(sg.out, a.vd, px, py, fr, acc);
+        return;
+    }
     const T* tab = reinterpret_cast<const T*>(a.keys) + sg.slot_base;
     const float* rows = a.rows + (size_t)sg.slot_base * VDP;
     const uint32_t sectors = sg.cap / K::kBucket;
     T key = ck_first<D>(q);
-    float acc[VDP];
 #pragma unroll
     for (int k = 0; k < VDP; ++k) acc[k] = 0.0f;
 #pragma unroll 1

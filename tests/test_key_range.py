@@ -1,5 +1,7 @@
 """Lattices whose keys lie at the ends of what a compact key's fields hold, and beyond: the
 results have to be those of the reference's int16 keys wherever the positions lie."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -103,3 +105,61 @@ def test_no_neighbour_across_a_field_of_sixteen_dimensions(gpu, monkeypatch, mod
         pos.append(p[has][:3])
     pos = np.concatenate(pos)
     check(gpu, pos, rng.uniform(0.5, 1, (len(pos), 4)).astype(np.float32))
+
+
+def transform_into(gpu, slice_pos, splat_pos, values, out):
+    """pgpu_gauss_transform of device memory with an output of the caller's choice, which may
+    be one of the inputs."""
+    d = splat_pos.shape[0]
+    views = [gpu._view(t, "view")[0] for t in (slice_pos, splat_pos, values, out)]
+    opt = gpu._options(gpu.MEM_DEVICE, "fp32", stream=gpu._torch_stream(values))
+    gpu._check(gpu.lib().pgpu_gauss_transform(C.byref(views[0]), C.byref(views[1]), C.byref(views[2]),
+                                              (C.c_float * d)(*[1.0] * d), d, C.byref(views[3]), C.byref(opt)))
+
+
+@pytest.mark.parametrize("into", ["new", "values", "slice"])
+@pytest.mark.parametrize("d,reach", [(1, 18000.0), (3, 9000.0), (5, 4500.0), (7, 600.0), (9, 2000.0), (16, 400.0)])
+def test_slice_positions_out_of_the_compact_range(gpu, d, reach, into):
+    """The splat's positions fit compact keys, a few of the slice's do not (they stay within the
+    reference's int16 keys) and have no vertices; the output may be one of the inputs."""
+    import torch
+    rng = np.random.default_rng(7 * d)
+    n = 40000 + len(into)   # images of their own shape: nothing is known of them
+    pos = (rng.integers(0, 4, (n, 1)) * 3.0 + rng.normal(0, 0.4, (n, d))).astype(np.float32)
+    other = (pos[::-1] + rng.normal(0, 0.3, (n, d))).astype(np.float32)
+    other[n - 700::7, d - 1] += np.linspace(-reach, reach, 100).astype(np.float32)
+    val = rng.uniform(0, 1, (n, d)).astype(np.float32)[:, :min(d, 8)]
+    if into == "slice" and val.shape[1] < d:
+        pytest.skip("as many values as positions, to write over them")
+    ref = oracle.oracle_lattice(pos, val, slice_pos=other).out
+    planar = lambda a: torch.from_numpy(np.ascontiguousarray(a.T).reshape(a.shape[1], 1, n)).cuda()
+    ts, tp, tv = planar(other), planar(pos), planar(val)
+    transform_into(gpu, tp, tp, tv, torch.empty_like(tv))   # the table's size is learned
+    out = {"new": torch.empty_like(tv), "values": tv, "slice": ts}[into]
+    transform_into(gpu, ts, tp, tv, out)
+    torch.cuda.synchronize()
+    assert rel_err(out.cpu().numpy().reshape(-1, n).T, ref) <= RTOL_FP32
+    assert gpu.last_stats()["retries"] == 0
+
+
+@pytest.mark.parametrize("d,sign", [(1, 1), (1, -1), (3, 1), (3, -1), (4, 1)])
+def test_slice_positions_at_the_ends_of_int16(gpu, d, sign):
+    """Vertices near one end of int16 and slice positions near both: keys that wrap around in
+    the reference's shorts wrap here too, and positions beyond int16 fail the call."""
+    rng = np.random.default_rng(3 * d + sign)
+    top = 32767 // (d + 1)
+    def at(q0, n):
+        q = np.zeros((n, d + 1))
+        q[:, 0], q[:, d] = q0, -q0
+        off = rng.uniform(-0.45, 0.45, (n, d + 1)) * (d + 1)
+        return positions(q * (d + 1) + off - off.mean(1, keepdims=True))
+    pos = at(sign * (top - 3), 500)
+    val = rng.uniform(0, 1, (500, 2)).astype(np.float32)
+    other = np.concatenate([at(sign * (top - 3), 300), at(sign * (top - 1), 300), at(-sign * (top - 1), 300)])
+    ref = oracle.oracle_lattice(pos, val, slice_pos=other).out
+    planar = lambda a: np.ascontiguousarray(a.T).reshape(a.shape[1], 1, len(a))
+    out = gpu.GaussTransform.apply(planar(other), planar(pos), planar(val), [1.0] * d)
+    assert rel_err(out.reshape(2, -1).T, ref) <= RTOL_FP32
+    with pytest.raises(gpu.PgpuError):
+        far = at(sign * (top + 3), 10)
+        gpu.GaussTransform.apply(planar(far), planar(pos), planar(val), [1.0] * d)
