@@ -828,8 +828,11 @@ __device__ __forceinline__ double blur3(double a, double b, double c) {
     return __dadd_rn(__dadd_rn(0.25 * a, 0.5 * b), 0.25 * c);
 }
 
-// Row of vertex u (zeros for an absent vertex, u < 0), in arithmetic type A.
-template <int VDP, typename PS, typename A>
+// Row of vertex u (zeros for an absent vertex, u < 0), in arithmetic type A.  FIXED: no kernel
+// writes src while this one runs, which is what a read-only load asks for.  Not so in a blur
+// pass: it is launched while the pass before it still writes these rows, so it reads them with
+// ordinary loads, which stay behind its wait for that pass.
+template <int VDP, typename PS, typename A, bool FIXED = true>
 __device__ __forceinline__ void load_row(const PS* src, int u, A (&r)[VDP]) {
     // rows of 4 are read as one vector; an absent vertex (u < 0) reads vertex 0's row,
     // which exists whenever any vertex does, and is then replaced by zeros
@@ -837,14 +840,16 @@ __device__ __forceinline__ void load_row(const PS* src, int u, A (&r)[VDP]) {
     if constexpr (std::is_same<PS, float>::value && VDP % 4 == 0) {
 #pragma unroll
         for (int k = 0; k < VDP; k += 4) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(src + base + k));
+            const float4* at = reinterpret_cast<const float4*>(src + base + k);
+            const float4 q = FIXED ? __ldg(at) : *at;
             r[k] = (A)q.x, r[k + 1] = (A)q.y, r[k + 2] = (A)q.z, r[k + 3] = (A)q.w;
         }
     } else if constexpr ((std::is_same<PS, __half>::value || std::is_same<PS, __nv_bfloat16>::value) &&
                          VDP % 4 == 0) {
 #pragma unroll
         for (int k = 0; k < VDP; k += 4) {
-            const uint2 q = __ldg(reinterpret_cast<const uint2*>(src + base + k));
+            const uint2* at = reinterpret_cast<const uint2*>(src + base + k);
+            const uint2 q = FIXED ? __ldg(at) : *at;
             const PS* h = reinterpret_cast<const PS*>(&q);
 #pragma unroll
             for (int j = 0; j < 4; ++j) r[k + j] = (A)Payload<PS>::load(h + j);
@@ -924,9 +929,9 @@ __device__ __forceinline__ void blurred_row(const PS* src, const int* nbr, size_
     }
     const int2 nb = load_pair(nbr, stride, (uint32_t)u);
     A r1[VDP], r0[VDP], r2[VDP];
-    load_row<VDP, PS, A>(src, nb.x, r1);
-    load_row<VDP, PS, A>(src, u, r0);
-    load_row<VDP, PS, A>(src, nb.y, r2);
+    load_row<VDP, PS, A, false>(src, nb.x, r1);
+    load_row<VDP, PS, A, false>(src, u, r0);
+    load_row<VDP, PS, A, false>(src, nb.y, r2);
     combine3<VDP, A, HOMOG>(r1, r0, r2, wc, out);
 }
 
@@ -982,12 +987,12 @@ __global__ void blur_kernel(BlurArgs a) {
             const int2 na = load_pair(a.nbrA, a.nbr_stride, vtx);
             const int2 nb = two ? load_pair(a.nbrA, a.nbr_stride, v2) : make_int2(-1, -1);
             A p1[VDP], p0[VDP], p2[VDP], q1[VDP], q0[VDP], q2[VDP];
-            load_row<VDP, PS, A>(src, na.x, p1);
-            load_row<VDP, PS, A>(src, (int)vtx, p0);
-            load_row<VDP, PS, A>(src, na.y, p2);
-            load_row<VDP, PS, A>(src, nb.x, q1);
-            load_row<VDP, PS, A>(src, two ? (int)v2 : -1, q0);
-            load_row<VDP, PS, A>(src, nb.y, q2);
+            load_row<VDP, PS, A, false>(src, na.x, p1);
+            load_row<VDP, PS, A, false>(src, (int)vtx, p0);
+            load_row<VDP, PS, A, false>(src, na.y, p2);
+            load_row<VDP, PS, A, false>(src, nb.x, q1);
+            load_row<VDP, PS, A, false>(src, two ? (int)v2 : -1, q0);
+            load_row<VDP, PS, A, false>(src, nb.y, q2);
             combine3<VDP, A, HOMOG>(p1, p0, p2, a.wc, out);
             put_row<VDP, PD, A, HOMOG>(a, dst, vtx, out);
             if (two) {
