@@ -674,7 +674,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
                 (uint64_t)(uintptr_t)E.tvals.p, (uint64_t)(uintptr_t)E.nbr.p, (uint64_t)(uintptr_t)E.rec.p,
                 (uint64_t)(uintptr_t)E.meta.p, (uint64_t)(uintptr_t)h,
                 (uint64_t)(uintptr_t)E.sval.p, (uint64_t)(uintptr_t)E.vlist.p, (uint64_t)(uintptr_t)E.vv0.p,
-                (uint64_t)(uintptr_t)E.vv1.p, (uint64_t)(uintptr_t)E.vkey0.p, (uint64_t)(uintptr_t)E.vf32.p,
+                (uint64_t)(uintptr_t)E.vv1.p, (uint64_t)(uintptr_t)E.vkey0.p, (uint64_t)(uintptr_t)E.vkeyn.p,
+                (uint64_t)(uintptr_t)E.vf32.p,
                 (uint64_t)vrows, (uint64_t)wide, (uint64_t)(uintptr_t)E.vkey.p,
                 (uint64_t)(uintptr_t)E.slot2vtx.p, (uint64_t)(uintptr_t)E.tags.p, (uint64_t)(uintptr_t)E.vtx2slot.p, (uint64_t)nbr_half, (uint64_t)B.tile_w};
             gk.reserve(gk.size() + 2 * (size_t)nseg);
