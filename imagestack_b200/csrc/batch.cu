@@ -727,10 +727,10 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
 }
 
 // The rest of a pass once st has run it: statuses, learned ratios, statistics.  Images
-// whose range overflowed are listed in *failed, with the larger range to use in *cap_next
-// (when given); their output is untouched (the slice skips them), while every other image
-// of the pass is finished.
-static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::vector<int>* failed,
+// whose range overflowed, or whose keys were too wide, are listed in *failed, with the range to
+// use in *cap_next (when given); their output is untouched (the slice skips them), while every
+// other image of the pass is finished.
+static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::vector<FailedImage>* failed,
                        std::vector<uint64_t>* cap_next) {
     const int d = B.d, nseg = (int)B.items.size();
     if (nseg == 0) return PGPU_OK;
@@ -746,7 +746,7 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
                         "image %d: positions leave the lattice's int16 key range (the reference's "
                         "keys wrap there and its rank indices leave [0, d]); scale them down", k);
         if (segstat[k] & kStatusWide) {   // rerun on int16-lane keys, now and later
-            failed->push_back(k);
+            failed->push_back({k, true});
             if (cap_next) cap_next->push_back(ps.cap[k]);
             retry = true;
             std::lock_guard<std::mutex> lk(g_ratio_mu);
@@ -754,7 +754,7 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
             g_wide_sigs.insert(ps.sig[k]);
         } else if (segstat[k] & (kStatusProbeLimit | kStatusSpinLimit)) {
             uint64_t c = std::max<uint64_t>((uint64_t)(ps.cap[k] * 2.5), (uint64_t)(counts[k] / ps.load * 2));
-            failed->push_back(k);
+            failed->push_back({k, false});
             if (cap_next) cap_next->push_back((c + 31) & ~31ull);
             retry = true;
         }
@@ -767,7 +767,7 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
         std::lock_guard<std::mutex> lk(g_ratio_mu);
         if (g_ratio_by_sig.size() > 4096) g_ratio_by_sig.clear();
         for (int k = 0; k < nseg; ++k) {
-            if (fi < failed->size() && (*failed)[fi] == k) {
+            if (fi < failed->size() && (*failed)[fi].item == k) {
                 ++fi;
                 continue;
             }
@@ -813,7 +813,7 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
 }
 
 static int run_batch_pass(Engine& E, const BatchJob& B, cudaStream_t st,
-                          const std::vector<uint64_t>* cap_in, std::vector<int>* failed,
+                          const std::vector<uint64_t>* cap_in, std::vector<FailedImage>* failed,
                           std::vector<uint64_t>* cap_next, int pass) {
     if (B.items.empty()) return PGPU_OK;
     PassState ps;
@@ -964,7 +964,7 @@ int enqueue_batch(Engine& E, const BatchJob& B, cudaStream_t st, unsigned char* 
     return enqueue_pass(E, B, st, nullptr, h, false, 0, ps);
 }
 
-int finish_batch(Engine& E, const BatchJob& B, const PassState& ps, std::vector<int>* failed) {
+int finish_batch(Engine& E, const BatchJob& B, const PassState& ps, std::vector<FailedImage>* failed) {
     return finish_pass(E, B, ps, failed, nullptr);
 }
 
@@ -975,7 +975,7 @@ static int run_passes(Engine& E, BatchJob cur, cudaStream_t st, pgpu_stats* sum)
     std::vector<uint64_t> caps;
     memset(sum, 0, sizeof(*sum));
     for (int pass = 0; pass < 6; ++pass) {
-        std::vector<int> failed;
+        std::vector<FailedImage> failed;
         std::vector<uint64_t> next;
         const int rc = run_batch_pass(E, cur, st, caps.empty() ? nullptr : &caps, &failed, &next, pass);
         if (rc) return rc;
@@ -999,11 +999,13 @@ static int run_passes(Engine& E, BatchJob cur, cudaStream_t st, pgpu_stats* sum)
             sum->tile_w = s.tile_w;
             return PGPU_OK;
         }
-        // (an image that did not fit compact keys is known by now, so the pass, with every
-        // image in it, runs on int16-lane keys)
+        // one image that did not fit compact keys takes the others of its next pass with it
         BatchJob again = cur;
         again.items.clear();
-        for (int k : failed) again.items.push_back(cur.items[k]);
+        for (const FailedImage& f : failed) {
+            again.items.push_back(cur.items[f.item]);
+            again.wide = again.wide || f.wide;
+        }
         caps = next;
         cur = std::move(again);
     }

@@ -674,7 +674,7 @@ void complete_oldest(Engine& E) {
     memset(&sum, 0, sizeof(sum));
     for (AsyncChunk& c : ab->chunks) {
         if (rc) break;
-        std::vector<int> failed;
+        std::vector<FailedImage> failed;
         const int r = finish_batch(E, c.job, c.ps, &failed);
         if (r) {
             rc = r;
@@ -694,7 +694,7 @@ void complete_oldest(Engine& E) {
             sum.tuned = c.job.autotune ? 2 : 0;
             sum.tiled += s.tiled;
         }
-        for (int k : failed) again.push_back(c.i0 + k);
+        for (const FailedImage& f : failed) again.push_back(c.i0 + f.item);
     }
     if (!rc && !again.empty()) {
         // the slots may hold later batches' images: wait for everything queued

@@ -208,9 +208,14 @@ bool tuned_settings(Engine& E, const BatchJob& B, BatchJob* out);
 // Queue the first pass of B on st with its metadata staged in the pinned buffer h (at
 // least batch_meta_bytes), without waiting for it.
 int enqueue_batch(Engine& E, const BatchJob& B, cudaStream_t st, unsigned char* h, PassState* ps);
-// Once st has run the pass: statuses, learned vertex ratios, statistics.  Images whose
-// range overflowed (their output left as it was) are listed in *failed.
-int finish_batch(Engine& E, const BatchJob& B, const PassState& ps, std::vector<int>* failed);
+// An image to be filtered again: its table overflowed, or (wide) it needs int16-lane keys.
+struct FailedImage {
+    int item;
+    bool wide;
+};
+// Once st has run the pass: statuses, learned vertex ratios, statistics.  Images to be
+// filtered again (their output left as it was) are listed in *failed.
+int finish_batch(Engine& E, const BatchJob& B, const PassState& ps, std::vector<FailedImage>* failed);
 
 struct LatticeJob {
     int d = 0, vd = 0, payload = 0;
