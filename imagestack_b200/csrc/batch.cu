@@ -92,8 +92,11 @@ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 std::mutex g_ratio_mu;
 std::unordered_map<uint64_t, double> g_ratio_by_sig;
 std::map<int, double> g_ratio;
-// signatures of images whose keys did not fit compact keys: their later lattices start on
-// int16-lane keys (a wrong entry costs time, not results)
+// Signatures of images whose latest lattice needed int16-lane keys: the next ones start on
+// them.  A signature holds no data, so an entry is a guess: it costs time, not results.  Every
+// finished pass on int16 lanes says whether its images would have fitted compact keys
+// (kStatusFar), so one far image does not hold back those that follow, and an image that fails
+// the call leaves nothing.
 std::unordered_set<uint64_t> g_wide_sigs;
 
 // Lattices on int16-lane keys: asked for (a rerun), FP64 accumulators, PGPU_KEYS=wide in the
@@ -465,6 +468,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sa.rec = replay_w ? E.rec.p : nullptr;
             sa.seg_status = (unsigned*)(dmeta + L.segstat);
             sa.blocks = (uint32_t)blocks;
+            // (the walk back onto the hyperplane moves a quotient by one)
+            sa.fit = (ops->max_quotient - 1) * (d + 1);
             if (!ops->splat(sa, vdp, B.payload, st)) return fail(PGPU_ERR_UNSUPPORTED, "splat variant");
             } else {
             CompactSplatArgs sa;
@@ -720,6 +725,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
         ps->timed = timed ? (graph ? 2 : 1) : 0;
         ps->nbr_half = nbr_half ? 1 : 0;
         ps->vertex_rows = vrows ? 1 : 0;
+        ps->wide = wide;
         ps->blur_pairs = blur_pairs ? 1 : 0;
         ps->tile_w = B.tile_w ? B.tile_w : 16;
         return PGPU_OK;
@@ -745,13 +751,10 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
             return fail(PGPU_ERR_ARGUMENT,
                         "image %d: positions leave the lattice's int16 key range (the reference's "
                         "keys wrap there and its rank indices leave [0, d]); scale them down", k);
-        if (segstat[k] & kStatusWide) {   // rerun on int16-lane keys, now and later
+        if (segstat[k] & kStatusWide) {   // rerun on int16-lane keys
             failed->push_back({k, true});
             if (cap_next) cap_next->push_back(ps.cap[k]);
             retry = true;
-            std::lock_guard<std::mutex> lk(g_ratio_mu);
-            if (g_wide_sigs.size() > 4096) g_wide_sigs.clear();
-            g_wide_sigs.insert(ps.sig[k]);
         } else if (segstat[k] & (kStatusProbeLimit | kStatusSpinLimit)) {
             uint64_t c = std::max<uint64_t>((uint64_t)(ps.cap[k] * 2.5), (uint64_t)(counts[k] / ps.load * 2));
             failed->push_back({k, false});
@@ -772,6 +775,12 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
                 continue;
             }
             done_vertices += counts[k];
+            if (ps.wide && (segstat[k] & kStatusFar)) {
+                if (g_wide_sigs.size() > 4096) g_wide_sigs.clear();
+                g_wide_sigs.insert(ps.sig[k]);
+            } else if (ps.wide) {
+                g_wide_sigs.erase(ps.sig[k]);
+            }
             if (!B.items[k].n) continue;
             const double r = (double)counts[k] / (double)B.items[k].n;
             g_ratio_by_sig[ps.sig[k]] = r;

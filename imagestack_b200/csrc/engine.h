@@ -197,6 +197,7 @@ struct PassState {
     int timed = 0;   // 0: no events, 1: events around every stage, 2: around a graph
     int nbr_half = 0;   // the neighbour search looked up one direction per axis
     int vertex_rows = 0;   // the splat filled vertex-ordered rows
+    bool wide = false;     // int16-lane keys
     int blur_pairs = 1;    // blur axes fused in pairs
     int tile_w = 16;       // tile splat tile width
 };

@@ -139,7 +139,8 @@ bool compact_slice(const CompactSliceArgs& a, int vdp, cudaStream_t st) {
     return false;
 }
 
-const DimOps kOps = {splat, neighbours, slice, compact_splat, compact_rank, compact_neighbours, compact_slice};
+const DimOps kOps = {splat, neighbours, slice, compact_splat, compact_rank, compact_neighbours, compact_slice,
+                     CompactKey<D>::kMaxQ};
 
 }  // namespace
 

@@ -24,6 +24,7 @@ constexpr unsigned kStatusProbeLimit = 1u;   // hash table too full: rerun with 
 constexpr unsigned kStatusSpinLimit = 2u;    // a pending slot never became ready
 constexpr unsigned kStatusKeyRange = 4u;     // an elevated coordinate left the int16 range
 constexpr unsigned kStatusWide = 8u;         // keys out of the compact keys' range: rerun with int16 lanes
+constexpr unsigned kStatusFar = 16u;         // a lattice on int16 lanes may need them (no failure)
 
 // ---------------------------------------------------------------------------------
 // Keys.  A vertex key is d int16 coordinates (the (d+1)-th is implied, the keys of

@@ -174,6 +174,8 @@ struct SplatArgs {
     uint32_t* vlist;
     uint32_t* vcount;
     uint32_t* seg_counts;
+    // a coordinate beyond this sets kStatusFar: the lattice may not fit compact keys (0: not asked)
+    int fit = 0;
 };
 
 // Appends of one block to the batch's vertex list: slots go to the block's shared-memory
@@ -489,6 +491,12 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     Simplex<D> sx;
     const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kSplatThreads, kSplatThreads};
     compute_simplex<D>(p, a.lc, sx, status, scr);
+    if (a.fit) {
+        bool far = false;
+#pragma unroll
+        for (int k = 0; k <= D; ++k) far = far || abs(sx.g[k]) > a.fit;
+        if (far && !(__ldcg(status) & kStatusFar)) atomicOr(status, kStatusFar);
+    }
     const uint32_t gi = sg.point_base + i;   // point number in the batch
     const uint32_t e0 = gi * (uint32_t)(D + 1);
     Acc* vals = reinterpret_cast<Acc*>(a.vals) + (size_t)sg.slot_base * VDP;

@@ -25,6 +25,7 @@ struct DimOps {
     void (*compact_rank)(const CompactRankArgs&, int sms, cudaStream_t);
     void (*compact_neighbours)(const CompactNbrArgs&, uint32_t vmax, int sms, cudaStream_t);
     bool (*compact_slice)(const CompactSliceArgs&, int vdp, cudaStream_t);
+    int max_quotient;   // of a greedy point that fits compact keys
 };
 
 // bytes of a compact key

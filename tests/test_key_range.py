@@ -163,3 +163,33 @@ def test_slice_positions_at_the_ends_of_int16(gpu, d, sign):
     with pytest.raises(gpu.PgpuError):
         far = at(sign * (top + 3), 10)
         gpu.GaussTransform.apply(planar(far), planar(pos), planar(val), [1.0] * d)
+
+
+def test_an_image_that_needs_wide_keys_does_not_mark_its_shape(gpu):
+    """Images of one shape: after one that needs int16 lanes the next starts on them; after one
+    that does not, or one that fails the call, compact keys are tried first (a rerun where
+    they do not fit)."""
+    rng = np.random.default_rng(3)
+    noise = rng.uniform(0, 1, (3, 61, 83)).astype(np.float32)   # nearly no vertex is shared, so
+    near, far = noise * np.float32(16.0), noise * np.float32(3000.0)   # both need the same table
+    bad = near.copy()
+    bad[1, 30, 40] = np.nan
+
+    def reruns(img):
+        out = img.copy()
+        gpu.Bilateral.apply(out, 6.0, 6.0, 0.0, 0.8)
+        pos, val = oracle.bilateral_points(img, img, 6.0, 0.8)
+        ref = oracle.oracle_lattice(pos, val).out
+        norm = (ref[:, :3] / ref[:, 3:4]).reshape(61, 83, 3).transpose(2, 0, 1)
+        assert rel_err(out, norm) <= RTOL_FP32
+        return gpu.last_stats()["retries"]
+
+    reruns(near)   # the table's size is learned
+    for _ in range(2):
+        assert reruns(near) == 0   # (on int16 lanes the second time round)
+        assert reruns(near) == 0
+        with pytest.raises(gpu.PgpuError):
+            gpu.Bilateral.apply(bad, 6.0, 6.0, 0.0, 0.8)
+        assert reruns(near) == 0
+        assert reruns(far) >= 1
+        assert reruns(far) == 0
