@@ -969,6 +969,16 @@ bool tuned_settings(Engine& E, const BatchJob& B, BatchJob* out) {
     return true;
 }
 
+std::vector<std::vector<int>> key_groups(const BatchJob& B) {
+    std::vector<uint64_t> sig;
+    for (const BatchItem& it : B.items) sig.push_back(item_signature(B.d, it.splat));
+    const std::vector<char> wide = known_wide(sig);
+    const bool all_wide = wide_forced(B);
+    std::vector<std::vector<int>> g(2);
+    for (size_t k = 0; k < sig.size(); ++k) g[!all_wide && wide[k] ? 1 : 0].push_back((int)k);
+    return g;
+}
+
 int enqueue_batch(Engine& E, const BatchJob& B, cudaStream_t st, unsigned char* h, PassState* ps) {
     return enqueue_pass(E, B, st, nullptr, h, false, 0, ps);
 }

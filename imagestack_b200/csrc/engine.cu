@@ -607,14 +607,14 @@ constexpr size_t kChunkPixels = size_t(1) << 22;
 }  // namespace
 
 namespace pgpu {
-// One queued chunk of a submitted host batch: its lattice job (device slot views), the
-// queued pass and the pinned buffer its metadata is staged in.
+// One queued pass of a submitted host batch: its lattice job (device slot views) and whose
+// images these are, the queued pass and the pinned buffer its metadata is staged in.
 struct AsyncChunk {
     BatchJob job;
     PassState ps;
     unsigned char* h = nullptr;
     size_t h_bytes = 0;
-    int i0 = 0, i1 = 0;
+    std::vector<int> images;   // the batch's image of each item
 };
 
 struct AsyncBatch {
@@ -654,7 +654,7 @@ void pinned_put(Engine& E, unsigned char* p, size_t bytes) {
 
 int bilateral_batch_host(Engine& E, cudaStream_t st, const pgpu_image* ims, const pgpu_image* outs,
                          int count, const float* filter_width, const float* color_sigma,
-                         const pgpu_options& opt, AsyncBatch* ab);
+                         const pgpu_options& opt, AsyncBatch* ab, bool wide = false);
 
 // Finish the oldest queued batch (its download stream has reached its event): statuses and
 // learned ratios of every chunk; images whose hash range overflowed were left unfiltered
@@ -669,7 +669,7 @@ void complete_oldest(Engine& E) {
         rc = fail(PGPU_ERR_CUDA, "queued batch: %s", cudaGetErrorString(ce));
         msg = last_error();
     }
-    std::vector<int> again;
+    std::vector<int> again[2];   // to be filtered again: as before, and on int16 lanes
     pgpu_stats sum;
     memset(&sum, 0, sizeof(sum));
     for (AsyncChunk& c : ab->chunks) {
@@ -694,23 +694,24 @@ void complete_oldest(Engine& E) {
             sum.tuned = c.job.autotune ? 2 : 0;
             sum.tiled += s.tiled;
         }
-        for (const FailedImage& f : failed) again.push_back(c.i0 + f.item);
+        for (const FailedImage& f : failed) again[f.wide].push_back(c.images[f.item]);
     }
-    if (!rc && !again.empty()) {
+    for (int wide = 0; wide < 2; ++wide) {
+        if (rc || again[wide].empty()) continue;
         // the slots may hold later batches' images: wait for everything queued
         cudaStreamSynchronize(E.copy_in);
         cudaStreamSynchronize(E.stream);
         cudaStreamSynchronize(E.copy_out);
         std::vector<pgpu_image> in, out;
         std::vector<float> fw, cs;
-        for (int i : again) {
+        for (int i : again[wide]) {
             in.push_back(ab->in[i]);
             out.push_back(ab->out[i]);
             fw.push_back(ab->fw[i]);
             cs.push_back(ab->cs[i]);
         }
         rc = bilateral_batch_host(E, E.stream, in.data(), out.data(), (int)in.size(), fw.data(), cs.data(),
-                                  ab->opt, nullptr);
+                                  ab->opt, nullptr, wide != 0);
         if (rc) msg = last_error();
         else sum.retries = 1;
     }
@@ -734,7 +735,7 @@ namespace {
 
 int bilateral_batch_host(Engine& E, cudaStream_t st, const pgpu_image* ims, const pgpu_image* outs,
                          int count, const float* filter_width, const float* color_sigma,
-                         const pgpu_options& opt, AsyncBatch* ab) {
+                         const pgpu_options& opt, AsyncBatch* ab, bool wide) {
     const int C = ims[0].channels;
     std::vector<int> cut{0};
     size_t acc = 0, slot_floats = 0, chunk_floats = 0;
@@ -815,17 +816,29 @@ int bilateral_batch_host(Engine& E, cudaStream_t st, const pgpu_image* ims, cons
             CUDA_TRY(cudaStreamWaitEvent(st, uploaded[slot_of[k]], 0));
             BatchJob B;
             bilateral_job(dv.data(), cut[k], cut[k + 1], filter_width, color_sigma, opt, B);
+            B.wide = wide;
             if (ab) {
                 // queued: the autotuner's choice, no host wait (checked when it completes)
-                AsyncChunk c;
-                c.i0 = cut[k];
-                c.i1 = cut[k + 1];
-                tuned_settings(E, B, &c.job);
-                c.h = pinned_get(E, batch_meta_bytes((int)c.job.items.size()), &c.h_bytes);
-                if (!c.h) return fail(PGPU_ERR_MEMORY, "pinned allocation for a queued batch failed");
-                ab->chunks.push_back(std::move(c));
-                AsyncChunk& q = ab->chunks.back();
-                if ((r = enqueue_batch(E, q.job, st, q.h, &q.ps))) break;
+                BatchJob tuned;
+                tuned_settings(E, B, &tuned);
+                const std::vector<std::vector<int>> groups = key_groups(tuned);
+                for (size_t g = 0; g < groups.size() && !r; ++g) {
+                    if (groups[g].empty()) continue;
+                    AsyncChunk c;
+                    c.job = tuned;
+                    c.job.wide = tuned.wide || g == 1;
+                    c.job.items.clear();
+                    for (int item : groups[g]) {
+                        c.job.items.push_back(tuned.items[item]);
+                        c.images.push_back(cut[k] + item);
+                    }
+                    c.h = pinned_get(E, batch_meta_bytes((int)c.job.items.size()), &c.h_bytes);
+                    if (!c.h) return fail(PGPU_ERR_MEMORY, "pinned allocation for a queued batch failed");
+                    ab->chunks.push_back(std::move(c));
+                    AsyncChunk& q = ab->chunks.back();
+                    r = enqueue_batch(E, q.job, st, q.h, &q.ps);
+                }
+                if (r) break;
             } else {
                 if ((r = run_batch(E, B, st))) break;
                 pgpu_stats s;

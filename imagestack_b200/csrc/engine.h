@@ -206,6 +206,9 @@ size_t batch_meta_bytes(int nseg);
 // Settings the autotuner chose for B's shape; false while its trials are not finished
 // (an untuned shape runs through run_batch, which times the trials).
 bool tuned_settings(Engine& E, const BatchJob& B, BatchJob* out);
+// The images of B in groups that one pass each can take: those to try on compact keys, and those
+// known to need int16 lanes (B.wide is set for these; none where all of B is on int16 lanes).
+std::vector<std::vector<int>> key_groups(const BatchJob& B);
 // Queue the first pass of B on st with its metadata staged in the pinned buffer h (at
 // least batch_meta_bytes), without waiting for it.
 int enqueue_batch(Engine& E, const BatchJob& B, cudaStream_t st, unsigned char* h, PassState* ps);

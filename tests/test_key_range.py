@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import oracle
+from imagestack_b200 import synth
 from test_gpu_parity import RTOL_FP32, rel_err
 
 pytestmark = pytest.mark.gpu
@@ -193,3 +194,34 @@ def test_an_image_that_needs_wide_keys_does_not_mark_its_shape(gpu):
         assert reruns(near) == 0
         assert reruns(far) >= 1
         assert reruns(far) == 0
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_queued_batch_with_an_image_known_to_need_wide_keys(gpu, graph):
+    """Queued batches in which one image needs int16 lanes, unknown and known: the others stay
+    on the tile splat of compact keys, and every result lands in its own output."""
+    imgs = [synth.image(w, h, 3, rects=6, seed=w) for w, h in ((150, 91), (98, 133), (64, 65), (77, 60))]
+    imgs[1] = (imgs[1] * 3000).astype(np.float32)   # colours thousands of sigmas apart
+    fw, cs = [6.0, 5.0, 8.0, 7.0], [0.1, 0.8, 0.2, 0.3]
+    expect = [im.copy() for im in imgs]
+    for im, f, c in zip(expect, fw, cs):
+        gpu.Bilateral.apply(im, f, f, 0.0, c, payload="fp64")
+    gpu.Bilateral.apply(imgs[1].copy(), fw[1], fw[1], 0.0, cs[1])   # known from here on
+    for _ in range(3):
+        out = [np.empty_like(im) for im in imgs]
+        gpu.bilateral_batch_submit(imgs, fw, cs, outputs=out, graph=graph).wait()
+        assert gpu.last_stats()["tiled"] >= 3 and gpu.last_stats()["retries"] == 0
+        for a, b in zip(out, expect):
+            assert rel_err(a, b, floor_frac=1e-2) <= RTOL_FP32
+    # nothing known of these shapes: the first batch finds out as it completes
+    imgs = [np.ascontiguousarray(im[:, 1 + int(graph):]) for im in imgs]
+    outs = [[np.empty_like(im) for im in imgs] for _ in range(3)]
+    tickets = [gpu.bilateral_batch_submit(imgs, fw, cs, outputs=out, graph=graph) for out in outs]
+    for t in tickets:
+        t.wait()
+    expect = [im.copy() for im in imgs]
+    for im, f, c in zip(expect, fw, cs):
+        gpu.Bilateral.apply(im, f, f, 0.0, c, payload="fp64")
+    for out in outs:
+        for a, b in zip(out, expect):
+            assert rel_err(a, b, floor_frac=1e-2) <= RTOL_FP32
