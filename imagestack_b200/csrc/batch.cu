@@ -156,11 +156,12 @@ std::vector<char> known_wide(const std::vector<uint64_t>& sig) {
     return w;
 }
 
-// Splat kernel per lattice: the tile splat (vertices found per 8x8 pixels first) where
-// neighbouring points share vertices, which the learned vertices-per-point ratio tells
-// (4K d=5 bilateral: 0.18); the direct splat for sparse lattices (ratio above
-// kTileRatioMax: measured on the mixed batch, 1.5 beats 0.8 by 2 % and 0.4 by 3 %), keys of
-// 128 bits and int16-lane keys.  With nothing learned yet for the image or its d, the tile splat.
+// Splat kernel per lattice, on either form of keys: the tile splat (the vertices of 8x8 pixels,
+// on int16 lanes of 16x16, found first) where neighbouring points share vertices, which the
+// learned vertices-per-point ratio tells (4K d=5 bilateral: 0.18); the direct splat for sparse
+// lattices (ratio above kTileRatioMax: measured on the mixed batch, 1.5 beats 0.8 by 2 % and
+// 0.4 by 3 %), keys of more than one word (d >= 8) and FP64 accumulators.  With nothing learned
+// yet for the image or its d, the tile splat.
 // PGPU_SPLAT=direct or =tile in the environment overrides the choice where both exist
 // (the parity tests compare the two).
 #ifndef PGPU_TILE_RATIO_MAX
@@ -173,8 +174,8 @@ int splat_forced() {
     return !mode ? 0 : !strcmp(mode, "direct") ? 1 : !strcmp(mode, "tile") ? 2 : 0;
 }
 
-bool tile_splat_for(const BatchJob& B, bool wide, int forced, double density, uint32_t n) {
-    const bool tile_ok = key_words(B.d) == 1 && !wide && forced != 1 &&
+bool tile_splat_for(const BatchJob& B, int forced, double density, uint32_t n) {
+    const bool tile_ok = key_words(B.d) == 1 && B.payload != kPayloadF64 && forced != 1 &&
                          (forced == 2 || B.splat == 0);
     return tile_ok && (forced == 2 || (density <= kTileRatioMax && n >= 256));
 }
@@ -306,7 +307,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     const int forced = splat_forced();
     std::vector<Segment> segs(nseg), slsegs(B.replay ? 0 : nseg);
     uint64_t blocks = 0, tile_blocks = 0, slice_blocks = 0;
-    const int tile_px = tile_px_for(n_total);
+    // (the tile splat on int16 lanes takes one pixel per thread of twice the threads)
+    const int tile_px = wide ? kWideTileThreads / kTileThreads : tile_px_for(n_total);
     int tiled_count = 0;
     for (int k = 0; k < nseg; ++k) {
         const BatchItem& it = B.items[k];
@@ -316,7 +318,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
         sgm.out = it.out;
         sgm.n = it.n;
         sgm.point_base = pbase[k];
-        const bool tiled = tile_splat_for(B, wide, forced, density[k], it.n);
+        const bool tiled = tile_splat_for(B, forced, density[k], it.n);
         uint32_t nb_splat = 0, nb_tile = 0, nb_slice = 0;
         segment_geometry(sgm, B.replay ? it.splat : it.slice, tiled, &nb_splat, &nb_tile, &nb_slice,
                          wide ? kSplatThreads : kDirectThreads, (uint32_t)B.tile_w, (uint32_t)tile_px);
@@ -468,6 +470,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             sa.rec = replay_w ? E.rec.p : nullptr;
             sa.seg_status = (unsigned*)(dmeta + L.segstat);
             sa.blocks = (uint32_t)blocks;
+            sa.tile_blocks = (uint32_t)tile_blocks;
             // (the walk back onto the hyperplane moves a quotient by one)
             sa.fit = (ops->max_quotient - 1) * (d + 1);
             if (!ops->splat(sa, vdp, B.payload, st)) return fail(PGPU_ERR_UNSUPPORTED, "splat variant");
@@ -1065,7 +1068,7 @@ int run_batch(Engine& E, const BatchJob& B, cudaStream_t st) {
         for (BatchJob& p : part) p.items.clear();
         for (int k = 0; k < nseg; ++k) {
             const int to = !all_wide && wide[k] ? 2
-                           : vrows && !tile_splat_for(cur, false, forced, density[k], cur.items[k].n) ? 1 : 0;
+                           : vrows && !tile_splat_for(cur, forced, density[k], cur.items[k].n) ? 1 : 0;
             part[to].items.push_back(cur.items[k]);
         }
     } else {

@@ -31,8 +31,20 @@ void splat_t(const SplatArgs& a, cudaStream_t st) {
     if (a.blocks) splat_kernel<D, VDP, Acc><<<a.blocks, kSplatThreads, 0, st>>>(a);
 }
 
+template <int VDP>
+void wide_tile_t(const SplatArgs& a, cudaStream_t st) {
+    if constexpr (key_words(D) == 1)
+        if (a.tile_blocks) wide_tile_kernel<D, VDP><<<a.tile_blocks, kWideTileThreads, 0, st>>>(a);
+}
+
 bool splat(const SplatArgs& a, int vdp, int payload, cudaStream_t st) {
     const bool f64 = payload == kPayloadF64;
+    if (a.tile_blocks && (f64 || key_words(D) > 1)) return false;
+    switch (vdp) {
+    case 2: wide_tile_t<2>(a, st); break;
+    case 4: wide_tile_t<4>(a, st); break;
+    case 8: wide_tile_t<8>(a, st); break;
+    }
     switch (vdp) {
     case 2: f64 ? splat_t<2, double>(a, st) : splat_t<2, float>(a, st); return true;
     case 4: f64 ? splat_t<4, double>(a, st) : splat_t<4, float>(a, st); return true;

@@ -6,8 +6,9 @@
 // Pipeline for one lattice (one image, or one segment of a batch):
 //   splat      one thread per point: positions from the planar images, elevation and
 //              simplex (src/Permutohedral.h:293-356), d+1 vertex keys, warp-aggregated
-//              insert into the open-addressed table and vector atomics of the weighted
-//              values into the slot's accumulator row; atomicMin of the first touch.
+//              insert into the open-addressed table (images of d <= 7: a tile's distinct
+//              vertices once each) and vector atomics of the weighted values into the
+//              slot's accumulator row; atomicMin of the first touch.
 //   mark       one bit per (point, remainder) entry: the entry that first touched a
 //              vertex gets its bit set.
 //   scan       prefix popcount of that bitmap: the rank of a first-touch entry among
@@ -169,6 +170,7 @@ struct SplatArgs {
     void* rec;             // optional replay record: rows and weights (store_record)
     unsigned* seg_status;  // one status word per segment
     uint32_t blocks;       // direct splat blocks of the batch
+    uint32_t tile_blocks;  // tile splat blocks of the batch (d <= 7, FP32 accumulators)
     // optional vertex list: every slot the splat creates is appended to vlist (vcount
     // entries, zeroed), and counted in its segment's seg_counts entry (zeroed)
     uint32_t* vlist;
@@ -464,6 +466,16 @@ constexpr int kSplatThreads = 256;
 #endif
 __host__ __device__ constexpr int splat_min_blocks(int d) { return d <= 5 ? 6 : d <= 6 ? 4 : d <= 8 ? 3 : 2; }
 
+// kStatusFar where the greedy point may not fit a compact key (SplatArgs::fit)
+template <int D>
+__device__ __forceinline__ void note_far(const Simplex<D>& sx, int fit, unsigned* status) {
+    if (!fit) return;
+    bool far = false;
+#pragma unroll
+    for (int k = 0; k <= D; ++k) far = far || abs(sx.g[k]) > fit;
+    if (far && !(__ldcg(status) & kStatusFar)) atomicOr(status, kStatusFar);
+}
+
 template <int D, int VDP, typename Acc>
 __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kernel(SplatArgs a) {
     constexpr int KW = key_words(D);
@@ -491,12 +503,7 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     Simplex<D> sx;
     const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kSplatThreads, kSplatThreads};
     compute_simplex<D>(p, a.lc, sx, status, scr);
-    if (a.fit) {
-        bool far = false;
-#pragma unroll
-        for (int k = 0; k <= D; ++k) far = far || abs(sx.g[k]) > a.fit;
-        if (far && !(__ldcg(status) & kStatusFar)) atomicOr(status, kStatusFar);
-    }
+    note_far<D>(sx, a.fit, status);
     const uint32_t gi = sg.point_base + i;   // point number in the batch
     const uint32_t e0 = gi * (uint32_t)(D + 1);
     Acc* vals = reinterpret_cast<Acc*>(a.vals) + (size_t)sg.slot_base * VDP;
@@ -629,6 +636,151 @@ __device__ __forceinline__ void load_point_xyt(const PointSource& s, uint32_t x,
 #pragma unroll
         for (int k = 0; k < D; ++k) if (k == c) p[k] = f;
         ++c; }
+}
+
+// ---------------------------------------------------------------------------------
+// tile splat on int16-lane keys: one block per 2D tile of kWideTileThreads pixels of one frame
+// ---------------------------------------------------------------------------------
+// For images whose coordinates leave the compact keys' range at d = 6 and 7 above all: 1080p at
+// sigma 8 and d = 7, or 4K video at sigma 4 and d = 6, where neighbouring pixels share their
+// vertices as in any image (1080p d = 7: 0.6 vertices per pixel of 8 entries).  Every entry's
+// key goes into a hash table of the block's own in shared memory (phase A), each distinct
+// vertex into the global table once (phase B), and then every lane adds its rows to the global
+// slots and writes its record (phase C).  A local slot's first touch is the smallest entry that
+// reached it, so the global minimum over tiles is the reference's first insertion; vertices,
+// keys and records equal the direct splat's.  An entry that finds no free local slot within
+// kWideTileProbe goes to the global table directly, so no tile can overflow.  Bound by the
+// contended swaps in shared memory.  Splat, direct -> tile: 1280x720 sigma 4 d = 7 0.239 -> 0.193
+// ms, 1080p sigma 8 d = 7 0.48 -> 0.335, four 4K frames sigma 4 d = 6 6.6 -> 4.3.
+constexpr int kWideTileThreads = 256;    // one pixel per thread
+constexpr int kWideTileSlots = 1024;     // shared-memory hash slots per block
+constexpr int kWideTileProbe = 64;
+__host__ __device__ constexpr int wide_tile_min_blocks(int d) { return d <= 5 ? 5 : d <= 6 ? 4 : 3; }
+
+// find-or-insert of a one-word key in the block's table; a new key's slot is appended to the
+// block's list of occupied slots.  -1: no slot within the probe limit.
+__device__ __forceinline__ int wide_tile_insert(uint4* t_key, uint16_t* t_list, uint32_t* t_count, const uint4& k) {
+    static_assert(kWideTileSlots == 1024, "the home slot has 10 bits");
+    const uint32_t h = k.x * 0x9E3779B1u + k.y * 0x85EBCA77u + k.z * 0xC2B2AE3Du + (k.w & 0xFFFFu) * 0x27D4EB2Fu;
+    uint32_t l = (h ^ (h >> 15)) * 0x2C1B3C6Du >> (32 - 10);
+#pragma unroll 1
+    for (int probe = 0; probe < kWideTileProbe; ++probe) {
+        uint4 w = t_key[l];
+        if (is_empty_word(w)) {
+            w = atomicCAS_block(&t_key[l], make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu), k);
+            if (is_empty_word(w)) {
+                t_list[atomicAdd(t_count, 1u)] = (uint16_t)l;
+                return (int)l;
+            }
+        }
+        if (words_equal(w, k)) return (int)l;
+        l = (l + 1) & (kWideTileSlots - 1);
+    }
+    return -1;
+}
+
+template <int D, int VDP>
+__global__ void __launch_bounds__(kWideTileThreads, wide_tile_min_blocks(D)) wide_tile_kernel(SplatArgs a) {
+    static_assert(key_words(D) == 1, "the tile splat handles one-word keys (d <= 7)");
+    __shared__ uint4 t_key[kWideTileSlots];
+    __shared__ uint32_t t_slot[kWideTileSlots];   // a local slot's first touch, then its global slot
+    __shared__ uint16_t t_list[kWideTileSlots];
+    __shared__ uint32_t s_new[kBlockListCap];
+    __shared__ float s_delta[(D + 1) * kWideTileThreads];
+    __shared__ unsigned char s_coord[(D + 1) * kWideTileThreads];
+    __shared__ Segment sg;
+    __shared__ uint32_t t_count, s_new_count, s_new_base;
+    const int kseg = segment_by<&Segment::tile_base>(a.segs, a.nseg, blockIdx.x);
+    for (int l = threadIdx.x; l < kWideTileSlots; l += kWideTileThreads) {
+        t_key[l] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+        t_slot[l] = 0xFFFFFFFFu;
+    }
+    if (threadIdx.x == 0) t_count = 0, s_new_count = 0;
+    load_segment(a.segs + kseg, sg);   // ends with a barrier
+    const BlockList blist{s_new, &s_new_count, &s_new_base};
+
+    unsigned* status = a.seg_status + kseg;
+    const TableView table{a.key0 + sg.slot_base, a.keyn + sg.slot_base, sg.cap, a.cap_total};
+    uint32_t* ft = a.ft ? a.ft + sg.slot_base : nullptr;
+    uint32_t bt, tx;
+    const uint32_t f = div_magic(blockIdx.x - sg.tile_base, sg.tiles_x * sg.tiles_y, sg.tile_fm, &bt);
+    const uint32_t ty = div_magic(bt, sg.tiles_x, sg.tile_xm, &tx);
+    const uint32_t px = (tx << sg.tile_shift) + (threadIdx.x & (sg.tile_w - 1));
+    const uint32_t py = ty * sg.tile_h + (threadIdx.x >> sg.tile_shift);
+    const uint32_t W = (uint32_t)sg.src.width, H = (uint32_t)sg.src.height;
+    const bool valid = px < W && py < H;
+
+    // Phase A: this pixel's simplex and the local slot of each of its vertices.  loc[r] >= 0:
+    // local slot; -1: not placed; <= -2: global slot -(loc + 2)
+    float v[VDP], bary[D + 1];
+    int loc[D + 1];
+    uint32_t gi = 0;
+    if (valid) {
+        float p[D];
+        load_point_xyt<D, VDP>(sg.src, px, py, f, p, v);
+        Simplex<D> sx;
+        const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kWideTileThreads, kWideTileThreads};
+        compute_simplex<D>(p, a.lc, sx, status, scr);
+        note_far<D>(sx, a.fit, status);
+        gi = sg.point_base + (f * H + py) * W + px;
+        const uint32_t e0 = gi * (uint32_t)(D + 1);
+        Key<1> key;
+        first_key<D>(sx, key);
+#pragma unroll
+        for (int r = 0; r <= D; ++r) {
+            if (r > 0) key_step<D>(key, scr.coord[(D - (r - 1)) * scr.coord_stride]);
+            bary[r] = sx.bary[r];
+            loc[r] = wide_tile_insert(t_key, t_list, &t_count, key.w[0]);
+            if (loc[r] >= 0) {
+                if (ft) atomicMin(&t_slot[loc[r]], e0 + (uint32_t)r);
+            } else {
+                const uint32_t home = home_slot(key_hash<1>(key), table.cap);
+                bool created = false;
+                const int s = table_insert<1>(table, key, home, __ldcg(&table.key0[home]), status, &created);
+                if (s >= 0) {
+                    if (ft) atomicMin(&ft[s], e0 + (uint32_t)r);
+                    if (created && a.vlist) block_list_append(blist, a, kseg, sg.slot_base + (uint32_t)s);
+                    loc[r] = -(s + 2);
+                }
+            }
+        }
+    }
+    __syncthreads();
+
+    // Phase B: each distinct vertex of the tile into the global table once
+    const uint32_t count = t_count;
+#pragma unroll 1
+    for (uint32_t j = threadIdx.x; j < count; j += kWideTileThreads) {
+        const int l = t_list[j];
+        Key<1> kk;
+        kk.w[0] = t_key[l];
+        const uint32_t home = home_slot(key_hash<1>(kk), table.cap);
+        bool created = false;
+        const int s = table_insert<1>(table, kk, home, __ldcg(&table.key0[home]), status, &created);
+        if (s >= 0 && ft) atomicMin(&ft[s], t_slot[l]);
+        if (created && a.vlist) block_list_append(blist, a, kseg, sg.slot_base + (uint32_t)s);
+        t_slot[l] = s >= 0 ? (uint32_t)s : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    if (a.vlist) block_list_flush(blist, a, kseg);
+
+    // Phase C: every lane's rows into its vertices' rows, and the replay record
+    if (!valid) return;
+    float* vals = reinterpret_cast<float*>(a.vals);
+    uint32_t row[D + 1];
+#pragma unroll
+    for (int r = 0; r <= D; ++r) {
+        const uint32_t s = loc[r] >= 0 ? t_slot[loc[r]] : loc[r] <= -2 ? (uint32_t)(-(loc[r] + 2)) : 0xFFFFFFFFu;
+        row[r] = s != 0xFFFFFFFFu ? sg.slot_base + s : 0xFFFFFFFFu;
+        if (s != 0xFFFFFFFFu) {
+            float c[VDP];
+#pragma unroll
+            for (int k = 0; k < VDP; ++k) c[k] = __fmul_rn(bary[r], v[k]);
+            atomic_add_row<VDP>(vals + (size_t)row[r] * VDP, c);
+        }
+        if (a.rec_slot) a.rec_slot[(size_t)r * a.n_total + gi] = row[r];
+    }
+    if (a.rec) store_record<D>(a.rec, a.n_total, gi, row, bary);
 }
 
 // ---------------------------------------------------------------------------------

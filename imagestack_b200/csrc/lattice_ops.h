@@ -15,6 +15,8 @@ inline int accum_bytes(int payload) { return payload == kPayloadF64 ? 8 : 4; }
 
 // kernels whose code depends on the number of position dimensions d
 struct DimOps {
+    // on int16-lane keys: the direct splat of a.blocks blocks and the tile splat of
+    // a.tile_blocks (d <= 7, FP32 accumulators)
     bool (*splat)(const SplatArgs&, int vdp, int payload, cudaStream_t);
     void (*neighbours)(const NbrArgs&, uint32_t vmax, int sms, cudaStream_t);
     bool (*slice)(const SliceArgs&, int vdp, int payload, bool homog, cudaStream_t);

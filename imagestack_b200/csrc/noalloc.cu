@@ -192,6 +192,7 @@ extern "C" int pgpu_bilateral_noalloc(const float* d_in, float* d_out, int width
     sa.rec_slot = (uint32_t*)(base + kOffRec);
     sa.seg_status = dstatus;
     sa.blocks = splat_blocks;
+    sa.tile_blocks = 0;
     sa.rec = nullptr;     // the slice recomputes the weights
     sa.vlist = nullptr;   // vertices numbered by first touch (mark, scan, assign below)
     sa.vcount = nullptr;

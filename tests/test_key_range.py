@@ -225,3 +225,23 @@ def test_queued_batch_with_an_image_known_to_need_wide_keys(gpu, graph):
     for out in outs:
         for a, b in zip(out, expect):
             assert rel_err(a, b, floor_frac=1e-2) <= RTOL_FP32
+
+
+@pytest.mark.parametrize("rows", ["slot", "vertex"])
+@pytest.mark.parametrize("mode", ["direct", "tile"])
+@pytest.mark.parametrize("c,w,h", [(1, 257, 33), (2, 16, 16), (3, 129, 66), (4, 33, 255), (5, 40, 47), (5, 300, 1)])
+def test_int16_lane_splats_of_images(gpu, monkeypatch, c, w, h, mode, rows):
+    """Both splats on int16 lanes over whole and ragged tiles, and their dumps."""
+    monkeypatch.setenv("PGPU_KEYS", "wide")
+    monkeypatch.setenv("PGPU_SPLAT", mode)
+    monkeypatch.setenv("PGPU_ROWS", rows)
+    img = synth.image(w, max(h, 2), c, rects=5, seed=w + h)[:, :h]
+    pos, val = oracle.bilateral_points(img, img, 3.0, 0.15)
+    if h > 1:
+        out = img.copy()
+        gpu.Bilateral.apply(out, 3.0, 3.0, 0.0, 0.15)
+        ref = oracle.oracle_lattice(pos, val).out
+        norm = (ref[:, :c] / ref[:, c:]).reshape(h, w, c).transpose(2, 0, 1)
+        assert rel_err(out, norm) <= RTOL_FP32
+        assert gpu.last_stats()["tiled"] == (1 if mode == "tile" else 0)
+    check(gpu, pos, val)
