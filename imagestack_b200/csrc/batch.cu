@@ -147,12 +147,44 @@ void learned_ratios(const BatchJob& B, std::vector<uint64_t>* sig, std::vector<d
     }
 }
 
+// Whether an image's pixel coordinates alone leave the compact keys' range.  Positions are the
+// guide's channels, then the enabled coordinates, and elevated coordinate i depends on
+// positions i-1 and up only, so those above the channels are known exactly, and their extremes
+// are at the image's corners.  (Images whose channels reach too far are found out by the splat.)
+// A first call of 1080p sigma 8, d = 7, is spared a splat on compact keys that comes to nothing.
+bool coordinates_too_wide(int d, int max_quotient, const LatticeConsts& lc, const PointSource& s) {
+    const int last[3] = {s.width - 1, s.height - 1, s.frames - 1};
+    double reach[kMaxD] = {};   // each position's largest magnitude, signed; the smallest is 0
+    int n = s.pos_channels;
+    for (int k = 0; k < 3 && n < d; ++k)
+        if ((s.coord_mask >> k) & 1) reach[n++] = (double)last[k] * s.coord_scale[k];
+    double coef[kMaxD] = {};    // of each position in elevated coordinate i (src/Permutohedral.h:293-299)
+    for (int i = d; i > s.pos_channels; --i) {
+        coef[i - 1] -= (double)i * lc.sf[i - 1];
+        if (i < d) coef[i] += (double)(i + 2) * lc.sf[i];
+        double lo = 0, hi = 0;
+        for (int j = i - 1; j < d; ++j) {
+            const double e = coef[j] * reach[j];
+            (e < 0 ? lo : hi) += e;
+        }
+        // (one more for the rounding to the nearest multiple of d+1 and FP32)
+        const double limit = (double)(d + 1) * (max_quotient + 2);
+        if (-lo > limit || hi > limit) return true;
+    }
+    return false;
+}
+
 // whether each image is known not to fit compact keys
-std::vector<char> known_wide(const std::vector<uint64_t>& sig) {
+std::vector<char> known_wide(const BatchJob& B, const std::vector<uint64_t>& sig) {
     std::vector<char> w(sig.size(), 0);
+    const DimOps* ops = dim_ops(B.d);
+    if (!ops) return w;
+    const LatticeConsts lc = make_consts(B.d);
+    for (size_t k = 0; k < sig.size(); ++k)
+        w[k] = coordinates_too_wide(B.d, ops->max_quotient, lc, B.items[k].splat) ? 1 : 0;
     std::lock_guard<std::mutex> lk(g_ratio_mu);
     if (!g_wide_sigs.empty())
-        for (size_t k = 0; k < sig.size(); ++k) w[k] = g_wide_sigs.count(sig[k]) ? 1 : 0;
+        for (size_t k = 0; k < sig.size(); ++k) w[k] = w[k] || g_wide_sigs.count(sig[k]);
     return w;
 }
 
@@ -287,7 +319,8 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     std::vector<double> ratio, density;
     learned_ratios(B, &sig, &ratio, &density);
     bool wide = wide_forced(B);
-    for (char w : known_wide(sig)) wide = wide || w;
+    if (!wide && !B.keys_sorted)
+        for (char w : known_wide(B, sig)) wide = wide || w;
     const bool use_tags = kw > 1;
     const int kb = compact_key_bytes(d);
     std::vector<uint64_t> cap(nseg);
@@ -975,7 +1008,7 @@ bool tuned_settings(Engine& E, const BatchJob& B, BatchJob* out) {
 std::vector<std::vector<int>> key_groups(const BatchJob& B) {
     std::vector<uint64_t> sig;
     for (const BatchItem& it : B.items) sig.push_back(item_signature(B.d, it.splat));
-    const std::vector<char> wide = known_wide(sig);
+    const std::vector<char> wide = known_wide(B, sig);
     const bool all_wide = wide_forced(B);
     std::vector<std::vector<int>> g(2);
     for (size_t k = 0; k < sig.size(); ++k) g[!all_wide && wide[k] ? 1 : 0].push_back((int)k);
@@ -1062,10 +1095,13 @@ int run_batch(Engine& E, const BatchJob& B, cudaStream_t st) {
         std::vector<uint64_t> sig;
         std::vector<double> ratio, density;
         learned_ratios(cur, &sig, &ratio, &density);
-        const std::vector<char> wide = known_wide(sig);
+        const std::vector<char> wide = known_wide(cur, sig);
         const bool vrows = vertex_rows_wanted(cur), all_wide = wide_forced(cur);
         const int forced = splat_forced();
-        for (BatchJob& p : part) p.items.clear();
+        for (BatchJob& p : part) {
+            p.items.clear();
+            p.keys_sorted = true;
+        }
         for (int k = 0; k < nseg; ++k) {
             const int to = !all_wide && wide[k] ? 2
                            : vrows && !tile_splat_for(cur, forced, density[k], cur.items[k].n) ? 1 : 0;

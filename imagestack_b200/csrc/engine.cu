@@ -827,6 +827,7 @@ int bilateral_batch_host(Engine& E, cudaStream_t st, const pgpu_image* ims, cons
                     AsyncChunk c;
                     c.job = tuned;
                     c.job.wide = tuned.wide || g == 1;
+                    c.job.keys_sorted = true;
                     c.job.items.clear();
                     for (int item : groups[g]) {
                         c.job.items.push_back(tuned.items[item]);

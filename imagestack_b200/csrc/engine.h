@@ -173,6 +173,7 @@ struct BatchJob {
                               // numbers vertices and fills vertex-ordered rows where it can
     int nbr_half = 1;         // one neighbour lookup per axis (1) or two (0)
     bool wide = false;        // int16-lane keys (a lattice whose keys do not fit compact keys)
+    bool keys_sorted = false; // the images known to need int16-lane keys are in a job of their own
     int tile_w = 0;           // tile splat tile width in pixels (0: the default, 16; height 256 / width)
     std::vector<BatchItem> items;
     // parity dumps (single-item jobs)

@@ -166,6 +166,22 @@ def test_slice_positions_at_the_ends_of_int16(gpu, d, sign):
         gpu.GaussTransform.apply(planar(far), planar(pos), planar(val), [1.0] * d)
 
 
+def test_images_too_large_for_compact_keys_start_on_wide_keys(gpu):
+    """Images whose pixel coordinates alone leave the fields' range: no rerun, at the first call
+    of a shape, for any place of the large coordinate."""
+    rng = np.random.default_rng(4)
+    for k, (w, h, sx, sy) in enumerate([(402, 90, 1.0, 9.0), (403, 91, 1.0, 9.0), (90, 410, 9.0, 1.0), (300, 50, 1.0, 8.0)]):
+        guide = rng.uniform(0, 1, (5, h, w)).astype(np.float32)   # nearly no vertex is shared
+        im = rng.uniform(0, 1, (2, h, w)).astype(np.float32)
+        out = im.copy()
+        gpu.JointBilateral.apply(out, guide, sx, sy, 0.0, 0.05)
+        assert k == 0 or gpu.last_stats()["retries"] == 0
+        pos, val = oracle.bilateral_points(im, guide, sx, 0.05, sigma_s_y=sy)
+        ref = oracle.oracle_lattice(pos, val).out
+        norm = (ref[:, :2] / ref[:, 2:]).reshape(h, w, 2).transpose(2, 0, 1)
+        assert rel_err(out, norm) <= RTOL_FP32
+
+
 def test_an_image_that_needs_wide_keys_does_not_mark_its_shape(gpu):
     """Images of one shape: after one that needs int16 lanes the next starts on them; after one
     that does not, or one that fails the call, compact keys are tried first (a rerun where
