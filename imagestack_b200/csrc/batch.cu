@@ -786,7 +786,8 @@ static int finish_pass(Engine& E, const BatchJob& B, const PassState& ps, std::v
         if (segstat[k] & kStatusKeyRange)
             return fail(PGPU_ERR_ARGUMENT,
                         "image %d: positions leave the lattice's int16 key range (the reference's "
-                        "keys wrap there and its rank indices leave [0, d]); scale them down", k);
+                        "keys wrap there and its rank indices leave [0, d]); scale them down",
+                        B.items[k].number >= 0 ? B.items[k].number : k);
         if (segstat[k] & kStatusWide) {   // rerun on int16-lane keys
             failed->push_back({k, true});
             if (cap_next) cap_next->push_back(ps.cap[k]);
@@ -1088,6 +1089,8 @@ int run_batch(Engine& E, const BatchJob& B, cudaStream_t st) {
         }
     }
     const int nseg = (int)cur.items.size();
+    for (int k = 0; k < nseg; ++k)   // passes take them in other orders
+        if (cur.items[k].number < 0) cur.items[k].number = k;
     BatchJob part[3] = {cur, cur, cur};   // vertex-ordered or plain, slot rows, int16-lane keys
     part[1].slot_rows = true;
     part[2].wide = true;

@@ -654,7 +654,7 @@ void pinned_put(Engine& E, unsigned char* p, size_t bytes) {
 
 int bilateral_batch_host(Engine& E, cudaStream_t st, const pgpu_image* ims, const pgpu_image* outs,
                          int count, const float* filter_width, const float* color_sigma,
-                         const pgpu_options& opt, AsyncBatch* ab, bool wide = false);
+                         const pgpu_options& opt, AsyncBatch* ab, bool wide = false, const int* numbers = nullptr);
 
 // Finish the oldest queued batch (its download stream has reached its event): statuses and
 // learned ratios of every chunk; images whose hash range overflowed were left unfiltered
@@ -711,7 +711,7 @@ void complete_oldest(Engine& E) {
             cs.push_back(ab->cs[i]);
         }
         rc = bilateral_batch_host(E, E.stream, in.data(), out.data(), (int)in.size(), fw.data(), cs.data(),
-                                  ab->opt, nullptr, wide != 0);
+                                  ab->opt, nullptr, wide != 0, again[wide].data());
         if (rc) msg = last_error();
         else sum.retries = 1;
     }
@@ -735,7 +735,7 @@ namespace {
 
 int bilateral_batch_host(Engine& E, cudaStream_t st, const pgpu_image* ims, const pgpu_image* outs,
                          int count, const float* filter_width, const float* color_sigma,
-                         const pgpu_options& opt, AsyncBatch* ab, bool wide) {
+                         const pgpu_options& opt, AsyncBatch* ab, bool wide, const int* numbers) {
     const int C = ims[0].channels;
     std::vector<int> cut{0};
     size_t acc = 0, slot_floats = 0, chunk_floats = 0;
@@ -817,6 +817,7 @@ int bilateral_batch_host(Engine& E, cudaStream_t st, const pgpu_image* ims, cons
             BatchJob B;
             bilateral_job(dv.data(), cut[k], cut[k + 1], filter_width, color_sigma, opt, B);
             B.wide = wide;
+            for (int i = cut[k]; i < cut[k + 1]; ++i) B.items[i - cut[k]].number = numbers ? numbers[i] : i;
             if (ab) {
                 // queued: the autotuner's choice, no host wait (checked when it completes)
                 BatchJob tuned;

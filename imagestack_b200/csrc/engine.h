@@ -155,6 +155,7 @@ struct BatchItem {
     PointSource slice;     // slice positions when the job does not replay
     uint32_t n_slice = 0;
     OutView out;
+    int number = -1;       // the caller's number for it (messages); its place in the job where -1
 };
 
 // Lattices that share d, value channels and payload, run by the same launches.

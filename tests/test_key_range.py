@@ -261,3 +261,17 @@ def test_int16_lane_splats_of_images(gpu, monkeypatch, c, w, h, mode, rows):
         assert rel_err(out, norm) <= RTOL_FP32
         assert gpu.last_stats()["tiled"] == (1 if mode == "tile" else 0)
     check(gpu, pos, val)
+
+
+def test_messages_name_the_image_of_the_batch(gpu):
+    """The image that fails a batch is named by its place in the caller's list, also where the
+    passes took the images in another order."""
+    imgs = [synth.image(90, 70, 3, rects=4, seed=s) for s in range(4)]
+    imgs[0] = (imgs[0] * 3000).astype(np.float32)   # int16 lanes
+    imgs[2][1, 5, 6] = np.nan
+    fw, cs = [5.0, 5.5, 6.0, 6.5], [0.8, 0.2, 0.3, 0.4]
+    for _ in range(2):
+        with pytest.raises(gpu.PgpuError, match="image 2:"):
+            gpu.bilateral_batch([im.copy() for im in imgs], fw, cs)
+        with pytest.raises(gpu.PgpuError, match="image 2:"):
+            gpu.bilateral_batch_submit([im.copy() for im in imgs], fw, cs).wait()
