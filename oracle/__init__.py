@@ -69,6 +69,10 @@ def _harness_path() -> str:
     return REF_HARNESS_FAST_SO if os.environ.get("PGPU_REFERENCE_BUILD") == "shipped" else REF_HARNESS_SO
 
 
+class ReferenceUnavailable(OSError):
+    """The reference build is not on this machine."""
+
+
 def reference_available() -> bool:
     return os.path.exists(_harness_path())
 
@@ -76,6 +80,9 @@ def reference_available() -> bool:
 def _load_ref():
     global _ref
     if _ref is None:
+        if not reference_available():
+            raise ReferenceUnavailable("no %s: the reference sources were not there to build it from"
+                                       % os.path.relpath(_harness_path(), os.path.dirname(HERE)))
         lib = C.CDLL(_harness_path())
         lib.refh_last_error.restype = C.c_char_p
         lib.refh_lattice_create.restype = C.c_void_p
