@@ -247,18 +247,24 @@ size_t batch_meta_bytes(int nseg) { return layout(nseg, false).total; }
 
 // Whether two axes per blur pass are faster than one, by the vertices and points expected.
 // A pair saves a pass over memory; it reads nine rows and two more pairs of neighbours in
-// places of their own where two passes read three rows each.  Blur, pairs against single:
-// - few vertices, where launches count: 64x64 (3.5 k) 13 us, 15; 512x512 sigma 8 (142 k) 20,
-//   21; from 200 k on single is faster: 256x256 sigma 4 (211 k) 26, 24; 4K sigma 32 (539 k)
-//   56, 44; 4K sigma 16 (1.5 M) 126, 102; video d=6 (1.4 M) 130, 108; d=8 (3.5 M) 346, 347;
-// - rows beyond L2 (over 3.5 M) whose neighbours are near in memory: 4K sigmas 4 and 0.3
-//   (3.9 M, 0.47 per point) 255, 281; 4 and 0.1 (10.9 M, 1.3 per point) 880, 925;
-// - and far apart: 4K sigmas 4 and 0.05 (25.6 M, 3.1 per point) 3256, 2577; 8 and 0.05 (12.2 M,
-//   1.47 per point) 1156, 1086; d=16, 2M points (15.4 M) 6833, 5787.
-// 16-bit rows: 256 images (9.3 M) 5.40 ms in all, 5.43.
-static bool pairs_pay(int d, int payload, double vertices, uint64_t points) {
-    if (payload != kPayloadF32 || vertices < 2e5) return true;
-    return vertices > 3.5e6 && d < 10 && vertices < 1.4 * (double)points;
+// places of their own where two passes read three rows each, but none for an absent neighbour.
+// Measured at 512x512 to 4K, d = 3 to 12, rows of 2, 4 and 8 values (FP32); blur, single over pairs:
+// - few vertices, where launches count: 1.1 to 1.4 up to 0.4 M, of 8 values up to 1 M (0.286 M
+//   d=12 54 against 40 us); from there on 0.83 to 1.05 (1.4 M d=6 108 against 130 us, 1.5 M
+//   d=5 102 against 126);
+// - rows of 2 and 4 values that L2 holds in part, 48 to 160 MB: 1.0 to 1.1 (4.1 M d=5, 65 MB,
+//   298 against 269 us; 7.6 M, 122 MB, 608 against 562); larger, 0.79 to 0.96 (25.6 M 2577
+//   against 3256);
+// - rows of 8 values beyond L2: 0.9 to 0.99 where vertices are shared (12.9 M d=6, 1.6 per
+//   point, 1703 against 1891), but 1.04 to 1.14 above 2.6 per point, where most neighbours are
+//   absent (58.9 M d=7 10.5 against 9.2 ms); at d=16 even then 0.85 (15.4 M 5787 against 6833).
+// Over these 118 lattices the rule is 0.5 % from the better of the two; one axis from 0.2 M
+// vertices on was 3 %, pairs always 2.4 %.  16-bit rows: mostly ties.
+static bool pairs_pay(int d, int vdp, int payload, double vertices, uint64_t points) {
+    const double bytes = vertices * vdp * 4.0, per_point = vertices / (double)std::max<uint64_t>(points, 1);
+    if (payload != kPayloadF32 || vertices < (vdp == 8 ? 1e6 : 4e5)) return true;
+    if (vdp < 8) return bytes > 48e6 && bytes < 160e6;
+    return d < 10 && bytes > 200e6 && per_point > 2.6;
 }
 
 // Queue one pass over the batch on st, its metadata staged in the pinned buffer h (E.hmeta
@@ -387,7 +393,7 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     const bool blur_pairs = blur_mode && !strcmp(blur_mode, "pairs") ? true
                           : blur_mode && !strcmp(blur_mode, "single") ? false
                                                                        : B.blur_pairs >= 0 ? B.blur_pairs != 0
-                                                                       : pairs_pay(d, B.payload, expected, n_total);
+                                                                       : pairs_pay(d, vdp, B.payload, expected, n_total);
     // one neighbour lookup per axis (whoever numbers a vertex marks its down neighbours
     // absent first); PGPU_NBR=half or =both in the environment overrides the job's choice
     const char* nbr_mode = std::getenv("PGPU_NBR");
