@@ -873,6 +873,7 @@ def run_ours(args):
             line["p50_ms"] = line["served"]["p50_ms"]
             line["p99_ms"] = line["served"]["p99_ms"]
         if world == 1 and not args.no_cpu_baseline:
+            import oracle
             # each on its own: one that fails is reported and never takes another's place
             legs = [("cpu_baseline", lambda: cpu_baseline_single("strict"))]
             if oracle.reference_available():

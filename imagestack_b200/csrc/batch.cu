@@ -258,7 +258,7 @@ size_t batch_meta_bytes(int nseg) { return layout(nseg, false).total; }
 // - rows of 8 values beyond L2: 0.9 to 0.99 where vertices are shared (12.9 M d=6, 1.6 per
 //   point, 1703 against 1891), but 1.04 to 1.14 above 2.6 per point, where most neighbours are
 //   absent (58.9 M d=7 10.5 against 9.2 ms); at d=16 even then 0.85 (15.4 M 5787 against 6833).
-// Over these 118 lattices the rule is 0.5 % from the better of the two; one axis from 0.2 M
+// Over these 124 lattices the rule is 0.5 % from the better of the two; one axis from 0.2 M
 // vertices on was 3 %, pairs always 2.4 %.  16-bit rows: mostly ties.
 static bool pairs_pay(int d, int vdp, int payload, double vertices, uint64_t points) {
     const double bytes = vertices * vdp * 4.0, per_point = vertices / (double)std::max<uint64_t>(points, 1);
