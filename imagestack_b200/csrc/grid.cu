@@ -71,7 +71,9 @@ __global__ void __launch_bounds__(kGridThreads) grid_minmax_kernel(PointSource s
     unsigned lo[D], hi[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) lo[c] = 0xFFFFFFFFu, hi[c] = 0u;
-    for (uint32_t b = blockIdx.x; b < total; b += gridDim.x) {
+    // (64 bits: total may be as large as 2^32 - 1, which a 32-bit count would step over)
+    for (uint64_t next = blockIdx.x; next < total; next += gridDim.x) {
+        const uint32_t b = (uint32_t)next;
         const uint32_t row = b / pieces, x0 = (b - row * pieces) * kMinmaxPixels + threadIdx.x;
         const uint32_t t = row / (uint32_t)src.height, y = row - t * (uint32_t)src.height;
         const float* at = src.pos.base + (long long)t * src.pos.tstride + (long long)y * src.pos.ystride;
