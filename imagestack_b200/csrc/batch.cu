@@ -289,11 +289,6 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     const size_t accb = accum_bytes(B.payload), payb = payload_bytes(B.payload);
     const LatticeConsts lc = make_consts(d);
     const bool dumps = B.rec_vtx || B.dump_splat;
-    // Slot tags for the neighbour lookups pay for multi-word keys (d >= 8): those lattices
-    // are sparse, most neighbours are absent, and the table is far larger than L2.  At
-    // lower d most neighbours exist and the table fits in L2, where the tag is one more
-    // dependent load (4K d=5: neighbours 0.18 -> 0.23 ms with tags; 2M points d=16:
-    // 25.8 -> 20.5 ms).
     const bool graph = B.use_graph && !dumps;
     // Vertices are numbered in the reference's first-insertion order only for parity dumps
     // (first touches, a bitmap and its prefix popcount); otherwise in the order the splat
@@ -327,6 +322,10 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
     bool wide = wide_forced(B);
     if (!wide && !B.keys_sorted)
         for (char w : known_wide(B, sig)) wide = wide || w;
+    // Slot tags for the neighbour lookups pay at d >= 8: those lattices are sparse, most
+    // neighbours are absent, and the table is far larger than L2 (2M points at d=16: neighbours
+    // 11.1 ms without tags, 7.2 with).  At lower d most neighbours exist and the table fits in
+    // L2, where the tag would be one more dependent load.
     const bool use_tags = kw > 1;
     const int kb = compact_key_bytes(d);
     std::vector<uint64_t> cap(nseg);
@@ -620,7 +619,6 @@ static int enqueue_pass(Engine& E, const BatchJob& B, cudaStream_t st,
             } else {
             CompactNbrArgs na;
             na.keys = E.key0.p;
-            na.segs = (const Segment*)(dmeta + L.segs);
             na.nseg = nseg;
             na.seg_slot_base = (const uint32_t*)(dmeta + L.slotbase);
             na.seg_status = (const unsigned*)(dmeta + L.segstat);

@@ -144,7 +144,7 @@ cudaError_t HostCopier::copy(const std::vector<HostPiece>& pieces, cudaMemcpyKin
     }
     size_t total = 0;
     for (const HostPiece& p : pieces) total += p.bytes;
-    const size_t chunk = std::min(std::max(total / 12 & ~(size_t)4095, kMinChunk + 0), kMaxChunk + 0);
+    const size_t chunk = std::min(std::max(total / 12 & ~(size_t)4095, kMinChunk), kMaxChunk);
     chunks_.clear();
     for (size_t k = 0; k < pieces.size(); ++k) {
         const HostPiece& p = pieces[k];

@@ -863,13 +863,13 @@ compact_tile_kernel(CompactSplatArgs a, const __grid_constant__ SegSource<PARAM>
 // ---------------------------------------------------------------------------------
 constexpr int kDirectThreads = 128;
 // (d=16, 2M points: two probes in flight and 6 blocks per SM 4.30 ms, four and 4 blocks 4.48)
-__host__ __device__ constexpr int direct_min_blocks(int) { return 6; }
+constexpr int kDirectMinBlocks = 6;
 template <int D>
 __host__ __device__ constexpr int direct_ahead() { return D <= 7 ? (D + 1 < 4 ? D + 1 : 4) : 2; }
 __host__ __device__ constexpr size_t direct_smem_bytes(int d) { return (size_t)(d + 1) * kDirectThreads * 12; }
 
 template <int D, int VDP>
-__global__ void __launch_bounds__(kDirectThreads, direct_min_blocks(D)) compact_direct_kernel(CompactSplatArgs a) {
+__global__ void __launch_bounds__(kDirectThreads, kDirectMinBlocks) compact_direct_kernel(CompactSplatArgs a) {
     using K = CompactKey<D>;
     using T = typename K::T;
     constexpr int AH = direct_ahead<D>();
@@ -1015,7 +1015,6 @@ enum RowGather { kRowsInPlace = 0, kRowsCopy, kRowsHalf, kRowsBf16, kRowsNormali
 
 struct CompactNbrArgs {
     const void* keys;
-    const Segment* segs;
     int nseg;
     const uint32_t* seg_slot_base;   // nseg + 1 slot boundaries
     const unsigned* seg_status;
