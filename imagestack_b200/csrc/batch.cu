@@ -906,7 +906,7 @@ static Engine::Tuning::Setting with_option(Engine::Tuning::Setting s, int k, int
     case 0: s.load = kTuneLoads[o]; break;
     case 1: s.splat = o; break;
     case 2: s.vertex_rows = o; break;
-    case 3: s.nbr_half = o; break;
+    case 3: s.nbr_half = 1 - o; break;   // one lookup, the starting point, first: it is timed already
     case 4: s.pairs = o == 0; break;
     case 5: s.blur_grid = o; break;
     case 6: s.tile_w = o == 0 ? 16 : 32; break;
