@@ -155,9 +155,15 @@ void learned_ratios(const BatchJob& B, std::vector<uint64_t>* sig, std::vector<d
 bool coordinates_too_wide(int d, int max_quotient, const LatticeConsts& lc, const PointSource& s) {
     const int last[3] = {s.width - 1, s.height - 1, s.frames - 1};
     double reach[kMaxD] = {};   // each position's largest magnitude, signed; the smallest is 0
+    double sum = 0;
     int n = s.pos_channels;
     for (int k = 0; k < 3 && n < d; ++k)
-        if ((s.coord_mask >> k) & 1) reach[n++] = (double)last[k] * s.coord_scale[k];
+        if ((s.coord_mask >> k) & 1) {
+            reach[n] = (double)last[k] * s.coord_scale[k];
+            sum += std::fabs(reach[n++]);
+        }
+    // (no position counts for more than sqrt(2/3) of a quotient: nearly every image ends here)
+    if (0.82 * sum < max_quotient) return false;
     double coef[kMaxD] = {};    // of each position in elevated coordinate i (src/Permutohedral.h:293-299)
     for (int i = d; i > s.pos_channels; --i) {
         coef[i - 1] -= (double)i * lc.sf[i - 1];
