@@ -466,14 +466,13 @@ constexpr int kSplatThreads = 256;
 #endif
 __host__ __device__ constexpr int splat_min_blocks(int d) { return d <= 5 ? 6 : d <= 6 ? 4 : d <= 8 ? 3 : 2; }
 
-// kStatusFar where the greedy point may not fit a compact key (SplatArgs::fit)
+// whether the greedy point may not fit a compact key (SplatArgs::fit)
 template <int D>
-__device__ __forceinline__ void note_far(const Simplex<D>& sx, int fit, unsigned* status) {
-    if (!fit) return;
+__device__ __forceinline__ bool is_far(const Simplex<D>& sx, int fit) {
     bool far = false;
 #pragma unroll
     for (int k = 0; k <= D; ++k) far = far || abs(sx.g[k]) > fit;
-    if (far && !(__ldcg(status) & kStatusFar)) atomicOr(status, kStatusFar);
+    return far && fit;
 }
 
 template <int D, int VDP, typename Acc>
@@ -495,15 +494,16 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     const uint32_t i = (blockIdx.x - sg.splat_base) * (uint32_t)kSplatThreads + threadIdx.x;
     const bool valid = i < sg.n;
     const unsigned active = __ballot_sync(0xFFFFFFFFu, valid);
-    if (valid) {
     unsigned* status = a.seg_status + kseg;
+    bool far = false;
+    if (valid) {
     const TableView table{a.key0 + sg.slot_base, a.keyn + sg.slot_base, sg.cap, a.cap_total};
     float p[D], v[VDP];
     load_point<D, VDP>(sg.src, i, p, v);
     Simplex<D> sx;
     const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kSplatThreads, kSplatThreads};
     compute_simplex<D>(p, a.lc, sx, status, scr);
-    note_far<D>(sx, a.fit, status);
+    far = is_far<D>(sx, a.fit);
     const uint32_t gi = sg.point_base + i;   // point number in the batch
     const uint32_t e0 = gi * (uint32_t)(D + 1);
     Acc* vals = reinterpret_cast<Acc*>(a.vals) + (size_t)sg.slot_base * VDP;
@@ -588,9 +588,10 @@ __global__ void __launch_bounds__(kSplatThreads, splat_min_blocks(D)) splat_kern
     }
     if (a.rec) store_record<D>(a.rec, a.n_total, gi, row, sx.bary);
     }
-    if (!a.vlist) return;
-    __syncthreads();
-    block_list_flush(blist, a, kseg);
+    // one note per block and at its end: a point that waits for the status word itself costs the
+    // splat of an image with many far ones 10 %
+    if (__syncthreads_or(far) && threadIdx.x == 0) atomicOr(status, kStatusFar);
+    if (a.vlist) block_list_flush(blist, a, kseg);
 }
 
 // point (x, y, t) of a source: positions and values as load_point
@@ -715,13 +716,14 @@ __global__ void __launch_bounds__(kWideTileThreads, wide_tile_min_blocks(D)) wid
     float v[VDP], bary[D + 1];
     int loc[D + 1];
     uint32_t gi = 0;
+    bool far = false;
     if (valid) {
         float p[D];
         load_point_xyt<D, VDP>(sg.src, px, py, f, p, v);
         Simplex<D> sx;
         const SimplexScratch scr{s_delta + threadIdx.x, s_coord + threadIdx.x, kWideTileThreads, kWideTileThreads};
         compute_simplex<D>(p, a.lc, sx, status, scr);
-        note_far<D>(sx, a.fit, status);
+        far = is_far<D>(sx, a.fit);
         gi = sg.point_base + (f * H + py) * W + px;
         const uint32_t e0 = gi * (uint32_t)(D + 1);
         Key<1> key;
@@ -745,7 +747,7 @@ __global__ void __launch_bounds__(kWideTileThreads, wide_tile_min_blocks(D)) wid
             }
         }
     }
-    __syncthreads();
+    if (__syncthreads_or(far) && threadIdx.x == 0) atomicOr(status, kStatusFar);
 
     // Phase B: each distinct vertex of the tile into the global table once
     const uint32_t count = t_count;
