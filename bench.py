@@ -823,8 +823,9 @@ def run_ours(args):
                          "traffic": (traffic["splat_dram_bytes"] * FRAMES_PER_STEP
                                      if "splat_dram_bytes" in traffic else None),
                          "algorithmic_bytes": splat_bytes,
-                         "note": "issue bound: the per-point simplex, keys and hashes, plus one "
-                                 "float4 L2 reduction per (point, vertex); see profiles/"},
+                         "note": "bound by shared-memory and L1 wavefronts (65 % of their rate), then by "
+                                 "the table's probes and one float4 L2 reduction per (point, "
+                                 "vertex); see profiles/"},
             "roofline_atomics": atomics,
             "roofline_blur": dict(roofline_stages["blur"], peak=hbm, unit="GB/s"),
             "roofline_slice": dict(roofline_stages["slice"], peak=hbm, unit="GB/s"),

@@ -13,11 +13,13 @@
 //    pending state, fences or second read;
 //  * the steps to the next remainder and to a neighbour are an add of one field, the hash
 //    a few 32-bit multiplies.
-// Quotients reach about 0.75 of a position in sigmas, so fields hold images thousands of
-// sigmas across at d <= 5 and hundreds at d = 6 and 7.  A point whose keys do not fit sets
-// kStatusWide in the splat, before anything is written, and the host runs the lattice again on
-// the int16-lane keys.  A slice at other positions asks for no rerun: a position out of the
-// fields' range takes the int16 arithmetic on its own (slice_far_point).
+// Quotients reach about 0.8 of a position in sigmas, so the fields hold images 2500 sigmas wide
+// and more at d <= 5 and d = 8, 640 at d = 6, 155 at d = 7, 315 at d = 9 to 12 and 75 from d = 13
+// on: 1080p does not fit d = 7 at sigma 8, nor d = 10 at sigma 4.  Images whose pixel coordinates
+// leave that range start on the int16-lane keys; a point whose keys do not fit sets kStatusWide
+// in the splat, before anything is written, and the host runs the lattice again on them.  A
+// slice at other positions asks for no rerun: a position out of the fields' range takes the
+// int16 arithmetic on its own (slice_far_point).
 #pragma once
 
 #include <type_traits>
